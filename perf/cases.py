@@ -167,7 +167,7 @@ def prepare(case, seed):
         s["data"] = api.DeviceData.from_colmajor(_data(case, B, gen, dev))
         return s
     m = s["m"] = api.CuMetaBitsProbCircuit(_circuit(case["tree"], case["vars"], case["cats"], case["k"]), DEVICE)
-    theta = _params(case, gen, dev)
+    theta = s["theta"] = _params(case, gen, dev)
     api.update_parameters(m, theta)
     S = B
     if kind in ("em", "em_soft"):
@@ -181,7 +181,7 @@ def prepare(case, seed):
             s["soft"] = _log_dirichlet(gen, rows * case["vars"], case["cats"], dev).view(
                 rows, case["vars"], case["cats"]).permute(2, 1, 0).contiguous().permute(2, 1, 0)
         s["ids"] = (torch.randperm(rows, generator=gen, device=dev) + 1).to(torch.int32)
-        s["next"], s["ll"], s["theta"] = 0, torch.zeros(1, device=dev), theta
+        s["next"], s["ll"] = 0, torch.zeros(1, device=dev)
         m.workspace(B)
     elif kind == "ll":
         rows = case["rows"]
@@ -199,7 +199,6 @@ def prepare(case, seed):
         m.workspace(1)
     elif kind == "sample":
         shp = api.noise_shapes(m, S)
-        s["theta"] = theta
         s["u_sum"] = torch.rand(shp[0], generator=gen, device=dev)
         s["u_leaf"] = torch.rand(shp[1], generator=gen, device=dev)
         m.workspace(1)
@@ -262,6 +261,231 @@ def work(case):
         "soft": {"bytes": 4.0 * B * (P + edges + v * c), "flops": 0.0},
         "nflows": {"bytes": data + 4.0 * B * P + 4.0 * P, "flops": 0.0},
     }[kind]
+
+
+# ---- the same outputs in 64 bits, by plain torch ----------------------------------------------------------
+class _Tree:
+    """The HCLT over one latent tree: children before parents, and where a variable's parameters lie in the flat vector
+    (sum blocks by layer and then in post-order, row = latent state of the variable, column = state of its child;
+    leaves in post-order behind them)."""
+
+    def __init__(self, case):
+        parent, k, c = _tree(case["tree"], case["vars"]), case["k"], case["cats"]
+        self.k, self.cats, self.ch = k, c, [[] for _ in parent]
+        for y, p in enumerate(parent):
+            if p >= 0:
+                self.ch[p].append(y)
+        self.root = int(np.nonzero(parent < 0)[0][0])
+        self.order, stack = [], [self.root]     # parents before children, last child first
+        while stack:
+            y = stack.pop()
+            self.order.append(y)
+            stack.extend(self.ch[y])
+        self.order.reverse()
+        self.inner = [y for y in self.order if self.ch[y]]
+        layer, key = {}, []
+        for pos, y in enumerate(self.order):
+            lay = max((layer[x] for x in self.ch[y]), default=0)
+            layer[y] = lay + (2 if len(self.ch[y]) > 1 else 1) if self.ch[y] else 0
+            if self.ch[y]:
+                key.append((layer[y], pos, y))
+        self.sum_at, at = {}, 0
+        for _, _, y in sorted(key):
+            r = 1 if y == self.root else k
+            self.sum_at[y] = (at, r)
+            at += r * k
+        self.leaf_at = {y: at + i * k * c for i, y in enumerate(self.order)}
+
+    def sums(self, p, y):
+        """[..., r, k] of a parameter tensor [..., P]."""
+        at, r = self.sum_at[y]
+        return p[..., at:at + r * self.k].unflatten(-1, (r, self.k))
+
+    def leaf(self, p, y):
+        """[..., k, cats]"""
+        at = self.leaf_at[y]
+        return p[..., at:at + self.k * self.cats].unflatten(-1, (self.k, self.cats))
+
+    def up(self, theta, leaf_value):
+        """Per inner variable: exp(x - max) [B, k] of its children's log-values, sums [B, r]; and the root's log-values."""
+        out, kept = {}, {}
+        for y in self.order:
+            if not self.ch[y]:
+                out[y] = leaf_value(y)
+                continue
+            x = leaf_value(y) + sum(out.pop(c) for c in self.ch[y])
+            top = x.max(1, keepdim=True).values
+            e = (x - top).exp_()
+            s = e @ self.sums(theta, y).exp().t()
+            kept[y] = (e, s)
+            out[y] = s.log() + top
+        return kept, out[self.root][:, 0]
+
+    def down(self, theta, kept):
+        """Yields (variable, flow of its leaf nodes [B, k], flow of its sum nodes over their sums [B, r] or None)."""
+        flow = {self.root: torch.ones_like(kept[self.root][1])}
+        for y in reversed(self.order):
+            f = flow.pop(y)
+            if not self.ch[y]:
+                yield y, f, None
+                continue
+            e, s = kept[y]
+            g = f / s
+            f = e * (g @ self.sums(theta, y).exp())
+            for c in self.ch[y]:
+                flow[c] = f
+            yield y, f, g
+
+
+def _exact_em(case, s, t, theta):
+    B, c = case["batch"], case["cats"]
+    ids = (s["ids"][:B] - 1).long()
+    if case["kind"] == "em_soft":
+        soft = s["soft"][ids].double()
+
+        def value(y):
+            return torch.logsumexp(soft[:, y, None, :] + t.leaf(theta, y)[None], 2)
+    else:
+        x = s["data"].t[:, ids].long()
+        miss = None if s["data"].miss is None else s["data"].miss[:, ids].bool()
+
+        def value(y):
+            v = t.leaf(theta, y)[:, x[y]].t()
+            return v if miss is None else v.masked_fill(miss[y][:, None], 0.0)
+    kept, ll = t.up(theta, value)
+    new = torch.empty_like(theta)
+
+    def blend(old, share):
+        return (0.9 * old.exp() + 0.1 * share).log()
+
+    for y, f, g in t.down(theta, kept):
+        if g is not None:
+            w = t.sums(theta, y)
+            stat = w.exp() * (g.t() @ kept.pop(y)[0]) + 0.1 / t.k
+            t.sums(new, y).copy_(blend(w, stat / stat.sum(1, keepdim=True)))
+        w = t.leaf(theta, y)
+        if case["kind"] == "em_soft":
+            e = soft[:, y, None, :] + w[None]
+            stat, lost = ((e - torch.logsumexp(e, 2, keepdim=True)).exp() * f[:, :, None]).sum(0), 0.0
+        else:
+            keep = 1.0 if miss is None else (~miss[y]).double()[:, None]
+            stat = torch.zeros(c, t.k, dtype=torch.float64, device=theta.device).index_add_(0, x[y], f * keep).t()
+            lost = (f * (1.0 - keep)).sum(0)[:, None]
+        total = stat.sum(1, keepdim=True) + lost + 0.1
+        t.leaf(new, y).copy_(blend(w, (stat + 0.1 / c + lost * w.exp()) / total))
+    return {"ll": ll.sum()[None], "theta": new}
+
+
+def _exact_kld(t, p1, p2):
+    """KLD(p1 || p2) per set, and the gradients with respect to both ([S, P])."""
+    up, below = {}, {}
+    for y in t.order:
+        a, b = t.leaf(p1, y), t.leaf(p2, y)
+        v = (a.exp() * (a - b)).sum(-1)
+        if t.ch[y]:
+            below[y] = v = v + sum(up.pop(c) for c in t.ch[y])
+            a, b = t.sums(p1, y), t.sums(p2, y)
+            v = (a.exp() * (v[:, None, :] + a - b)).sum(-1)
+        up[y] = v
+    g1, g2 = torch.empty_like(p1), torch.empty_like(p2)
+    grad = {t.root: torch.ones_like(up[t.root])}
+    for y in reversed(t.order):
+        g = grad.pop(y)
+        if t.ch[y]:
+            a, b = t.sums(p1, y), t.sums(p2, y)
+            e = g[:, :, None] * a.exp()
+            t.sums(g1, y).copy_(e * (below.pop(y)[:, None, :] + a - b + 1.0))
+            t.sums(g2, y).copy_(-e)
+            g = e.sum(1)
+            grad.update((c, g) for c in t.ch[y])
+        d = t.leaf(p1, y) - t.leaf(p2, y)
+        t.leaf(g1, y).copy_(g[:, :, None] * (d + 1.0))
+        t.leaf(g2, y).copy_(g[:, :, None] * d.exp())     # the sign that the gradient of a leaf is returned with
+    return up[t.root][:, 0], g1, g2
+
+
+def _exact_adam(t, q, p):
+    k0, g, _ = _exact_kld(t, q[None], p[None])
+    g = g[0]
+    b1, b2 = (float(np.float32(1) - np.float32(b)) for b in (0.9, 0.999))     # the rates are float32 arguments
+    m, v = b1 * g, b2 * g * g
+    q = q - 1e-2 * (m / b1) / ((v / b2).sqrt() + 1e-8)
+    for y in t.order:
+        for part in ([t.sums(q, y)] if t.ch[y] else []) + [t.leaf(q, y)]:
+            part -= torch.logsumexp(part, -1, keepdim=True)
+    return {"kld": k0, "q": q, "m": m, "v": v}
+
+
+def _exact_soft(case, t, p, u):
+    key = (p[:, :u.shape[1]] - (-(u * (1.0 - 1e-6) + 1e-6).log()).log()) / 0.7
+    out = torch.empty(p.shape[0], case["vars"], case["cats"], dtype=torch.float64, device=p.device)
+    prob = {t.root: p.new_ones(p.shape[0], 1)}
+    for y in reversed(t.order):
+        w = prob.pop(y)
+        if t.ch[y]:
+            w = (w[:, :, None] * torch.softmax(t.sums(key, y), -1)).sum(1)
+            prob.update((c, w) for c in t.ch[y])
+        out[:, y] = (w[:, :, None] * t.leaf(p, y).exp()).sum(1)
+    return out
+
+
+def _exact_nflows(case, s, t, theta):
+    x = s["data"].t.long()
+    kept, _ = t.up(theta, lambda y: t.leaf(theta, y)[:, x[y]].t())
+    out = torch.full((theta.numel(), case["batch"]), -math.inf, dtype=torch.float64, device=theta.device)
+    eps = float(np.float32(1e-8))
+    for y, f, g in t.down(theta, kept):
+        if g is not None:
+            at, r = t.sum_at[y]
+            flow = t.sums(theta, y).exp()[:, :, None] * g.t()[:, None, :] * kept.pop(y)[0].t()[None]
+            out[at:at + r * t.k] = (flow / (eps + flow.sum(1, keepdim=True)) + eps).log_().flatten(0, 1)
+        at = t.leaf_at[y]
+        out[at:at + t.k * t.cats].unflatten(0, (t.k, t.cats)).scatter_(1, x[y].expand(t.k, 1, -1), (f / f).log().t()[:, None])
+    return out.t()
+
+
+def _exact_mi(case, s):
+    x = s["data"].t.long()
+    v, c, n = case["vars"], case["cats"], case["batch"]
+    hot = torch.zeros(v, c, n, device=x.device).scatter_(1, x[:, None], 1.0)     # counts are exact in float32
+    total = n + 0.1
+    single = ((hot.sum(2).double() + 0.1 / c) / total).log()
+    hot = hot.view(v * c, n)
+    out = torch.empty(v, v, dtype=torch.float64, device=x.device)
+    step = max(1, (1 << 27) // (v * c * c))
+    for i in range(0, v, step):
+        p = (hot[i * c:(i + step) * c] @ hot.t()).view(-1, c, v, c).double().add_(0.1 / (c * c)).div_(total)
+        out[i:i + step] = (p * (p.log() - single[i:i + step, :, None, None] - single)).sum((1, 3))
+    return out
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    s = prepare(case, seed)
+    if kind == "sample":
+        return None
+    if kind == "mi":
+        return _exact_mi(case, s)
+    t = _Tree(case)
+    if kind == "soft":
+        return _exact_soft(case, t, s["params"].double(), s["u"].double())
+    if kind == "kld":
+        k, g1, g2 = _exact_kld(t, s["p1"].double(), s["p2"].double())
+        return {"kld": k, "g1": g1, "g2": g2}
+    if kind == "kld_adam":
+        return _exact_adam(t, s["q"].double(), s["theta"].double())
+    theta = s["theta"].double()
+    if kind == "nflows":
+        return _exact_nflows(case, s, t, theta)
+    if kind == "ll":
+        x, miss, out = s["data"].t.long(), s["data"].miss, []
+        for r in range(0, case["rows"], 2048):
+            def value(y):
+                v = t.leaf(theta, y)[:, x[y, r:r + 2048]].t()
+                return v if miss is None else v.masked_fill(miss[y, r:r + 2048].bool()[:, None], 0.0)
+            out.append(t.up(theta, value)[1])
+        return torch.cat(out)
+    return _exact_em(case, s, t, theta)
 
 
 def tolerance(case):
