@@ -206,6 +206,9 @@ int32_t pcb_normalize_params(pcb_circuit* c, float* params_dev, uint32_t S, int3
  * The matching of two circuits' parameters (compute_mbpc_mapping) stays host code of the caller. */
 int32_t pcb_map_param_columns(float* dst_dev, const float* src_dev, uint32_t S, const uint32_t* ids_dst_dev,
                               const uint32_t* ids_src_dev, uint32_t n, pcb_stream s);
+/* dst[s + S*p] = src[s*P + p]: parameter sets (or uniforms) of a row-major host framework as the [S, P]
+ * column-major matrix every per-set entry point takes.  dst and src do not overlap. */
+int32_t pcb_param_columns(float* dst_dev, const float* src_dev, uint32_t S, uint64_t P, pcb_stream s);
 /* Node ids (1-based) of the heads of a multi-head circuit, in head order. */
 int32_t pcb_get_head_roots(pcb_circuit* c, uint32_t* roots_host, uint64_t n);
 

@@ -625,7 +625,18 @@ def _params_matrix(mbpc, p: ArrayLike) -> torch.Tensor:
         p = torch.from_numpy(np.atleast_2d(p).astype(np.float32, copy=False))
     if p.dim() == 1:
         p = p[None, :]
-    return p.to(mbpc.device).t().contiguous()
+    return _columns(mbpc, p.to(mbpc.device))
+
+
+def _columns(mbpc, p: torch.Tensor) -> torch.Tensor:
+    """`p.t().contiguous()`; a row-major float32 matrix of several rows goes through the library's own kernel."""
+    if p.dim() == 2 and p.dtype == torch.float32 and p.is_contiguous() and 1 < p.shape[0] < 32 * 65535 and p.shape[1] > 1 \
+            and not p.requires_grad:
+        out = torch.empty(p.shape[1], p.shape[0], dtype=torch.float32, device=p.device)
+        with torch.cuda.device(p.device):
+            _lib.check(mbpc.lib.pcb_param_columns(_ptr(out), _ptr(p), p.shape[0], p.shape[1], _stream(p.device)))
+        return out
+    return p.t().contiguous()
 
 
 def kld(mbpc: CuMetaBitsProbCircuit, params1: ArrayLike, params2: ArrayLike):
@@ -655,8 +666,10 @@ def kld_backward(mbpc: CuMetaBitsProbCircuit, params1=None, params2=None, reuse=
     assert reuse is not None, "call kld() first and pass its reuse tuple"
     ws, p1, p2, S = reuse
     P = num_parameters(mbpc)
-    g1 = torch.zeros(P, S, dtype=torch.float32, device=mbpc.device)
-    g2 = torch.zeros(P, S, dtype=torch.float32, device=mbpc.device)
+    # every parameter of a single-root circuit is written; the skipped edges of a fake root are not
+    make = torch.zeros if mbpc.info.num_heads else torch.empty
+    g1 = make(P, S, dtype=torch.float32, device=mbpc.device)
+    g2 = make(P, S, dtype=torch.float32, device=mbpc.device)
     _lib.check(mbpc.lib.pcb_kld_backward(mbpc.handle, ws, _ptr(p1), _ptr(p2), S, _ptr(g1), _ptr(g2),
                                          _stream(mbpc.device)))
     return g1.t(), g2.t()
@@ -806,7 +819,7 @@ def gumbel_sample(mbpc: CuMetaBitsProbCircuit, params: ArrayLike, num_vars: int,
     ud = None
     if not no_gumbel:
         assert u is not None, "pass uniforms `u` or no_gumbel=True"
-        ud = torch.as_tensor(u, dtype=torch.float32).to(mbpc.device).t().contiguous()
+        ud = _columns(mbpc, torch.as_tensor(u, dtype=torch.float32).to(mbpc.device))
     ws = mbpc.workspace(1)
     out = torch.empty(par_buffer_size, num_vars, S, dtype=torch.float32, device=mbpc.device)
     _lib.check(mbpc.lib.pcb_sample_soft(mbpc.handle, ws, _ptr(p), Sp, _ptr(ud), temperature, S, _ptr(out),

@@ -431,6 +431,13 @@ function map_pc_parameters!(params1::CuMatrix{Float32}, params2::CuMatrix{Float3
     params1
 end
 
+"[S, P] parameters from a row-major buffer ([P, S] as Julia sees it)"
+function param_columns!(dst::CuMatrix{Float32}, src::CuMatrix{Float32})
+    check(ccall((:pcb_param_columns, libpcb200), Int32, (CuPtr{Cfloat}, CuPtr{Cfloat}, UInt32, UInt64, Ptr{Cvoid}),
+                dst, src, size(dst, 1), size(dst, 2), stream()))
+    dst
+end
+
 "normalized_flows_with_prealloc(mbpc_xz, mbpc_z, data) — utils/cuda_preallocation.jl:287-304, mapping = (ids_z, ids_xz)"
 function normalized_flows(c_xz::PcbCircuit, c_z::PcbCircuit, data::CuMatrix{UInt8}, mapping; batch_size = size(data, 1))
     nf = per_sample_normalized_flows(c_xz, data; batch_size)
