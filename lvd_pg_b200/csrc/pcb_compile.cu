@@ -567,8 +567,8 @@ int32_t pcb_ws_ensure_sets(pcb_workspace* ws, uint32_t S, int need) {
   pcb_circuit* c = ws->c;
   PCB_CUDA(cudaSetDevice(c->device));
   if ((need & (PCB_WS_NODES | PCB_WS_EDGES)) && S > ws->S_cap) {
-    for (void* p : {(void*)ws->klds, (void*)ws->grads, (void*)ws->eprob, (void*)ws->cum}) if (p) cudaFree(p);
-    ws->klds = ws->grads = ws->eprob = ws->cum = nullptr;
+    for (void* p : {(void*)ws->klds, (void*)ws->grads, (void*)ws->eprob}) if (p) cudaFree(p);
+    ws->klds = ws->grads = ws->eprob = nullptr;
     ws->S_cap = S;
     // a handful of sets stays unpadded: the per-node values of neighbouring nodes then share 32-byte
     // sectors, which is what the gathers of a single-set KLD chain pay for
@@ -580,10 +580,8 @@ int32_t pcb_ws_ensure_sets(pcb_workspace* ws, uint32_t S, int need) {
     PCB_CUDA(cudaMalloc((void**)&ws->grads, (size_t)c->N * ws->ldS * sizeof(float)));
     ws->have_kld = false;
   }
-  if ((need & PCB_WS_EDGES) && !ws->eprob) {   // the relaxed sampler's per-edge and per-group matrices
+  if ((need & PCB_WS_EDGES) && !ws->eprob)   // the relaxed sampler's per-edge matrix
     PCB_CUDA(cudaMalloc((void**)&ws->eprob, (size_t)std::max(1u, c->n_inner) * ws->ldS * sizeof(float)));
-    PCB_CUDA(cudaMalloc((void**)&ws->cum, (size_t)std::max(1u, c->n_groups) * ws->ldS * sizeof(float)));
-  }
   // a pending entry of the walk stands for a sub-circuit over a scope disjoint from the other
   // pending ones, so V + 2 slots always suffice for a decomposable circuit
   ws->stack_cap = c->V + 2;
@@ -608,7 +606,7 @@ extern "C" int32_t pcb_workspace_destroy(pcb_workspace* ws) {
   if (ws->step_exec) cudaGraphExecDestroy(ws->step_exec);
   if (ws->kld_exec) cudaGraphExecDestroy(ws->kld_exec);
   for (void* p : {(void*)ws->mars, (void*)ws->flows, (void*)ws->blk_mx, (void*)ws->klds, (void*)ws->grads,
-                  (void*)ws->eprob, (void*)ws->cum, (void*)ws->stack, (void*)ws->sample_status, (void*)ws->ids_stage, (void*)ws->ll_tmp, (void*)ws->mn_part, (void*)ws->mn_tickets,
+                  (void*)ws->eprob, (void*)ws->stack, (void*)ws->sample_status, (void*)ws->ids_stage, (void*)ws->ll_tmp, (void*)ws->mn_part, (void*)ws->mn_tickets,
                   (void*)ws->kld_t_dev})
     if (p) cudaFree(p);
   delete ws;

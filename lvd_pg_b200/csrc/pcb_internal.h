@@ -256,8 +256,7 @@ struct pcb_workspace {
   int32_t* sample_status = nullptr;   // status word of the hard sampler's walk
   float* klds = nullptr;     // [N][ldS]
   float* grads = nullptr;    // [N][ldS]  (also td_probs)
-  float* eprob = nullptr;    // [n_inner][ldS]
-  float* cum = nullptr;      // [n_groups][ldS]
+  float* eprob = nullptr;    // [n_inner][ldS] normalised edge weights of the relaxed sampler
   uint32_t* stack = nullptr; // [S_cap][stack_cap]
   uint32_t stack_cap = 0;
   uint32_t kld_S = 0;
@@ -360,7 +359,23 @@ inline cudaError_t pcb_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
 #ifdef __CUDACC__
 __device__ __forceinline__ void pcb_grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pcb_grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// asynchronous copies of single floats into shared memory: any number in flight, no registers, no alignment rule
+__device__ __forceinline__ void pcb_copy4_async(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void pcb_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 #endif
+
+// the dense blocks whose parents lie in layer `lay`, and the largest row and child count over them
+static inline uint32_t pcb_layer_blocks(const pcb_circuit* c, uint32_t lay) {
+  return lay >= 1 && lay <= c->L ? c->h_dense_off[lay + 1] - c->h_dense_off[lay] : 0;
+}
+static inline void pcb_layer_extent(const pcb_circuit* c, uint32_t lay, uint32_t& R, uint32_t& K) {
+  for (uint32_t i = 0; i < pcb_layer_blocks(c, lay); ++i) {
+    const PcbDenseBlock& b = c->h_dense[c->h_dense_off[lay] + i];
+    R = b.R > R ? b.R : R; K = b.K > K ? b.K : K;
+  }
+}
 
 // entry points implemented across translation units and used by pcb_em_step
 int32_t pcb_allreduce_aggr(pcb_circuit* c, cudaStream_t st);
@@ -370,7 +385,7 @@ int32_t pcb_allreduce_range(pcb_circuit* c, uint64_t first, uint64_t count, cuda
 int32_t pcb_dense_forward(pcb_circuit* c, pcb_workspace* ws, uint32_t layer, cudaStream_t st);
 int32_t pcb_dense_backward(pcb_circuit* c, pcb_workspace* ws, uint32_t layer, cudaStream_t st);
 // which of a workspace's per-set buffers a call needs: node matrices (klds / grads), the walk stacks of the
-// one-warp-per-sample sampler, the relaxed sampler's per-edge matrices
+// one-warp-per-sample sampler, the relaxed sampler's per-edge matrix
 enum { PCB_WS_NODES = 1, PCB_WS_STACK = 2, PCB_WS_EDGES = 4 };
 int32_t pcb_ws_ensure_sets(pcb_workspace* ws, uint32_t S, int need);
 int32_t pcb_dense_tc_forward(pcb_circuit* c, pcb_workspace* ws, uint32_t layer, cudaStream_t st);

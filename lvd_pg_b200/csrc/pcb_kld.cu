@@ -138,11 +138,6 @@ struct KldLayer {
   uint32_t root; float* root_out;
 };
 
-__device__ __forceinline__ void copy4_async(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 __global__ void __launch_bounds__(KLD_THREADS) kld_up_layer_kernel(KldLayer a) {
   extern __shared__ float park[];   // [slots][p1 | p2][threads], then the staged values
   __shared__ float red[KLD_THREADS];
@@ -159,8 +154,8 @@ __global__ void __launch_bounds__(KLD_THREADS) kld_up_layer_kernel(KldLayer a) {
     const size_t base = ((size_t)b.pid0 + (size_t)(on ? i : 0) * b.K) * a.S + s0 + (on ? s : 0);
     if (on)
       for (uint32_t j = jg, m = 0; j < b.K && m < a.slots; j += JG, ++m) {
-        copy4_async(mine + (2 * m) * KLD_THREADS, a.p1 + base + (size_t)j * a.S);
-        copy4_async(mine + (2 * m + 1) * KLD_THREADS, a.p2 + base + (size_t)j * a.S);
+        pcb_copy4_async(mine + (2 * m) * KLD_THREADS, a.p1 + base + (size_t)j * a.S);
+        pcb_copy4_async(mine + (2 * m + 1) * KLD_THREADS, a.p2 + base + (size_t)j * a.S);
       }
     pcb_grid_dep_wait();
     const uint32_t cj = KLD_STAGE / a.St;
@@ -182,7 +177,7 @@ __global__ void __launch_bounds__(KLD_THREADS) kld_up_layer_kernel(KldLayer a) {
         for (uint32_t u = 0; u < 8; ++u)
           if (q < J && s < St && g0 + u * J < n) stage[(g0 + u * J) * a.St + s] = v0[u] + v1[u];
       }
-      if (c0 == 0) copies_wait();
+      if (c0 == 0) pcb_copies_wait();
       __syncthreads();
       if (on)
         for (; j < c0 + n; j += JG, ++m) {
@@ -372,12 +367,12 @@ __global__ void __launch_bounds__(KLD_THREADS) kld_down_layer_kernel(KldLayer a)
     float ck = 0.0f;
     if (on) {
       for (uint32_t i = ig, m = 0; i < b.R && m < a.slots; i += IG, ++m) {
-        copy4_async(mine + (2 * m) * KLD_THREADS, a.p1 + base + i * step);
-        copy4_async(mine + (2 * m + 1) * KLD_THREADS, a.p2 + base + i * step);
+        pcb_copy4_async(mine + (2 * m) * KLD_THREADS, a.p1 + base + i * step);
+        pcb_copy4_async(mine + (2 * m + 1) * KLD_THREADS, a.p2 + base + i * step);
       }
       ck = a.klds[(size_t)(b.c0 + j) * a.ld + s0 + s];
       if (b.d0 != PCB_NONE) ck += a.klds[(size_t)(b.d0 + j) * a.ld + s0 + s];
-      copies_wait();
+      pcb_copies_wait();
       for (uint32_t i = ig, m = 0; i < b.R && m < a.slots; i += IG, ++m) {
         const float x = mine[(2 * m) * KLD_THREADS], ea = expf(x);
         mine[(2 * m + 1) * KLD_THREADS] = ea * (ck + x - mine[(2 * m + 1) * KLD_THREADS]) + ea;
@@ -621,23 +616,11 @@ __global__ void renorm_kernel(float* __restrict__ theta, uint32_t n_groups, cons
 // with the caller's copies: two sets 240 against 264 us, four sets 397 against 228 us).
 constexpr uint32_t KLD_WARP_SETS = 2;
 
-uint32_t kld_layer_blocks(const pcb_circuit* c, uint32_t lay) {
-  return lay >= 1 && lay <= c->L ? c->h_dense_off[lay + 1] - c->h_dense_off[lay] : 0;
-}
-
-// largest row and child count over the dense blocks with parents in `lay`
-void kld_layer_extent(const pcb_circuit* c, uint32_t lay, uint32_t& R, uint32_t& K) {
-  for (uint32_t i = 0; i < kld_layer_blocks(c, lay); ++i) {
-    const PcbDenseBlock& b = c->h_dense[c->h_dense_off[lay] + i];
-    R = std::max(R, b.R); K = std::max(K, b.K);
-  }
-}
-
 KldLayer kld_layer(pcb_circuit* c, pcb_workspace* ws, const float* p1, const float* p2, uint32_t S, uint32_t lay) {
   KldLayer a;
   memset(&a, 0, sizeof(a));
   a.klds = ws->klds; a.grads = ws->grads; a.p1 = p1; a.p2 = p2; a.ld = ws->ldS; a.S = S; a.St = std::min(S, 32u);
-  if (kld_layer_blocks(c, lay)) a.blk = c->dense + c->h_dense_off[lay];
+  if (pcb_layer_blocks(c, lay)) a.blk = c->dense + c->h_dense_off[lay];
   a.kind = c->kind; a.n_estart = c->n_estart; a.n_ecount = c->n_ecount; a.n_pid0 = c->n_pid0;
   a.e_prime = c->e_prime; a.e_sub = c->e_sub; a.in_off = c->in_off; a.in_ent = c->in_ent; a.root = c->N - 1;
   return a;
@@ -653,7 +636,7 @@ cudaError_t kld_launch_layer(pcb_circuit* c, void (*kernel)(KldLayer), KldLayer&
   });
   if (e != cudaSuccess) return e;
   const uint32_t J = KLD_THREADS / a.St;
-  a.dense_ctas = kld_layer_blocks(c, lay) * a.per_blk;
+  a.dense_ctas = pcb_layer_blocks(c, lay) * a.per_blk;
   const uint32_t ctas = a.dense_ctas + (a.count + J - 1) / J;
   ++c->prof.launches[PCB_K_KLD];
   return pcb_launch_pdl(kernel, dim3(ctas, (a.S + a.St - 1) / a.St), dim3(KLD_THREADS),
@@ -704,7 +687,7 @@ extern "C" int32_t pcb_kld(pcb_circuit* c, pcb_workspace* ws, const float* param
     a.count = c->h_up_sparse_off[lay] - c->h_up_sparse_off[lay - 1];
     a.root_out = kld_out_dev;
     uint32_t R = 0, K = 1;
-    kld_layer_extent(c, lay, R, K);
+    pcb_layer_extent(c, lay, R, K);
     // a thread should have about twelve edges (24 KB of parameters in flight per CTA): rows that share a CTA
     const uint32_t J = KLD_THREADS / a.St;
     a.rows = R ? std::min({std::max(1u, (J * 12 + K / 2) / K), J, R}) : 1;
@@ -746,13 +729,13 @@ extern "C" int32_t pcb_kld_backward(pcb_circuit* c, pcb_workspace* ws, const flo
     a.nodes = c->down_sparse + c->h_down_sparse_off[lay];
     a.count = c->h_down_sparse_off[lay + 1] - c->h_down_sparse_off[lay];
     uint32_t R = 0, K = 1;
-    kld_layer_extent(c, (uint32_t)lay + 1, R, K);
+    pcb_layer_extent(c, (uint32_t)lay + 1, R, K);
     // children of a CTA: whole 256-byte runs of parameters; the rest of the threads split the rows
     const uint32_t J = KLD_THREADS / a.St;
     a.rows = std::min({std::max(1u, 64 / a.St), J, K});
     a.per_blk = (K + a.rows - 1) / a.rows;
     a.slots = std::min(KLD_SLOTS, ((R ? R : 1) + J / a.rows - 1) / (J / a.rows));
-    if (!a.count && !kld_layer_blocks(c, (uint32_t)lay + 1)) continue;
+    if (!a.count && !pcb_layer_blocks(c, (uint32_t)lay + 1)) continue;
     PCB_CUDA(kld_launch_layer(c, kld_down_layer_kernel, a, (uint32_t)lay + 1, chained, st));
     chained = true;
   }

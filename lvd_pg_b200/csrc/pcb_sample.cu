@@ -25,9 +25,7 @@ struct Shape2 {
   dim3 block, grid;
 };
 Shape2 shape_for(uint32_t S, uint32_t items) {
-  uint32_t bx = 1;
-  while (bx < S && bx < 32) bx <<= 1;
-  uint32_t by = 128 / bx;
+  const uint32_t bx = std::min(S, 32u), by = 128 / bx;   // consecutive threads take consecutive words
   Shape2 s;
   s.block = dim3(bx, by, 1);
   s.grid = dim3((items + by - 1) / by, (S + bx - 1) / bx, 1);
@@ -339,45 +337,188 @@ __global__ void __launch_bounds__(CW * 32) sample_hard_cta_kernel(
 
 // ---- soft sampling ------------------------------------------------------------------------------
 // unnormalised relaxed edge probabilities and their per-node sums; cum is stored per sum NODE
-__global__ void soft_params_kernel(float* __restrict__ eprob, float* __restrict__ cum, uint32_t ld, uint32_t S,
-                                   const float* __restrict__ params, uint32_t Sp, const float* __restrict__ u,
-                                   float temperature, const uint32_t* __restrict__ grp_node, uint32_t n_groups,
-                                   const uint32_t* __restrict__ n_pid0, const uint32_t* __restrict__ n_ecount) {
-  uint32_t g = blockIdx.x * blockDim.y + threadIdx.y;
-  uint32_t s = blockIdx.y * blockDim.x + threadIdx.x;
-  if (g >= n_groups || s >= S) return;
-  uint32_t n = grp_node[g];
-  uint32_t pid0 = n_pid0[n], cnt = n_ecount[n];
-  const size_t ps = Sp == 1 ? 0 : s, pld = Sp;
-  float sum = 0.0f;
-  for (uint32_t j = 0; j < cnt; ++j) {
-    float logp = params[ps + pld * (size_t)(pid0 + j)];
-    double gv = 0.0;
-    if (u) gv = -log(-log((double)u[s + (size_t)S * (pid0 + j)] * (1.0 - 1e-6) + 1e-6));
-    float unnorm = (float)exp(((double)logp + gv) / (double)temperature);
-    eprob[(size_t)(pid0 + j) * ld + s] = unnorm;
-    sum += unnorm;
+// ---- relaxed sampling: exp((log p + gumbel) / T) of every sum edge, normalised per sum node ------------------
+// The keys are formed in fp64 like the reference's (sample.jl:24-54 promotes through its Float64 literals), with
+// logarithm and exponential by table and short polynomial (P. T. P. Tang, ACM TOMS 15 (1989) and 16 (1990)): the
+// result is rounded to fp32 (6e-8), a hundred times the error of these series, and eight fp64 operations per logarithm
+// replace the forty or more of one that is exact to the last bit.  Arguments outside the tables'
+// range (u outside (0, 1), |z| >= 600, NaN) take the CUDA functions.  fp64 units and HBM are the bounds: 24 x 1.7 M
+// edges 462 -> 285 us, now with the division by the node's sum that the top-down pass made before.
+constexpr uint32_t SOFT_THREADS = 256;
+struct SoftTables {
+  double2 lg[128];     // 1/c and log c of 128 intervals of [sqrt(1/2), sqrt 2)
+  double ex[256];      // 2^(i/256)
+};
+
+__device__ __forceinline__ void soft_tables_fill(SoftTables* t) {
+  for (uint32_t i = threadIdx.x; i < 128; i += blockDim.x) {
+    const double mid = __hiloint2double((int)(0x3fe6a09eu + (i << 13) + (1u << 12)), 0);
+    // the two intervals around one keep c = 1: log x is then the polynomial in x - 1 alone, relatively exact there
+    const double rcp = (i == 74 || i == 75) ? 1.0 : 1.0 / mid;
+    t->lg[i] = make_double2(rcp, -log(rcp));
   }
-  cum[(size_t)n * ld + s] = sum;
+  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) t->ex[i] = exp2((double)i / 256.0);
+  __syncthreads();
 }
 
-__global__ void soft_down_kernel(float* __restrict__ td, uint32_t ld, uint32_t S, const float* __restrict__ eprob,
-                                 const float* __restrict__ cum, const uint32_t* __restrict__ nodes, uint32_t count,
-                                 uint32_t root, const uint32_t* __restrict__ in_off,
-                                 const PcbInEntry* __restrict__ in_ent) {
-  uint32_t i = blockIdx.x * blockDim.y + threadIdx.y;
-  uint32_t s = blockIdx.y * blockDim.x + threadIdx.x;
-  if (i >= count || s >= S) return;
-  uint32_t n = nodes[i];
-  uint32_t i0 = in_off[n], i1 = in_off[n + 1];
-  float acc = (i0 == i1 && n == root) ? 1.0f : 0.0f;
+// log of a positive normal double: |r| <= 2^-7 and the series ends after r^4, a relative 7e-10 at most
+__device__ __forceinline__ double soft_log(double x, const SoftTables* t) {
+  const int hi = __double2hiint(x), tmp = hi - 0x3fe6a09e, e = tmp >> 20;
+  const double m = __hiloint2double(hi - (e << 20), __double2loint(x));
+  const double2 c = t->lg[(tmp >> 13) & 127];
+  const double r = fma(m, c.x, -1.0);
+  const double q = fma(r, fma(r, fma(r, -0.25, 1.0 / 3.0), -0.5), 1.0);
+  const double ed = __hiloint2double(0x43300000, e ^ (int)0x80000000) - (4503599627370496.0 + 2147483648.0);   // (double)e
+  return fma(ed, 0.69314718055994530942, fma(r, q, c.y));
+}
+
+// exp(z) rounded to fp32, |z| < 600: |r| <= ln2 / 512, the series ends after r^2, a relative 4e-10
+__device__ __forceinline__ float soft_exp(double z, const SoftTables* t) {
+  const double shift = 6755399441055744.0;   // 1.5 * 2^52: the sum's low word is the rounded integer
+  const double s = fma(z, 256.0 / 0.69314718055994530942, shift);
+  const int n = __double2loint(s);
+  const double r = fma(s - shift, -0.69314718055994530942 / 256.0, z);
+  const double p = fma(fma(r, 0.5, 1.0), r, 1.0) * t->ex[n & 255];
+  return (float)__hiloint2double(__double2hiint(p) + ((n >> 8) << 20), __double2loint(p));
+}
+
+__device__ __forceinline__ float soft_weight(float logp, float u, bool noise, double inv_t, const SoftTables* t) {
+  double g = 0.0;
+  if (noise) {
+    const double x = fma((double)u, 1.0 - 1e-6, 1e-6);
+    g = u > 0.0f && u < 1.0f ? -soft_log(-soft_log(x, t), t) : -log(-log(x));
+  }
+  const double z = ((double)logp + g) * inv_t;
+  return fabs(z) < 600.0 ? soft_exp(z, t) : (float)exp(z);
+}
+
+// Threads are laid out (set, edge) with the set fastest, `rows` sum nodes per pass of a block; a thread keeps its up
+// to eight edges in registers between the sum and the division, wider nodes go through memory.
+__global__ void __launch_bounds__(SOFT_THREADS, 4) soft_params_kernel(
+    float* __restrict__ w, uint32_t ld, uint32_t S, uint32_t St, uint32_t rows, const float* __restrict__ params,
+    uint32_t Sp, const float* __restrict__ u, double inv_t, const uint32_t* __restrict__ grp_node, uint32_t n_groups,
+    const uint32_t* __restrict__ n_pid0, const uint32_t* __restrict__ n_ecount) {
+  __shared__ SoftTables tab;
+  __shared__ float red[SOFT_THREADS];
+  soft_tables_fill(&tab);
+  const uint32_t s0 = blockIdx.y * St, sw = min(St, S - s0), J = SOFT_THREADS / St, JG = J / rows;
+  const uint32_t q = threadIdx.x / St, s = threadIdx.x % St, r = q / JG, jg = q % JG;
+  const bool lane_on = q < JG * rows && s < sw;
+  const size_t ps = Sp == 1 ? 0 : s0 + s;
+  for (uint32_t g0 = blockIdx.x * rows; g0 < n_groups; g0 += gridDim.x * rows) {
+    const bool on = lane_on && g0 + r < n_groups;
+    uint32_t pid0 = 0, cnt = 0;
+    if (on) {
+      const uint32_t n = grp_node[g0 + r];
+      pid0 = n_pid0[n]; cnt = n_ecount[n];
+    }
+    const float* pp = params + ps + (size_t)Sp * pid0;
+    const float* pu = u ? u + s0 + s + (size_t)S * pid0 : nullptr;
+    float* pw = w + (size_t)pid0 * ld + s0 + s;
+    float x[8], y[8], sum = 0.0f;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+      const uint32_t j = jg + k * JG;
+      x[k] = j < cnt ? pp[(size_t)Sp * j] : 0.0f;
+      y[k] = u && j < cnt ? __ldcs(pu + (size_t)S * j) : 0.5f;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k)
+      if (jg + k * JG < cnt) { x[k] = soft_weight(x[k], y[k], u != nullptr, inv_t, &tab); sum += x[k]; }
+    for (uint32_t j = jg + 8 * JG; j < cnt; j += JG) {
+      const float e = soft_weight(pp[(size_t)Sp * j], u ? pu[(size_t)S * j] : 0.5f, u != nullptr, inv_t, &tab);
+      pw[(size_t)ld * j] = e;
+      sum += e;
+    }
+    red[threadIdx.x] = sum;
+    __syncthreads();
+    float total = 0.0f;
+    if (on)
+      for (uint32_t k = 0; k < JG; ++k) total += red[(r * JG + k) * St + s];
+    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k)
+      if (jg + k * JG < cnt) pw[(size_t)ld * (jg + k * JG)] = x[k] / total;
+    for (uint32_t j = jg + 8 * JG; j < cnt; j += JG) pw[(size_t)ld * j] /= total;
+  }
+}
+
+// One launch per layer, from the root down: the dense blocks with parents in the layer above hand their probability
+// to their children, the other nodes of the layer pull from their parents (all parents were completed by earlier
+// launches).  The weights of a CTA are copied into shared memory before the wait on the preceding launch, one private
+// slot per thread and row; after it the parents' values are staged in one batch.  784 variables x 64 latents x 24
+// samples: 993 -> 155 us over the 20 layers (one thread walked all parents of a child before).
+constexpr uint32_t SOFT_SLOTS = 40, SOFT_STAGE = 8 * SOFT_THREADS;
+
+struct SoftLayer {
+  float* td; const float* w;
+  uint32_t ld, S, St, JC, per_blk, dense_ctas, slots;
+  const PcbDenseBlock* blk;
+  const uint32_t* nodes; uint32_t count, root;
+  const uint32_t* in_off; const PcbInEntry* in_ent;
+};
+
+__global__ void __launch_bounds__(SOFT_THREADS) soft_down_kernel(SoftLayer a) {
+  extern __shared__ float park[];
+  __shared__ float red[SOFT_THREADS];
+  pcb_grid_dep_launch();
+  const uint32_t s0 = blockIdx.y * a.St, sw = min(a.St, a.S - s0), J = SOFT_THREADS / a.St;
+  const uint32_t q = threadIdx.x / a.St, s = threadIdx.x % a.St;
+  if (blockIdx.x < a.dense_ctas) {
+    const PcbDenseBlock b = a.blk[blockIdx.x / a.per_blk];
+    const uint32_t JC = a.JC, IG = J / JC;
+    const uint32_t jj = q % JC, ig = q / JC, j = blockIdx.x % a.per_blk * JC + jj;
+    const bool on = ig < IG && s < sw && j < b.K;
+    const float* base = a.w + ((size_t)b.pid0 + (on ? j : 0)) * a.ld + s0 + (on ? s : 0);
+    const size_t step = (size_t)b.K * a.ld;
+    float* const mine = park + threadIdx.x;
+    float* const stage = park + (size_t)a.slots * SOFT_THREADS;
+    if (on)
+      for (uint32_t i = ig, m = 0; i < b.R && m < a.slots; i += IG, ++m) pcb_copy4_async(mine + m * SOFT_THREADS, base + i * step);
+    pcb_grid_dep_wait();
+    const uint32_t ci = SOFT_STAGE / a.St;
+    float acc = 0.0f;
+    uint32_t i = ig, m = 0;
+    for (uint32_t c0 = 0; c0 < b.R; c0 += ci) {
+      const uint32_t n = min(ci, b.R - c0);
+      const float* tp = a.td + (size_t)(b.p0 + c0) * a.ld + s0 + s;
+      float v[8];
+      for (uint32_t g0 = q; g0 < n; g0 += 8 * J) {
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) v[k] = q < J && s < sw && g0 + k * J < n ? tp[(size_t)(g0 + k * J) * a.ld] : 0.0f;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k)
+          if (q < J && s < sw && g0 + k * J < n) stage[(g0 + k * J) * a.St + s] = v[k];
+      }
+      if (c0 == 0) pcb_copies_wait();
+      __syncthreads();
+      if (on)
+        for (; i < c0 + n; i += IG, ++m)
+          acc += stage[(i - c0) * a.St + s] * (m < a.slots ? mine[m * SOFT_THREADS] : base[i * step]);
+      if (c0 + ci < b.R) __syncthreads();
+    }
+    red[threadIdx.x] = acc;
+    __syncthreads();
+    if (on && ig == 0) {
+      float t = 0.0f;
+      for (uint32_t k = 0; k < IG; ++k) t += red[threadIdx.x + k * JC * a.St];
+      a.td[(size_t)(b.c0 + j) * a.ld + s0 + s] = t;
+      if (b.d0 != PCB_NONE) a.td[(size_t)(b.d0 + j) * a.ld + s0 + s] = t;
+    }
+    return;
+  }
+  const uint32_t k = (blockIdx.x - a.dense_ctas) * J + q;
+  pcb_grid_dep_wait();
+  if (q >= J || k >= a.count || s >= sw) return;
+  const uint32_t n = a.nodes[k], i0 = a.in_off[n], i1 = a.in_off[n + 1];
+  float acc = (i0 == i1 && n == a.root) ? 1.0f : 0.0f;
   for (uint32_t x = i0; x < i1; ++x) {
-    PcbInEntry en = in_ent[x];
-    float tp = td[(size_t)en.parent * ld + s];
-    if (en.pid != PCB_NONE) tp *= eprob[(size_t)en.pid * ld + s] / cum[(size_t)en.parent * ld + s];
+    const PcbInEntry en = a.in_ent[x];
+    float tp = a.td[(size_t)en.parent * a.ld + s0 + s];
+    if (en.pid != PCB_NONE) tp *= a.w[(size_t)en.pid * a.ld + s0 + s];
     acc += tp;
   }
-  td[(size_t)n * ld + s] = acc;
+  a.td[(size_t)n * a.ld + s0 + s] = acc;
 }
 
 __global__ void soft_leaf_kernel(const float* __restrict__ td, uint32_t ld, uint32_t S,
@@ -461,23 +602,44 @@ extern "C" int32_t pcb_sample_soft(pcb_circuit* c, pcb_workspace* ws, const floa
   if (st0 != PCB_OK) return st0;
   cudaStream_t st = (cudaStream_t)s;
   const uint32_t ld = ws->ldS;
-  ws->have_kld = false;  // klds rows are reused for the per-node normalisers
-  float* cum = ws->klds;
+  ws->have_kld = false;  // the node gradients' rows hold the probabilities
   float* td = ws->grads;
+  const uint32_t St = std::min(S, 32u), J = SOFT_THREADS / St, tiles = (S + St - 1) / St;
   PCB_CUDA(cudaMemsetAsync(out_dev, 0, (size_t)S * c->V * c->max_cats * sizeof(float), st));
   if (c->n_groups) {
-    Shape2 sh = shape_for(S, c->n_groups);
+    // about eight edges per thread: sum nodes that share a pass of a block
+    const uint32_t rows = std::max(1u, std::min(J, J * 8 / std::max(1u, c->max_group)));
+    const uint32_t passes = (c->n_groups + rows - 1) / rows;
     ++c->prof.launches[PCB_K_SAMPLE];
-    soft_params_kernel<<<sh.grid, sh.block, 0, st>>>(ws->eprob, cum, ld, S, params_dev, Sp, u_dev, temperature,
-                                                     c->grp_node, c->n_groups, c->n_pid0, c->n_ecount);
+    soft_params_kernel<<<dim3(std::min(passes, std::max(1u, 148 * 4 / tiles)), tiles), SOFT_THREADS, 0, st>>>(
+        ws->eprob, ld, S, St, rows, params_dev, Sp, u_dev, 1.0 / (double)temperature, c->grp_node, c->n_groups,
+        c->n_pid0, c->n_ecount);
   }
+  static PcbPerDeviceOnce once;
+  PCB_CUDA(once.run([&]() {
+    return cudaFuncSetAttribute(soft_down_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)((SOFT_SLOTS * SOFT_THREADS + SOFT_STAGE) * sizeof(float)));
+  }));
+  bool chained = false;   // the first launch waits for the weights in full, the others for the launch before them
+  SoftLayer a;
+  a.td = td; a.w = ws->eprob; a.ld = ld; a.S = S; a.St = St; a.root = c->N - 1; a.in_off = c->in_off; a.in_ent = c->in_ent;
   for (int64_t lay = c->L; lay >= 0; --lay) {
-    uint32_t o0 = c->h_down_all_off[lay], o1 = c->h_down_all_off[lay + 1];
-    if (o1 == o0) continue;
-    Shape2 sh = shape_for(S, o1 - o0);
+    const uint32_t blocks = pcb_layer_blocks(c, (uint32_t)lay + 1);
+    a.blk = blocks ? c->dense + c->h_dense_off[lay + 1] : nullptr;
+    a.nodes = c->down_sparse + c->h_down_sparse_off[lay];
+    a.count = c->h_down_sparse_off[lay + 1] - c->h_down_sparse_off[lay];
+    if (!blocks && !a.count) continue;
+    uint32_t R = 1, K = 1;
+    pcb_layer_extent(c, (uint32_t)lay + 1, R, K);
+    a.JC = std::min({std::max(1u, 64 / St), J, K});   // children of a CTA: runs of 256 bytes of weights
+    a.per_blk = (K + a.JC - 1) / a.JC;
+    a.slots = std::min(SOFT_SLOTS, (R + J / a.JC - 1) / (J / a.JC));
+    a.dense_ctas = blocks * a.per_blk;
     ++c->prof.launches[PCB_K_SAMPLE];
-    soft_down_kernel<<<sh.grid, sh.block, 0, st>>>(td, ld, S, ws->eprob, cum, c->down_all + o0, o1 - o0, c->N - 1,
-                                                   c->in_off, c->in_ent);
+    PCB_CUDA(pcb_launch_pdl(soft_down_kernel, dim3(a.dense_ctas + (a.count + J - 1) / J, tiles), dim3(SOFT_THREADS),
+                            blocks ? (a.slots * SOFT_THREADS + SOFT_STAGE) * sizeof(float) : 0, st,
+                            c->pdl && chained, a));
+    chained = true;
   }
   if (c->n_inputs) {
     Shape2 sh = shape_for(S, c->n_inputs);
