@@ -378,6 +378,12 @@ int32_t compile(const pcb_circuit_desc* d, pcb_circuit* c) {
   PCB_TRY(upload(&c->in_ent, in_ent, &bytes));
   PCB_TRY(upload(&c->dense, c->h_dense, &bytes));
   PCB_TRY(upload(&c->grp_node, grp_node, &bytes));
+  {
+    std::vector<uint32_t> loose;
+    for (uint32_t n : grp_node) if (!in_dense[n]) loose.push_back(n);
+    c->n_grp_loose = (uint32_t)loose.size();
+    if (c->n_grp_loose) PCB_TRY(upload(&c->grp_loose, loose, &bytes));
+  }
   {  // leaf chunks: inputs sorted by variable (stable), cut every PCB_LEAF_CHUNK leaves
     std::vector<uint32_t> order(NI), lvar, loff;
     for (uint32_t i = 0; i < NI; ++i) order[i] = i;
@@ -456,7 +462,7 @@ void free_circuit(pcb_circuit* c) {
   void* ptrs[] = {c->theta, c->aggr, c->kind, c->n_estart, c->n_ecount, c->n_pid0, c->n_region, c->e_prime,
                   c->e_sub, c->in_node, c->in_var, c->in_cats, c->in_poff, c->in_foff, c->node2input,
                   c->up_all, c->up_sparse, c->down_all, c->down_sparse, c->in_off, c->in_ent, c->dense,
-                  c->grp_node, c->lchunk_var, c->lchunk_off, c->lchunk_inputs, c->status, c->w_img, c->dense_img, c->w_img16, c->dense_img16,
+                  c->grp_node, c->grp_loose, c->lchunk_var, c->lchunk_off, c->lchunk_inputs, c->status, c->w_img, c->dense_img, c->w_img16, c->dense_img16,
                   c->lgrp_var, c->lgrp_off, c->s_node, c->s_leaf, c->n_head, c->head_roots, c->up_same, c->var_cats, c->check_word};
   for (void* p : ptrs) if (p) cudaFree(p);
   if (c->ev_g0) cudaEventDestroy(c->ev_g0);

@@ -135,6 +135,8 @@ struct pcb_circuit {
   PcbInEntry* in_ent = nullptr;
   PcbDenseBlock* dense = nullptr; // sorted by parent layer
   uint32_t* grp_node = nullptr;   // [n_groups] sum node of each parameter group
+  uint32_t* grp_loose = nullptr;  // [n_grp_loose] those outside dense blocks
+  uint32_t n_grp_loose = 0;
 
   // ---- host copies of the small per-layer tables ----
   std::vector<uint32_t> h_up_all_off, h_up_sparse_off;      // [L+1] (index = layer-1)

@@ -223,23 +223,183 @@ __global__ void __launch_bounds__(TPB) norm_sum4_kernel(const float* __restrict_
   for (uint32_t j = NS_REG4; j < cnt; ++j) put(j, edge_flow(j));
 }
 
+// A handful of nodes (the root beside a circuit's dense blocks): 32 examples per block and the node's edges dealt out
+// over eight warps, where one thread per example walks all of them one after the other above (the 64 edges of a single
+// root, 512 rows: 67 -> 9 us).
+constexpr uint32_t SPLIT_W = 8, SPLIT_REG = 16;
+__global__ void __launch_bounds__(32 * SPLIT_W) norm_split_kernel(
+    const float* __restrict__ flows, const float* __restrict__ mars, uint32_t ld, uint32_t B, Params p,
+    const uint32_t* __restrict__ grp_node, const uint4* __restrict__ s_node, const uint32_t* __restrict__ e_prime,
+    const uint32_t* __restrict__ e_sub, const int32_t* __restrict__ row_ids, uint32_t row_start, float* __restrict__ out,
+    uint64_t out_rows) {
+  __shared__ float part[SPLIT_W][32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, b = blockIdx.y * 32 + lane;
+  const uint32_t n = grp_node[blockIdx.x];
+  const uint4 sn = s_node[n];
+  const bool on = b < B;
+  const int64_t row = on ? data_row(row_ids, row_start, b) : 0;
+  const float pf = on ? flows[(size_t)n * ld + b] : 0.0f, pm = on ? mars[(size_t)n * ld + b] : 0.0f;
+  auto edge_flow = [&](uint32_t j) {
+    if (!on) return 0.0f;
+    const uint32_t sb = e_sub[sn.x + j];
+    float child = mars[(size_t)e_prime[sn.x + j] * ld + b] + p.at(row, (uint64_t)sn.z + j);
+    if (sb != PCB_NONE) child += mars[(size_t)sb * ld + b];
+    return pf == 0.0f ? 0.0f : pf * __expf(child - pm);
+  };
+  float ef[SPLIT_REG], total = 0.0f;
+#pragma unroll
+  for (uint32_t k = 0; k < SPLIT_REG; ++k) {
+    const uint32_t j = warp + k * SPLIT_W;
+    ef[k] = j < sn.y ? edge_flow(j) : 0.0f;
+    total += ef[k];
+  }
+  for (uint32_t j = warp + SPLIT_REG * SPLIT_W; j < sn.y; j += SPLIT_W) total += edge_flow(j);
+  part[warp][lane] = total;
+  __syncthreads();
+  total = 1e-8f;
+  for (uint32_t k = 0; k < SPLIT_W; ++k) total += part[k][lane];
+  if (!on) return;
+  const float inv = 1.0f / total;
+  float* const o = out + (size_t)row + (size_t)out_rows * sn.z;
+#pragma unroll
+  for (uint32_t k = 0; k < SPLIT_REG; ++k) {
+    const uint32_t j = warp + k * SPLIT_W;
+    if (j < sn.y) o[(size_t)out_rows * j] = __logf(ef[k] * inv + 1e-8f);
+  }
+  for (uint32_t j = warp + SPLIT_REG * SPLIT_W; j < sn.y; j += SPLIT_W)
+    o[(size_t)out_rows * j] = __logf(edge_flow(j) * inv + 1e-8f);
+}
+
+// The dense blocks with the circuit's own parameters.  An edge's flow is pf * w * x / sum(w * x) with x = exp(child -
+// block maximum) per example, so a block of threads forms x once for 128 examples and all children (shared memory) and
+// serves NB_PAR parents from it: per edge two products and one logarithm remain, where the kernels above fetch both
+// children and take an exponential (two for wide nodes) per edge.  x can underflow only where the forward pass, which
+// shifts by the same maximum, has dropped the term as well.  Bound: HBM (the [rows, P] output).  512 rows of a
+// 784-variable, 64-latent circuit, 3.5 GB: 2488 -> 628 us.  Neighbouring blocks take neighbouring examples of the
+// same parameters, so the pieces of an output column are written at the same time.
+constexpr uint32_t NB_TPB = 256, NB_EX = 128, NB_PAR = 32, NB_MAX_K = 320;
+
+template <bool VEC>   // VEC: rows of the output start at multiples of four, a lane takes four consecutive examples
+__global__ void __launch_bounds__(NB_TPB) norm_block_kernel(
+    const float* __restrict__ flows, const float* __restrict__ mars, const float* __restrict__ blk_mx, uint32_t ld, uint32_t B,
+    const float* __restrict__ theta, const PcbDenseBlock* __restrict__ blocks, uint32_t tiles, uint32_t chunks,
+    const int32_t* __restrict__ row_ids, uint32_t row_start, float* __restrict__ out, uint64_t out_rows) {
+  extern __shared__ float4 nb_smem[];
+  const uint32_t tile = blockIdx.x % tiles, rest = blockIdx.x / tiles;
+  const PcbDenseBlock blk = blocks[rest / chunks];
+  const uint32_t i0 = rest % chunks * NB_PAR, K = blk.K;
+  if (i0 >= blk.R) return;
+  const uint32_t np = min(NB_PAR, blk.R - i0), b0 = tile * NB_EX;
+  float* const x = reinterpret_cast<float*>(nb_smem);   // [K][NB_EX]
+  float* const w = x + (size_t)K * NB_EX;               // [NB_PAR][K]
+  {
+    const uint32_t e = threadIdx.x % NB_EX, b = b0 + e;
+    const float m = b < B ? blk_mx[(size_t)blk.mx_row * ld + b] : 0.0f;
+#pragma unroll 4
+    for (uint32_t j = threadIdx.x / NB_EX; j < K; j += NB_TPB / NB_EX) {
+      float t = 0.0f;
+      if (b < B) {
+        t = mars[(size_t)(blk.c0 + j) * ld + b];
+        if (blk.d0 != PCB_NONE) t += mars[(size_t)(blk.d0 + j) * ld + b];
+        t = expf(t - m);
+      }
+      x[j * NB_EX + e] = t;
+    }
+    const float* th = theta + blk.pid0 + (size_t)i0 * K;
+    for (uint32_t k = threadIdx.x; k < np * K; k += NB_TPB) w[k] = expf(__ldg(th + k));
+  }
+  __syncthreads();
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t ex[4];
+  int64_t row[4];
+#pragma unroll
+  for (uint32_t k = 0; k < 4; ++k) {
+    ex[k] = VEC ? lane * 4 + k : lane + 32 * k;
+    row[k] = b0 + ex[k] < B ? data_row(row_ids, row_start, b0 + ex[k]) : -1;
+  }
+  auto load_x = [&](uint32_t j, float (&v)[4]) {
+    if (VEC) {
+      const float4 q = *reinterpret_cast<const float4*>(x + j * NB_EX + lane * 4);
+      v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) v[k] = x[j * NB_EX + ex[k]];
+    }
+  };
+  for (uint32_t i = warp * 2; i < np; i += NB_TPB / 32 * 2) {   // two parents at a time share the reads of x
+    const uint32_t two = min(2u, np - i);
+    const float* w0 = w + (size_t)i * K;
+    const float* w1 = w + (size_t)(i + two - 1) * K;
+    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (uint32_t j = 0; j < K; ++j) {
+      float v[4];
+      load_x(j, v);
+      const float a = w0[j], b = w1[j];
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) { s0[k] = fmaf(a, v[k], s0[k]); s1[k] = fmaf(b, v[k], s1[k]); }
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {   // flow / (1e-8 + sum of the flows), the flows of a node adding up to pf
+      const size_t at = (size_t)(blk.p0 + i0 + i) * ld + b0 + ex[k];
+      const float f0 = row[k] >= 0 ? flows[at] : 0.0f, f1 = row[k] >= 0 ? flows[at + (size_t)(two - 1) * ld] : 0.0f;
+      s0[k] = f0 == 0.0f ? 0.0f : f0 / (s0[k] * (f0 + 1e-8f));
+      s1[k] = f1 == 0.0f ? 0.0f : f1 / (s1[k] * (f1 + 1e-8f));
+    }
+    float* const o = out + (size_t)out_rows * (blk.pid0 + (size_t)(i0 + i) * K);
+    const size_t next = two == 2 ? (size_t)out_rows * K : 0;   // a single last parent is written twice, the same values
+#pragma unroll 2
+    for (uint32_t j = 0; j < K; ++j) {
+      float v[4];
+      load_x(j, v);
+      const float a = w0[j], b = w1[j];
+      float* const q = o + (size_t)out_rows * j;
+      float v0[4], v1[4];
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) { v0[k] = __logf(a * v[k] * s0[k] + 1e-8f); v1[k] = __logf(b * v[k] * s1[k] + 1e-8f); }
+      if (VEC && row[3] >= 0) {
+        __stcs(reinterpret_cast<float4*>(q + row[0]), make_float4(v0[0], v0[1], v0[2], v0[3]));
+        __stcs(reinterpret_cast<float4*>(q + next + row[0]), make_float4(v1[0], v1[1], v1[2], v1[3]));
+      } else {
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+          if (row[k] >= 0) { __stcs(q + row[k], v0[k]); __stcs(q + next + row[k], v1[k]); }
+      }
+    }
+  }
+}
+
 // A learnable leaf hands its whole flow to the observed category (get_edge_flow,
 // nodes/fixable_categorical_dist.jl:162-176): log(flow / flow) = 0 there and log(0) = -inf elsewhere;
-// a leaf without flow gives 0 / 0 as in the reference.
-__global__ void norm_leaf_kernel(const float* __restrict__ flows, uint32_t ld, uint32_t B, uint64_t P,
-                                 const uint32_t* __restrict__ in_node, const uint32_t* __restrict__ in_var,
-                                 const uint32_t* __restrict__ in_cats, const uint64_t* __restrict__ in_poff,
-                                 const uint8_t* __restrict__ data, uint64_t num_rows,
-                                 const int32_t* __restrict__ row_ids, uint32_t row_start, float* __restrict__ out,
-                                 uint64_t out_rows) {
-  const uint32_t i = blockIdx.x, b = blockIdx.y * blockDim.x + threadIdx.x;
-  if (b >= B || in_poff[i] >= P) return;
+// a leaf without flow gives 0 / 0 as in the reference.  One block per chunk of leaves of one variable, whose observed
+// values it reads once.  Bound: HBM (the output); 512 rows of 50176 binary leaves 215 -> 70 us.
+__global__ void __launch_bounds__(TPB) norm_leaf_kernel(
+    const float* __restrict__ flows, uint32_t ld, uint32_t B, uint64_t P, const uint32_t* __restrict__ lchunk_var,
+    const uint32_t* __restrict__ lchunk_off, const uint32_t* __restrict__ lchunk_inputs, const uint32_t* __restrict__ in_node,
+    const uint32_t* __restrict__ in_cats, const uint64_t* __restrict__ in_poff, const uint8_t* __restrict__ data,
+    uint64_t num_rows, const int32_t* __restrict__ row_ids, uint32_t row_start, float* __restrict__ out, uint64_t out_rows) {
+  const uint32_t first = lchunk_off[blockIdx.x], n = lchunk_off[blockIdx.x + 1] - first;
+  __shared__ uint32_t s_node[PCB_LEAF_CHUNK], s_cats[PCB_LEAF_CHUNK];
+  __shared__ uint64_t s_off[PCB_LEAF_CHUNK];
+  if (threadIdx.x < n) {
+    const uint32_t i = lchunk_inputs[first + threadIdx.x];
+    s_node[threadIdx.x] = in_node[i]; s_cats[threadIdx.x] = in_cats[i]; s_off[threadIdx.x] = in_poff[i];
+  }
+  __syncthreads();
+  const uint32_t b = blockIdx.y * TPB + threadIdx.x;
+  if (b >= B) return;
   const int64_t row = data_row(row_ids, row_start, b);
-  const size_t di = (size_t)row + (size_t)num_rows * in_var[i];
-  const float f = flows[(size_t)in_node[i] * ld + b];
-  const uint32_t x = data[di], C = in_cats[i];
-  for (uint32_t c = 0; c < C; ++c)
-    out[(size_t)row + (size_t)out_rows * (in_poff[i] + c)] = logf((c == x ? f : 0.0f) / f);
+  const uint32_t x = data[(size_t)row + (size_t)num_rows * lchunk_var[blockIdx.x]];
+  float f[PCB_LEAF_CHUNK];
+#pragma unroll
+  for (uint32_t k = 0; k < PCB_LEAF_CHUNK; ++k) f[k] = k < n && s_off[k] < P ? flows[(size_t)s_node[k] * ld + b] : 0.0f;
+#pragma unroll
+  for (uint32_t k = 0; k < PCB_LEAF_CHUNK; ++k) {
+    if (k >= n || s_off[k] >= P) continue;
+    const float one = f[k] / f[k] - 1.0f;   // log of 1, or NaN without flow
+    float* const o = out + (size_t)row + (size_t)out_rows * s_off[k];
+    for (uint32_t c = 0; c < s_cats[k]; ++c) __stcs(o + (size_t)out_rows * c, c == x ? one : one - INFINITY);
+  }
 }
 
 // normalize_params (misc.jl:363-392, 405-447): on a [S, P] matrix of parameter sets, in place.
@@ -349,21 +509,46 @@ extern "C" int32_t pcb_normalized_flows(pcb_circuit* c, pcb_workspace* ws, const
   }
   const bool quads = !ev->row_ids_dev && (ev->row_start - 1) % 4 == 0 && ev->num_rows % 4 == 0 &&
                      (reinterpret_cast<uintptr_t>(out_dev) & 15) == 0 && (!params_dev || (reinterpret_cast<uintptr_t>(params_dev) & 15) == 0);
-  if (c->n_groups && quads) {
+  // dense blocks whose children fit in shared memory take the block kernel; of the other sum nodes a few are split
+  // over warps, many (64 keep every SM busy at 512 rows) take one thread per example
+  const bool block_path = !params_dev && c->n_dense && c->max_dense_K <= NB_MAX_K;
+  const uint32_t* groups = block_path ? c->grp_loose : c->grp_node;
+  const uint32_t n_groups = block_path ? c->n_grp_loose : c->n_groups;
+  if (block_path) {
+    const uint32_t tiles = (B + NB_EX - 1) / NB_EX, chunks = (c->max_dense_R + NB_PAR - 1) / NB_PAR;
+    PCB_REQUIRE((uint64_t)c->n_dense * chunks * tiles <= 0x7fffffffull, "too many dense blocks for one launch");
+    const size_t sm = (size_t)c->max_dense_K * (NB_EX + NB_PAR) * sizeof(float);
+    static PcbPerDeviceOnce once;
+    PCB_CUDA(once.run([]() {
+      const int most = (int)(NB_MAX_K * (NB_EX + NB_PAR) * sizeof(float));
+      const cudaError_t e = cudaFuncSetAttribute(norm_block_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+      return e != cudaSuccess ? e : cudaFuncSetAttribute(norm_block_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    }));
     ++c->prof.launches[PCB_K_MISC];
-    norm_sum4_kernel<<<dim3(c->n_groups, (B + 4 * TPB - 1) / (4 * TPB)), TPB, 0, st>>>(
-        ws->flows, ws->mars, ws->ld, B, p, c->grp_node, c->s_node, c->e_prime, c->e_sub, ev->row_start, out_dev, ev->num_rows);
-  } else if (c->n_groups) {
+    (quads ? norm_block_kernel<true> : norm_block_kernel<false>)<<<c->n_dense * chunks * tiles, NB_TPB, sm, st>>>(
+        ws->flows, ws->mars, ws->blk_mx, ws->ld, B, c->theta, c->dense, tiles, chunks, ev->row_ids_dev, ev->row_start, out_dev,
+        ev->num_rows);
+  }
+  if (n_groups && n_groups <= 64) {
     ++c->prof.launches[PCB_K_MISC];
-    norm_sum_kernel<<<grid2(c->n_groups, B), TPB, 0, st>>>(ws->flows, ws->mars, ws->ld, B, p, c->grp_node, c->s_node,
-                                                          c->e_prime, c->e_sub, ev->row_ids_dev, ev->row_start, out_dev,
-                                                          ev->num_rows);
+    norm_split_kernel<<<dim3(n_groups, (B + 31) / 32), 32 * SPLIT_W, 0, st>>>(
+        ws->flows, ws->mars, ws->ld, B, p, groups, c->s_node, c->e_prime, c->e_sub, ev->row_ids_dev, ev->row_start, out_dev,
+        ev->num_rows);
+  } else if (n_groups && quads) {
+    ++c->prof.launches[PCB_K_MISC];
+    norm_sum4_kernel<<<dim3(n_groups, (B + 4 * TPB - 1) / (4 * TPB)), TPB, 0, st>>>(
+        ws->flows, ws->mars, ws->ld, B, p, groups, c->s_node, c->e_prime, c->e_sub, ev->row_start, out_dev, ev->num_rows);
+  } else if (n_groups) {
+    ++c->prof.launches[PCB_K_MISC];
+    norm_sum_kernel<<<grid2(n_groups, B), TPB, 0, st>>>(ws->flows, ws->mars, ws->ld, B, p, groups, c->s_node,
+                                                        c->e_prime, c->e_sub, ev->row_ids_dev, ev->row_start, out_dev,
+                                                        ev->num_rows);
   }
   if (c->n_inputs) {
     ++c->prof.launches[PCB_K_MISC];
-    norm_leaf_kernel<<<grid2(c->n_inputs, B), TPB, 0, st>>>(ws->flows, ws->ld, B, c->P, c->in_node, c->in_var, c->in_cats,
-                                                           c->in_poff, ev->data_dev, ev->num_rows, ev->row_ids_dev,
-                                                           ev->row_start, out_dev, ev->num_rows);
+    norm_leaf_kernel<<<grid2(c->n_lchunks, B), TPB, 0, st>>>(
+        ws->flows, ws->ld, B, c->P, c->lchunk_var, c->lchunk_off, c->lchunk_inputs, c->in_node, c->in_cats, c->in_poff,
+        ev->data_dev, ev->num_rows, ev->row_ids_dev, ev->row_start, out_dev, ev->num_rows);
   }
   PCB_CUDA(cudaGetLastError());
   return PCB_OK;
