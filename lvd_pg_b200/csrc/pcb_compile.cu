@@ -265,7 +265,7 @@ int32_t compile(const pcb_circuit_desc* d, pcb_circuit* c) {
         if (excl && d0 != PCB_NONE) excl = indeg(d0 + t) == R && !dense_child[d0 + t];
       }
       if (!excl) { i = j; continue; }
-      PcbDenseBlock blk{n, R, K, c0, d0, n_pid0[n], (uint32_t)c->h_dense.size(), 0};
+      PcbDenseBlock blk{n, R, K, c0, d0, n_pid0[n], (uint32_t)c->h_dense.size(), PCB_NONE};
       c->h_dense.push_back(blk);
       for (uint32_t r = 0; r < R; ++r) in_dense[n + r] = 1;
       for (uint32_t t = 0; t < K; ++t) { dense_child[c0 + t] = 1; if (d0 != PCB_NONE) dense_child[d0 + t] = 1; }
@@ -277,6 +277,111 @@ int32_t compile(const pcb_circuit_desc* d, pcb_circuit* c) {
   }
   c->h_dense_off[c->L + 1] = (uint32_t)c->h_dense.size();
   c->n_dense = (uint32_t)c->h_dense.size();
+
+  // ---- the steps of an EM pass ----------------------------------------------------------------
+  // The up layers count a product layer below every block of sums, but a block whose prime children are products of
+  // consecutive, exclusive runs of nodes can form those products itself (their values are sums of the runs' values,
+  // and their flows are the runs' flows).  Without these fused products a circuit has about half as many dependent
+  // steps: step of a node = 1 + highest step below it, a fused product taking none.
+  std::vector<uint8_t> fused(N, 0), fused_src(N, 0);
+  std::vector<uint32_t> src_list;
+  for (PcbDenseBlock& b : c->h_dense) {
+    b.src = PCB_NONE;
+    const uint32_t m = ecount[b.c0];
+    std::vector<uint32_t> bases;
+    bool ok = kind[b.c0] == PCB_PRODUCT && m >= 1;
+    for (uint32_t i = 0; ok && i < m; ++i) {
+      const uint32_t e = estart[b.c0] + i;
+      for (uint32_t x : {d->up_prime[e], d->up_sub[e]}) if (x) bases.push_back(x - 1);
+    }
+    ok = ok && bases.size() <= PCB_MAX_SOURCES;
+    for (uint32_t t = 0; ok && t < b.K; ++t) {
+      const uint32_t n = b.c0 + t;
+      ok = kind[n] == PCB_PRODUCT && ecount[n] == m;
+      size_t x = 0;
+      for (uint32_t i = 0; ok && i < m; ++i) {
+        const uint32_t e = estart[n] + i;
+        for (uint32_t y : {d->up_prime[e], d->up_sub[e]})
+          if (y) { ok = ok && x < bases.size() && y - 1 == bases[x] + t && indeg(y - 1) == 1 && !dense_child[y - 1]; ++x; }
+      }
+      ok = ok && x == bases.size();
+    }
+    if (!ok) continue;
+    b.src = (uint32_t)src_list.size();
+    src_list.push_back((uint32_t)bases.size());
+    src_list.insert(src_list.end(), bases.begin(), bases.end());
+    for (uint32_t t = 0; t < b.K; ++t) {
+      fused[b.c0 + t] = 1;
+      for (uint32_t x : bases) fused_src[x + t] = 1;
+    }
+  }
+  if (src_list.empty()) src_list.push_back(0);
+  std::vector<uint32_t> step(N, 0), same_as(N);
+  for (uint32_t n = 0; n < N; ++n) same_as[n] = n;
+  for (const PcbDenseBlock& b : c->h_dense)
+    for (uint32_t r = 1; r < b.R; ++r) same_as[b.p0 + r] = b.p0;
+  for (uint32_t lay = 1; lay <= c->L; ++lay)
+    for (uint32_t n : layer_nodes[lay]) {
+      if (same_as[n] != n) { step[n] = step[same_as[n]]; continue; }   // the parents of a block have the same children
+      uint32_t top = 0;
+      for (uint32_t e = estart[n]; e < estart[n] + ecount[n]; ++e)
+        for (uint32_t x : {d->up_prime[e], d->up_sub[e]}) if (x) top = std::max(top, step[x - 1]);
+      step[n] = fused[n] ? top : top + 1;
+      c->n_steps = std::max(c->n_steps, step[n]);
+    }
+  // blocks by up layer for the passes over parameter sets, by step for the EM passes
+  std::vector<PcbDenseBlock> by_layer_blocks = c->h_dense;
+  c->h_layer_dense = by_layer_blocks;
+  c->h_layer_dense_off = c->h_dense_off;
+  std::stable_sort(c->h_dense.begin(), c->h_dense.end(),
+                   [&](const PcbDenseBlock& x, const PcbDenseBlock& y) { return step[x.p0] < step[y.p0]; });
+  const uint32_t T = c->n_steps;
+  c->h_dense_off.assign(T + 2, 0);
+  for (const PcbDenseBlock& b : c->h_dense) ++c->h_dense_off[step[b.p0] + 1];
+  for (uint32_t t = 0; t <= T; ++t) c->h_dense_off[t + 1] += c->h_dense_off[t];
+  // thin blocks: sum nodes outside dense blocks whose children are consecutive runs (the root); upward only
+  std::vector<PcbDenseBlock> thin;
+  std::vector<std::vector<uint32_t>> loose(T + 1), products(T + 1), pulled(T + 1), sources(T + 1);
+  std::vector<std::vector<PcbDenseBlock>> thin_at(T + 1);
+  std::vector<uint32_t> consumer(N, 0);   // step of the block that forms a fused product
+  for (const PcbDenseBlock& b : c->h_dense)
+    if (b.src != PCB_NONE) for (uint32_t t = 0; t < b.K; ++t) consumer[b.c0 + t] = step[b.p0];
+  for (uint32_t lay = 1; lay <= c->L; ++lay)
+    for (uint32_t n : layer_nodes[lay]) {
+      if (in_dense[n]) continue;
+      if (fused[n]) { products[consumer[n]].push_back(n); continue; }
+      bool run = allow_dense && kind[n] == PCB_SUM && ecount[n] >= MIN_K;
+      const uint32_t e0 = estart[n];
+      for (uint32_t j = 0; run && j < ecount[n]; ++j)
+        run = d->up_prime[e0 + j] == d->up_prime[e0] + j && (d->up_sub[e0] ? d->up_sub[e0 + j] == d->up_sub[e0] + j : !d->up_sub[e0 + j]);
+      if (run) thin_at[step[n]].push_back(PcbDenseBlock{n, 1, ecount[n], d->up_prime[e0] - 1, d->up_sub[e0] ? d->up_sub[e0] - 1 : PCB_NONE,
+                                                        n_pid0[n], PCB_NONE, PCB_NONE});
+      else loose[step[n]].push_back(n);
+    }
+  for (uint32_t n = 0; n < N; ++n) {
+    if (dense_child[n]) continue;
+    if (fused_src[n]) sources[consumer[in_ent[in_off[n]].parent]].push_back(n);
+    else pulled[step[n]].push_back(n);
+  }
+  std::vector<uint32_t> st_up, st_down, st_prod, st_src;
+  auto flatten = [&](std::vector<std::vector<uint32_t>>& lists, std::vector<uint32_t>& flat, std::vector<uint32_t>& off) {
+    off.assign(T + 2, 0);
+    for (uint32_t t = 0; t <= T; ++t) { off[t] = (uint32_t)flat.size(); flat.insert(flat.end(), lists[t].begin(), lists[t].end()); }
+    off[T + 1] = (uint32_t)flat.size();
+  };
+  // nodes a step computes one by one: the loose ones, then the thin blocks' (which the chain kernel takes as blocks)
+  c->h_st_thin_off.assign(T + 2, 0);
+  for (uint32_t t = 0; t <= T; ++t) {
+    c->h_st_thin_off[t] = (uint32_t)thin.size();
+    thin.insert(thin.end(), thin_at[t].begin(), thin_at[t].end());
+    for (const PcbDenseBlock& b : thin_at[t]) loose[t].push_back(b.p0);
+  }
+  c->h_st_thin_off[T + 1] = (uint32_t)thin.size();
+  c->h_thin = thin;
+  flatten(loose, st_up, c->h_st_up_off);
+  flatten(pulled, st_down, c->h_st_down_off);
+  flatten(products, st_prod, c->h_st_prod_off);
+  flatten(sources, st_src, c->h_st_src_off);
 
   // ---- layer lists --------------------------------------------------------------------------
   std::vector<uint32_t> up_all, up_sparse, down_all, down_sparse;
@@ -377,13 +482,29 @@ int32_t compile(const pcb_circuit_desc* d, pcb_circuit* c) {
   PCB_TRY(upload(&c->in_off, in_off, &bytes));
   PCB_TRY(upload(&c->in_ent, in_ent, &bytes));
   PCB_TRY(upload(&c->dense, c->h_dense, &bytes));
-  PCB_TRY(upload(&c->grp_node, grp_node, &bytes));
-  {
+  {  // the small tables of the steps share one allocation
     std::vector<uint32_t> loose;
     for (uint32_t n : grp_node) if (!in_dense[n]) loose.push_back(n);
     c->n_grp_loose = (uint32_t)loose.size();
-    if (c->n_grp_loose) PCB_TRY(upload(&c->grp_loose, loose, &bytes));
+    std::vector<uint32_t> pack;
+    auto put = [&](const void* src, size_t bytes_of) {
+      const size_t at = pack.size();
+      pack.resize(at + pcb_round_up((uint32_t)((bytes_of + 3) / 4), 4), 0);
+      if (bytes_of) memcpy(pack.data() + at, src, bytes_of);
+      return at;
+    };
+    const size_t o_ld = put(c->h_layer_dense.data(), c->h_layer_dense.size() * sizeof(PcbDenseBlock));
+    const size_t o_th = put(c->h_thin.data(), c->h_thin.size() * sizeof(PcbDenseBlock));
+    const size_t o_sl = put(src_list.data(), src_list.size() * 4), o_up = put(st_up.data(), st_up.size() * 4);
+    const size_t o_dn = put(st_down.data(), st_down.size() * 4), o_pr = put(st_prod.data(), st_prod.size() * 4);
+    const size_t o_sr = put(st_src.data(), st_src.size() * 4), o_lo = put(loose.data(), loose.size() * 4);
+    PCB_TRY(upload(&c->step_tables, pack, &bytes));
+    uint32_t* const t = c->step_tables;
+    c->layer_dense = reinterpret_cast<PcbDenseBlock*>(t + o_ld); c->thin = reinterpret_cast<PcbDenseBlock*>(t + o_th);
+    c->src_list = t + o_sl; c->st_up = t + o_up; c->st_down = t + o_dn; c->st_prod = t + o_pr; c->st_src = t + o_sr;
+    c->grp_loose = t + o_lo;
   }
+  PCB_TRY(upload(&c->grp_node, grp_node, &bytes));
   {  // leaf chunks: inputs sorted by variable (stable), cut every PCB_LEAF_CHUNK leaves
     std::vector<uint32_t> order(NI), lvar, loff;
     for (uint32_t i = 0; i < NI; ++i) order[i] = i;
@@ -432,6 +553,10 @@ int32_t compile(const pcb_circuit_desc* d, pcb_circuit* c) {
     if (const char* e = getenv("PCB_TC_KSPLIT")) { int v = atoi(e); c->tc_ksplit = (v == 1 || v == 2 || v == 4) ? v : 0; }
     if (const char* e = getenv("PCB_TC_NSPLIT")) { int v = atoi(e); c->tc_nsplit = (v == 1 || v == 2 || v == 4) ? v : 0; }
     if (const char* e = getenv("PCB_TC_A_STAGES")) { int v = atoi(e); c->tc_a_stages = (v == 2 || v == 4 || v == 8) ? v : 0; }
+    // the fp32 chain kernels take the small steps; a request for a particular tensor-core variant turns them off
+    if (const char* e = getenv("PCB_CHAIN_MACS")) c->chain_macs = strtoull(e, nullptr, 10);
+    const char* tc_impl = getenv("PCB_TC_IMPL");
+    c->chain = !(getenv("PCB_CHAIN") && atoi(getenv("PCB_CHAIN")) == 0) && !c->tc_ksplit && !c->tc_nsplit && !c->tc_a_stages && !tc_impl && !impl && c->use_tc;
     if (const char* e = getenv("PCB_EDGE_IMPL")) c->edge_ld = !strcmp(e, "ld");
     if (c->use_tc) PCB_TRY(pcb_dense_tc_prepare(c, &bytes));
   }
@@ -462,7 +587,7 @@ void free_circuit(pcb_circuit* c) {
   void* ptrs[] = {c->theta, c->aggr, c->kind, c->n_estart, c->n_ecount, c->n_pid0, c->n_region, c->e_prime,
                   c->e_sub, c->in_node, c->in_var, c->in_cats, c->in_poff, c->in_foff, c->node2input,
                   c->up_all, c->up_sparse, c->down_all, c->down_sparse, c->in_off, c->in_ent, c->dense,
-                  c->grp_node, c->grp_loose, c->lchunk_var, c->lchunk_off, c->lchunk_inputs, c->status, c->w_img, c->dense_img, c->w_img16, c->dense_img16,
+                  c->grp_node, c->step_tables, c->lchunk_var, c->lchunk_off, c->lchunk_inputs, c->status, c->w_img, c->dense_img, c->w_img16, c->dense_img16,
                   c->lgrp_var, c->lgrp_off, c->s_node, c->s_leaf, c->n_head, c->head_roots, c->up_same, c->var_cats, c->check_word};
   for (void* p : ptrs) if (p) cudaFree(p);
   if (c->ev_g0) cudaEventDestroy(c->ev_g0);

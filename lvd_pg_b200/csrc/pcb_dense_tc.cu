@@ -955,19 +955,25 @@ int32_t pcb_dense_tc_flush_edges(pcb_circuit* c, pcb_workspace* ws, cudaStream_t
   return PCB_OK;
 }
 
+// Edge statistics: steps are visited top down and their blocks are stored step after step, so
+// consecutive steps extend one block range downwards.  The range is launched once it holds
+// enough tiles for a few waves of CTAs; most steps alone would fill only a few SMs.  Called before
+// the step's child flows are launched (the statistics need its parents' flows only).
+int32_t pcb_dense_tc_note_edges(pcb_circuit* c, pcb_workspace* ws, uint32_t step, cudaStream_t st) {
+  const uint32_t o0 = c->h_dense_off[step], o1 = c->h_dense_off[step + 1];
+  if (o1 == o0 || c->skip_stats) return PCB_OK;
+  if (c->edge_hi > c->edge_lo && c->edge_lo != o1) PCB_TRY(pcb_dense_tc_flush_edges(c, ws, st));
+  if (c->edge_hi <= c->edge_lo) c->edge_hi = o1;
+  c->edge_lo = o0;
+  uint32_t tiles = ((c->max_dense_R + TM - 1) / TM) * ((c->max_dense_K + TN_MAX - 1) / TN_MAX);
+  if (!c->side || (c->edge_hi - c->edge_lo) * tiles >= c->edge_batch_tiles) PCB_TRY(pcb_dense_tc_flush_edges(c, ws, st));
+  return PCB_OK;
+}
+
 int32_t pcb_dense_tc_backward(pcb_circuit* c, pcb_workspace* ws, uint32_t layer, cudaStream_t st) {
   uint32_t o0 = c->h_dense_off[layer], o1 = c->h_dense_off[layer + 1];
   if (o1 == o0) return PCB_OK;
-  // Edge statistics: layers are visited top down and their blocks are stored layer after layer, so
-  // consecutive layers extend one block range downwards.  The range is launched once it holds
-  // enough tiles for a few waves of CTAs; most layers alone would fill only a few SMs.
-  if (!c->skip_stats) {
-    if (c->edge_hi > c->edge_lo && c->edge_lo != o1) PCB_TRY(pcb_dense_tc_flush_edges(c, ws, st));
-    if (c->edge_hi <= c->edge_lo) c->edge_hi = o1;
-    c->edge_lo = o0;
-    uint32_t tiles = ((c->max_dense_R + TM - 1) / TM) * ((c->max_dense_K + TN_MAX - 1) / TN_MAX);
-    if (!c->side || (c->edge_hi - c->edge_lo) * tiles >= c->edge_batch_tiles) PCB_TRY(pcb_dense_tc_flush_edges(c, ws, st));
-  }
+  PCB_TRY(pcb_dense_tc_note_edges(c, ws, layer, st));
   if (c->tc_mn) return pcb_dense_mn_backward_child(c, ws, layer, st);
   TcArgs args = make_args(c, ws, o0);
   {

@@ -21,6 +21,7 @@
 #include <cstring>
 
 #include "pcb_internal.h"
+#include "pcb_sparse.cuh"
 #include "pcb_tc.cuh"
 
 namespace {
@@ -37,122 +38,14 @@ __device__ __forceinline__ int64_t data_row(const int32_t* row_ids, uint32_t row
   return row_ids ? (int64_t)row_ids[b] - 1 : (int64_t)row_start - 1 + b;
 }
 
-// One thread per (node, four consecutive examples): every row access is a 16-byte load, so a warp
-// keeps 512 bytes per request in flight (the chain node -> edge list -> child row is four dependent
-// loads deep; with one example per thread it ran at a third of the memory roof).  Sum nodes: two
-// passes over the children (max, then sum of exp), one exp per edge instead of the exp + log of a
-// binary fold.  The last thread of a row may cover padding examples: the row pitch is a multiple
-// of 32, and whatever lands in the padding is never read as a result.
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
-__device__ __forceinline__ float4 adds4(float4 a, float s) { return make_float4(a.x + s, a.y + s, a.z + s, a.w + s); }
-__device__ __forceinline__ float4 max4(float4 a, float4 b) {
-  return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w));
+__global__ void sparse_up_kernel(PcbSparseUp a, const uint32_t* __restrict__ nodes) {
+  pcb_grid_dep_launch();
+  pcb_sparse_up_node(a, nodes[blockIdx.x], (blockIdx.y * blockDim.x + threadIdx.x) * 4u);
 }
 
-__global__ void sparse_up_kernel(float* __restrict__ mars, uint32_t ld, uint32_t B,
-                                 const uint32_t* __restrict__ nodes, const uint8_t* __restrict__ kind,
-                                 const uint32_t* __restrict__ n_estart, const uint32_t* __restrict__ n_ecount,
-                                 const uint32_t* __restrict__ n_pid0, const uint32_t* __restrict__ e_prime,
-                                 const uint32_t* __restrict__ e_sub, const float* __restrict__ theta) {
+__global__ void sparse_down_kernel(PcbSparseDown a, const uint32_t* __restrict__ nodes) {
   pcb_grid_dep_launch();
-  uint32_t n = nodes[blockIdx.x];
-  uint32_t b = (blockIdx.y * blockDim.x + threadIdx.x) * 4u;
-  if (b >= B) return;
-  uint32_t e0 = n_estart[n], cnt = n_ecount[n];
-  pcb_grid_dep_wait();   // everything above is static circuit data
-  auto child = [&](uint32_t j) {
-    float4 v = ld4(mars + (size_t)e_prime[e0 + j] * ld + b);
-    uint32_t sb = e_sub[e0 + j];
-    if (sb != PCB_NONE) v = add4(v, ld4(mars + (size_t)sb * ld + b));
-    return v;
-  };
-  float4 out;
-  if (kind[n] == PCB_SUM) {
-    const float* w = theta + n_pid0[n];
-    float4 mx = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-    for (uint32_t j = 0; j < cnt; ++j) mx = max4(mx, adds4(child(j), __ldg(w + j)));
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (uint32_t j = 0; j < cnt; ++j) {
-      const float4 v = adds4(child(j), __ldg(w + j));
-      // a maximum of -inf (every child impossible) gives exp(nan): masked below
-      acc.x += __expf(v.x - mx.x); acc.y += __expf(v.y - mx.y); acc.z += __expf(v.z - mx.z); acc.w += __expf(v.w - mx.w);
-    }
-    out.x = mx.x == -INFINITY ? -INFINITY : mx.x + __logf(acc.x);
-    out.y = mx.y == -INFINITY ? -INFINITY : mx.y + __logf(acc.y);
-    out.z = mx.z == -INFINITY ? -INFINITY : mx.z + __logf(acc.z);
-    out.w = mx.w == -INFINITY ? -INFINITY : mx.w + __logf(acc.w);
-  } else {
-    out = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (uint32_t j = 0; j < cnt; ++j) out = add4(out, child(j));
-  }
-  *reinterpret_cast<float4*>(mars + (size_t)n * ld + b) = out;
-}
-
-// Pull-based top-down pass: flows[n][b] = sum over incoming edges of the edge flow
-//   product parent: flows[parent]; sum parent: flows[parent] * exp(child value + logp - mars[parent]).
-// The root (no incoming edge, last node) gets 1, any other parentless node 0.
-// Multi-head circuits (head_mask != null): the flow of head h starts at head_mask[row, h], every
-// other parentless node at 0 (src-jl/multi_head_pc/flow.jl:141-176).
-struct HeadInit {
-  const uint32_t* n_head;
-  const float* head_mask;
-  uint64_t mask_rows;
-  const int32_t* row_ids;
-  uint32_t row_start;
-};
-__global__ void sparse_down_kernel(float* __restrict__ flows, const float* __restrict__ mars, uint32_t ld,
-                                   uint32_t B, const uint32_t* __restrict__ nodes, uint32_t root,
-                                   const uint32_t* __restrict__ in_off, const PcbInEntry* __restrict__ in_ent,
-                                   const float* __restrict__ theta, float* __restrict__ aggr, HeadInit hi) {
-  pcb_grid_dep_launch();
-  uint32_t n = nodes[blockIdx.x];
-  uint32_t b = (blockIdx.y * blockDim.x + threadIdx.x) * 4u;
-  const bool any = b < B;                      // examples b .. b+3, those below B count
-  const uint32_t bb = any ? b : 0;
-  const bool a0 = b < B, a1 = b + 1 < B, a2 = b + 2 < B, a3 = b + 3 < B;
-  uint32_t i0 = in_off[n], i1 = in_off[n + 1];
-  pcb_grid_dep_wait();   // everything above is static circuit data
-  float4 acc;
-  if (hi.head_mask) {
-    const uint32_t h = hi.n_head[n];
-    acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (h != PCB_NONE) {
-      const float* mk = hi.head_mask + (size_t)hi.mask_rows * h;
-      if (a0) acc.x = mk[data_row(hi.row_ids, hi.row_start, b)];
-      if (a1) acc.y = mk[data_row(hi.row_ids, hi.row_start, b + 1)];
-      if (a2) acc.z = mk[data_row(hi.row_ids, hi.row_start, b + 2)];
-      if (a3) acc.w = mk[data_row(hi.row_ids, hi.row_start, b + 3)];
-    }
-  } else {
-    const float init = (i0 == i1 && n == root) ? 1.0f : 0.0f;
-    acc = make_float4(init, init, init, init);
-  }
-  const float4 my = ld4(mars + (size_t)n * ld + bb);
-  for (uint32_t i = i0; i < i1; ++i) {
-    PcbInEntry en = in_ent[i];
-    float4 f = ld4(flows + (size_t)en.parent * ld + bb);
-    if (en.pid != PCB_NONE) {
-      const float4 pm = ld4(mars + (size_t)en.parent * ld + bb);
-      const float lp = __ldg(theta + en.pid);
-      // order of additions as in flow.jl:55-58: prime + logp, then + sub
-      float4 child;
-      if (en.sib == PCB_NONE) {
-        child = adds4(my, lp);
-      } else {
-        const float4 sv = ld4(mars + (size_t)en.sib * ld + bb);
-        child = (en.flags & 1u) ? add4(adds4(my, lp), sv) : add4(adds4(sv, lp), my);
-      }
-      f.x *= __expf(child.x - pm.x); f.y *= __expf(child.y - pm.y);
-      f.z *= __expf(child.z - pm.z); f.w *= __expf(child.w - pm.w);
-      if (aggr && (en.flags & 1u)) {   // aggr == null: flows only (uniform over the grid)
-        float s = warp_sum((a0 ? f.x : 0.0f) + (a1 ? f.y : 0.0f) + (a2 ? f.z : 0.0f) + (a3 ? f.w : 0.0f));
-        if ((threadIdx.x & 31) == 0) atomicAdd(aggr + en.pid, s);
-      }
-    }
-    acc = add4(acc, f);
-  }
-  if (any) *reinterpret_cast<float4*>(flows + (size_t)n * ld + b) = acc;
+  pcb_sparse_down_node(a, nodes[blockIdx.x], (blockIdx.y * blockDim.x + threadIdx.x) * 4u);
 }
 
 // leaf statistics: aggr[foff + x_b] += flows[leaf][b] * w_b ; missing -> slot C
@@ -809,10 +702,13 @@ static int32_t forward_impl(pcb_circuit* c, pcb_workspace* ws, const pcb_evidenc
   ws->row_ids = ev.row_ids_dev; ws->row_start = ev.row_start; ws->have_forward = false;
   ws->soft = ev.soft_dev; ws->head_mask = ev.head_mask_dev;
   ws->soft_reg = ev.soft_dev ? 0.0f : ev.soft_reg; ws->soft_width = ev.soft_reg_width;
-  if (c->use_tc) PCB_TRY(pcb_dense_tc_refresh(c, st));
+  bool tensor = false;   // weight images are rebuilt only for a pass that reads them
+  for (uint32_t t = 1; t <= c->n_steps && !tensor; ++t)
+    tensor = c->h_dense_off[t + 1] > c->h_dense_off[t] && !pcb_chain_takes(c, ws, t);
+  if (c->use_tc && tensor) PCB_TRY(pcb_dense_tc_refresh(c, st));
   // the arrival counters of the K-split dense tiles return to zero by themselves; a pass that a lost
   // wait cut short must not leave a stale count to the next one
-  if (ws->mn_tickets) PCB_CUDA(cudaMemsetAsync(ws->mn_tickets, 0, 296 * sizeof(uint32_t), st));
+  if (ws->mn_tickets && tensor) PCB_CUDA(cudaMemsetAsync(ws->mn_tickets, 0, 296 * sizeof(uint32_t), st));
   if (c->n_inputs) {
     PcbProfScope ps(c, st, PCB_K_LEAF_FWD);
     if (ws->soft || ws->soft_reg > 0.0f) {
@@ -826,24 +722,28 @@ static int32_t forward_impl(pcb_circuit* c, pcb_workspace* ws, const pcb_evidenc
                                                       ev.miss_dev, ev.num_rows, ev.row_ids_dev, ev.row_start);
     }
   }
-  const bool fwd_split = c->fwd_split;
-  for (uint32_t lay = 1; lay <= c->L; ++lay) {
-    uint32_t o0 = c->h_up_sparse_off[lay - 1], o1 = c->h_up_sparse_off[lay];
-    // The sparse nodes and the dense blocks of one layer do not depend on each other (both read
-    // lower layers only): with a side stream the two kernels of a layer run side by side.
-    const bool has_dense = c->h_dense_off[lay + 1] > c->h_dense_off[lay];
-    const bool split = c->side && !c->prof.on && fwd_split && o1 > o0 && has_dense;
-    cudaStream_t ss = st;
+  auto sparse_up = [&](const uint32_t* nodes, uint32_t n, cudaStream_t ss, bool pdl) -> int32_t {
+    if (!n) return PCB_OK;
+    PcbProfScope ps(c, ss, PCB_K_SPARSE_UP);
+    PCB_CUDA(pcb_launch_pdl(sparse_up_kernel, grid2v(n, B), dim3(TPB), 0, ss, pdl, pcb_sparse_up_args(c, ws), nodes));
+    return PCB_OK;
+  };
+  for (uint32_t t = 1; t <= c->n_steps; ++t) {
+    if (pcb_chain_takes(c, ws, t)) {   // everything of the step in one launch
+      PCB_TRY(pcb_chain_forward(c, ws, t, st));
+      continue;
+    }
+    // The products that the step's dense blocks form over their sources come first here; the other nodes and the
+    // blocks do not depend on each other (both read earlier steps only): with a side stream they run side by side.
+    PCB_TRY(sparse_up(c->st_prod + c->h_st_prod_off[t], c->h_st_prod_off[t + 1] - c->h_st_prod_off[t], st, c->pdl));
+    const uint32_t n = c->h_st_up_off[t + 1] - c->h_st_up_off[t];
+    const bool split = c->side && !c->prof.on && c->fwd_split && n && c->h_dense_off[t + 1] > c->h_dense_off[t];
     if (split) {
       PCB_CUDA(cudaEventRecord(c->ev_fork, st));
       PCB_CUDA(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-      ss = c->side;
     }
-    if (o1 > o0)
-      { PcbProfScope ps(c, ss, PCB_K_SPARSE_UP); pcb_launch_pdl(sparse_up_kernel, grid2v(o1 - o0, B), dim3(TPB), 0, ss, c->pdl && !split, ws->mars, ws->ld, B, c->up_sparse + o0, c->kind,
-                                                          c->n_estart, c->n_ecount, c->n_pid0, c->e_prime,
-                                                          c->e_sub, c->theta); }
-    PCB_TRY(pcb_dense_forward(c, ws, lay, st));
+    PCB_TRY(sparse_up(c->st_up + c->h_st_up_off[t], n, split ? c->side : st, c->pdl && !split));
+    PCB_TRY(pcb_dense_forward(c, ws, t, st));
     if (split) {
       PCB_CUDA(cudaEventRecord(c->ev_join, c->side));
       PCB_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
@@ -930,35 +830,45 @@ static int32_t backward_impl(pcb_circuit* c, pcb_workspace* ws, const float* wei
   PCB_CUDA(cudaSetDevice(c->device));
   const uint32_t B = ws->B;
   PCB_REQUIRE(!c->n_heads || ws->head_mask, "the flows of a multi-head circuit need a head mask");
-  const HeadInit hi{c->n_head, ws->head_mask, ws->num_rows, ws->row_ids, ws->row_start};
+  const PcbHeadInit hi{c->n_head, ws->head_mask, ws->num_rows, ws->row_ids, ws->row_start};
   c->edge_lo = c->edge_hi = 0;
-  auto sparse_down = [&](int64_t lay, cudaStream_t ss, bool pdl) -> int32_t {
-    uint32_t o0 = c->h_down_sparse_off[lay], o1 = c->h_down_sparse_off[lay + 1];
-    if (o1 > o0) {
-      PcbProfScope ps(c, ss, PCB_K_SPARSE_DOWN);
-      PCB_CUDA(pcb_launch_pdl(sparse_down_kernel, grid2v(o1 - o0, B), dim3(TPB), 0, ss, pdl, ws->flows, ws->mars, ws->ld,
-                              B, c->down_sparse + o0, c->N - 1, c->in_off, c->in_ent, c->theta, c->skip_stats ? nullptr : c->aggr, hi));
-    }
+  auto sparse_down = [&](const uint32_t* nodes, uint32_t n, cudaStream_t ss, bool pdl) -> int32_t {
+    if (!n) return PCB_OK;
+    PcbProfScope ps(c, ss, PCB_K_SPARSE_DOWN);
+    PCB_CUDA(pcb_launch_pdl(sparse_down_kernel, grid2v(n, B), dim3(TPB), 0, ss, pdl, pcb_sparse_down_args(c, ws, hi), nodes));
     return PCB_OK;
   };
-  // Layer l: its sparse nodes pull their flows, then its dense blocks push flows to their children.
-  // The sparse nodes of layer l-1 read parents of layers >= l that are never children of a layer-l
-  // block, so they do not wait for the layer-l blocks: with a second side stream they run beside them.
+  auto pulled = [&](uint32_t t, cudaStream_t ss, bool pdl) {
+    return sparse_down(c->st_down + c->h_st_down_off[t], c->h_st_down_off[t + 1] - c->h_st_down_off[t], ss, pdl);
+  };
+  // Step t: its dense blocks push flows to their children (and to the nodes their fused products are products of),
+  // and the other nodes of step t - 1, whose parents all lie in steps >= t and are never children of a step-t block,
+  // pull theirs.  The first launch of the pass waits for the forward pass in full: the chain kernels read node values
+  // before they wait for the launch ahead of them.
   const bool split = c->side2 && !c->prof.on && c->bwd_split;
-  PCB_TRY(sparse_down(c->L, st, c->pdl));
-  for (int64_t lay = c->L; lay >= 1; --lay) {
-    const bool has_dense = c->h_dense_off[lay + 1] > c->h_dense_off[lay];
-    const bool has_sparse = c->h_down_sparse_off[lay] > c->h_down_sparse_off[lay - 1];
-    if (split && has_dense && has_sparse) {
-      PCB_CUDA(cudaEventRecord(c->ev_fork2, st));
-      PCB_CUDA(cudaStreamWaitEvent(c->side2, c->ev_fork2, 0));
-      PCB_TRY(sparse_down(lay - 1, c->side2, false));
-      PCB_TRY(pcb_dense_backward(c, ws, (uint32_t)lay, st));
-      PCB_CUDA(cudaEventRecord(c->ev_join2, c->side2));
-      PCB_CUDA(cudaStreamWaitEvent(st, c->ev_join2, 0));
+  PCB_TRY(pulled(c->n_steps, st, false));
+  for (uint32_t t = c->n_steps; t >= 1; --t) {
+    const uint32_t dense = c->h_dense_off[t + 1] - c->h_dense_off[t], others = c->h_st_down_off[t] - c->h_st_down_off[t - 1];
+    if (!dense) {
+      PCB_TRY(pulled(t - 1, st, c->pdl));
+    } else if (pcb_chain_takes(c, ws, t)) {
+      PCB_TRY(pcb_dense_tc_note_edges(c, ws, t, st));
+      PCB_TRY(pcb_chain_backward(c, ws, t, hi, st));
     } else {
-      PCB_TRY(pcb_dense_backward(c, ws, (uint32_t)lay, st));
-      PCB_TRY(sparse_down(lay - 1, st, c->pdl));
+      const bool beside = split && others;
+      if (beside) {   // the pulling nodes beside the blocks on a second side stream
+        PCB_CUDA(cudaEventRecord(c->ev_fork2, st));
+        PCB_CUDA(cudaStreamWaitEvent(c->side2, c->ev_fork2, 0));
+        PCB_TRY(pulled(t - 1, c->side2, false));
+      }
+      PCB_TRY(pcb_dense_backward(c, ws, t, st));
+      PCB_TRY(sparse_down(c->st_src + c->h_st_src_off[t], c->h_st_src_off[t + 1] - c->h_st_src_off[t], st, c->pdl));
+      if (beside) {
+        PCB_CUDA(cudaEventRecord(c->ev_join2, c->side2));
+        PCB_CUDA(cudaStreamWaitEvent(st, c->ev_join2, 0));
+      } else {
+        PCB_TRY(pulled(t - 1, st, c->pdl));
+      }
     }
   }
   if (c->use_tc && !c->skip_stats) PCB_TRY(pcb_dense_tc_flush_edges(c, ws, st));

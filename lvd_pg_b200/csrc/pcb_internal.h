@@ -39,8 +39,9 @@ struct PcbDenseBlock {
   uint32_t d0;    // first sub child or PCB_NONE
   uint32_t pid0;  // first parameter id
   uint32_t mx_row;  // row of the per-block max buffer in the workspace
-  uint32_t pad;
+  uint32_t src;     // the prime children are fused products: where their list [count, first nodes of the runs] starts in src_list
 };
+#define PCB_MAX_SOURCES 24   // runs a fused product may add up
 
 // Where a dense block's weight images live (floats into w_img): exp(theta) split into TF32 hi/lo
 // and stored as operand tiles [column tile][K chunk][hi | lo][rows x 32 floats, 128-byte swizzle].
@@ -133,7 +134,18 @@ struct pcb_circuit {
   uint32_t* down_sparse = nullptr;
   uint32_t* in_off = nullptr;     // [N+1] CSR by child
   PcbInEntry* in_ent = nullptr;
-  PcbDenseBlock* dense = nullptr; // sorted by parent layer
+  PcbDenseBlock* dense = nullptr; // sorted by step
+  PcbDenseBlock* layer_dense = nullptr;   // the same sorted by parent layer
+  // the steps of an EM pass (1 .. n_steps): blocks with their fused products, thin blocks (single sum nodes over
+  // consecutive children, upward only) and nodes taken one by one
+  uint32_t n_steps = 0;
+  uint32_t* step_tables = nullptr;   // the allocation that holds the tables below, layer_dense and grp_loose
+  PcbDenseBlock* thin = nullptr;
+  uint32_t* src_list = nullptr;   // [count, runs ...] per fused block
+  uint32_t* st_up = nullptr;      // nodes a step computes one by one (thin blocks' nodes last)
+  uint32_t* st_down = nullptr;    // nodes that pull their flows, by their own step
+  uint32_t* st_prod = nullptr;    // fused products by the step that uses them
+  uint32_t* st_src = nullptr;     // ... and the nodes they are products of
   uint32_t* grp_node = nullptr;   // [n_groups] sum node of each parameter group
   uint32_t* grp_loose = nullptr;  // [n_grp_loose] those outside dense blocks
   uint32_t n_grp_loose = 0;
@@ -141,8 +153,13 @@ struct pcb_circuit {
   // ---- host copies of the small per-layer tables ----
   std::vector<uint32_t> h_up_all_off, h_up_sparse_off;      // [L+1] (index = layer-1)
   std::vector<uint32_t> h_down_all_off, h_down_sparse_off;  // [L+2] (index = layer)
-  std::vector<uint32_t> h_dense_off;                        // [L+1] blocks by parent layer
+  std::vector<uint32_t> h_dense_off;                        // [n_steps+2] blocks by step
   std::vector<PcbDenseBlock> h_dense;
+  std::vector<uint32_t> h_layer_dense_off;                  // [L+2] blocks by parent layer
+  std::vector<PcbDenseBlock> h_layer_dense, h_thin;
+  std::vector<uint32_t> h_st_up_off, h_st_down_off, h_st_prod_off, h_st_src_off, h_st_thin_off;   // [n_steps+2]
+  uint64_t chain_macs = 0;      // PCB_CHAIN_MACS: cost limit of the fp32 chain kernels (0: the built-in rule, ~0: always)
+  bool chain = true;            // PCB_CHAIN=0: dense blocks always on the tensor cores
   uint32_t n_dense = 0;
   uint32_t max_dense_K = 0, max_dense_R = 0;
 
@@ -365,16 +382,19 @@ __device__ __forceinline__ void pcb_grid_dep_launch() { asm volatile("griddepcon
 __device__ __forceinline__ void pcb_copy4_async(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
+__device__ __forceinline__ void pcb_copy16_async(float* dst, const float* src) {   // both 16-byte aligned
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
 __device__ __forceinline__ void pcb_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 #endif
 
 // the dense blocks whose parents lie in layer `lay`, and the largest row and child count over them
 static inline uint32_t pcb_layer_blocks(const pcb_circuit* c, uint32_t lay) {
-  return lay >= 1 && lay <= c->L ? c->h_dense_off[lay + 1] - c->h_dense_off[lay] : 0;
+  return lay >= 1 && lay <= c->L ? c->h_layer_dense_off[lay + 1] - c->h_layer_dense_off[lay] : 0;
 }
 static inline void pcb_layer_extent(const pcb_circuit* c, uint32_t lay, uint32_t& R, uint32_t& K) {
   for (uint32_t i = 0; i < pcb_layer_blocks(c, lay); ++i) {
-    const PcbDenseBlock& b = c->h_dense[c->h_dense_off[lay] + i];
+    const PcbDenseBlock& b = c->h_layer_dense[c->h_layer_dense_off[lay] + i];
     R = b.R > R ? b.R : R; K = b.K > K ? b.K : K;
   }
 }
@@ -384,6 +404,18 @@ int32_t pcb_allreduce_aggr(pcb_circuit* c, cudaStream_t st);
 // checked mode: validates row ids and categories of a batch, synchronises, PCB_ERR_INVALID with the first finding
 int32_t pcb_check_batch(pcb_circuit* c, const pcb_evidence& ev, cudaStream_t st);
 int32_t pcb_allreduce_range(pcb_circuit* c, uint64_t first, uint64_t count, cudaStream_t st);
+// pcb_chain.cu: one step of a pass on the fp32 chain kernels
+bool pcb_chain_takes(const pcb_circuit* c, const pcb_workspace* ws, uint32_t step);
+struct PcbHeadInit {
+  const uint32_t* n_head;
+  const float* head_mask;
+  uint64_t mask_rows;
+  const int32_t* row_ids;
+  uint32_t row_start;
+};
+int32_t pcb_chain_forward(pcb_circuit* c, pcb_workspace* ws, uint32_t step, cudaStream_t st);
+int32_t pcb_chain_backward(pcb_circuit* c, pcb_workspace* ws, uint32_t step, const PcbHeadInit& hi, cudaStream_t st);
+int32_t pcb_dense_tc_note_edges(pcb_circuit* c, pcb_workspace* ws, uint32_t step, cudaStream_t st);
 int32_t pcb_dense_forward(pcb_circuit* c, pcb_workspace* ws, uint32_t layer, cudaStream_t st);
 int32_t pcb_dense_backward(pcb_circuit* c, pcb_workspace* ws, uint32_t layer, cudaStream_t st);
 // which of a workspace's per-set buffers a call needs: node matrices (klds / grads), the walk stacks of the

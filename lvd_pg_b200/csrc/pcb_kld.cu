@@ -620,7 +620,7 @@ KldLayer kld_layer(pcb_circuit* c, pcb_workspace* ws, const float* p1, const flo
   KldLayer a;
   memset(&a, 0, sizeof(a));
   a.klds = ws->klds; a.grads = ws->grads; a.p1 = p1; a.p2 = p2; a.ld = ws->ldS; a.S = S; a.St = std::min(S, 32u);
-  if (pcb_layer_blocks(c, lay)) a.blk = c->dense + c->h_dense_off[lay];
+  if (pcb_layer_blocks(c, lay)) a.blk = c->layer_dense + c->h_layer_dense_off[lay];
   a.kind = c->kind; a.n_estart = c->n_estart; a.n_ecount = c->n_ecount; a.n_pid0 = c->n_pid0;
   a.e_prime = c->e_prime; a.e_sub = c->e_sub; a.in_off = c->in_off; a.in_ent = c->in_ent; a.root = c->N - 1;
   return a;

@@ -625,7 +625,7 @@ extern "C" int32_t pcb_sample_soft(pcb_circuit* c, pcb_workspace* ws, const floa
   a.td = td; a.w = ws->eprob; a.ld = ld; a.S = S; a.St = St; a.root = c->N - 1; a.in_off = c->in_off; a.in_ent = c->in_ent;
   for (int64_t lay = c->L; lay >= 0; --lay) {
     const uint32_t blocks = pcb_layer_blocks(c, (uint32_t)lay + 1);
-    a.blk = blocks ? c->dense + c->h_dense_off[lay + 1] : nullptr;
+    a.blk = blocks ? c->layer_dense + c->h_layer_dense_off[lay + 1] : nullptr;
     a.nodes = c->down_sparse + c->h_down_sparse_off[lay];
     a.count = c->h_down_sparse_off[lay + 1] - c->h_down_sparse_off[lay];
     if (!blocks && !a.count) continue;
