@@ -595,6 +595,7 @@ void free_circuit(pcb_circuit* c) {
   if (c->gstream) cudaStreamDestroy(c->gstream);
   if (c->ev_fork2) cudaEventDestroy(c->ev_fork2);
   if (c->ev_join2) cudaEventDestroy(c->ev_join2);
+  if (c->ev_sort) cudaEventDestroy(c->ev_sort);
   for (cudaEvent_t ev : {c->ev_c0, c->ev_c1, c->ev_c2, c->ev_c3}) if (ev) cudaEventDestroy(ev);
   if (c->comm_stream) cudaStreamDestroy(c->comm_stream);
   if (c->side2) cudaStreamDestroy(c->side2);
@@ -666,10 +667,13 @@ extern "C" int32_t pcb_workspace_create(pcb_circuit* c, uint32_t max_batch, int3
     delete ws;
     return pcb_fail(PCB_ERR_CUDA, std::string("workspace allocation: ") + cudaGetErrorString(e3));
   }
-  if (cudaMalloc((void**)&ws->ids_stage, (size_t)max_batch * sizeof(int32_t)) != cudaSuccess) {
+  // the staged row ids and, behind them, the sorted examples of the leaf statistics
+  const size_t ids = pcb_round_up(max_batch, 32), order = (size_t)c->V * pcb_round_up(max_batch, 256);
+  if (cudaMalloc((void**)&ws->ids_stage, (ids + order) * sizeof(int32_t)) != cudaSuccess) {
     pcb_workspace_destroy(ws);
     return pcb_fail(PCB_ERR_CUDA, "workspace allocation: row id staging");
   }
+  ws->leaf_order = reinterpret_cast<uint32_t*>(ws->ids_stage) + ids;
   {
     int32_t st = pcb_dense_edge_prepare_ws(ws);
     if (st != PCB_OK) { pcb_workspace_destroy(ws); return st; }

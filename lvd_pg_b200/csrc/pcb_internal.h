@@ -191,7 +191,7 @@ struct pcb_circuit {
   bool side_busy = false;
   // second side stream: the sparse nodes of layer l-1 take their flows while the dense blocks of layer l run
   cudaStream_t side2 = nullptr;
-  cudaEvent_t ev_fork2 = nullptr, ev_join2 = nullptr;
+  cudaEvent_t ev_fork2 = nullptr, ev_join2 = nullptr, ev_sort = nullptr;
   cudaStream_t gstream = nullptr;   // stands in for the legacy default stream, which cannot be captured
   cudaEvent_t ev_g0 = nullptr, ev_g1 = nullptr;
   bool graph_enabled = true;
@@ -251,6 +251,7 @@ struct pcb_workspace {
   uint64_t step_launches[PCB_K_COUNT] = {0};   // launches of one replay, per kernel class
   int32_t* ids_stage = nullptr;                 // [max_batch]
   bool exec_end_w_valid = false;                // w_img_valid after a replay of step_exec
+  uint32_t* leaf_order = nullptr;   // [slices of 256][V][256] sorted examples of a batch per variable (leaf statistics)
   float* ll_tmp = nullptr;                      // [max_batch] per-example log-likelihoods of a multi-head step
   // tensor maps over mars / flows for the copy-fed edge-statistics kernel (128-byte opaque objects)
   alignas(64) unsigned char tm[3][128];
