@@ -33,6 +33,8 @@ constexpr uint32_t MAX_DIM = 512;
 constexpr uint32_t RSTEP = TPB / 8;
 constexpr uint32_t XP = EX + 8;  // pitch of the value tile and of the weights on the way down: the four rows and eight
 constexpr uint32_t WPD = OUT + 8;   // columns that the lanes of an operand fragment read lie in 32 different banks
+// 96 latents at 1024 examples 654 (tensor-core kernel) against 682 us a step, 128 at 2048 1134 against 1228 us
+constexpr uint32_t EDGE_NARROW_DIM = 64;
 constexpr uint32_t SPARSE = 128; // threads on one node outside the blocks: 512 examples
 
 struct ChainArgs {
@@ -339,6 +341,103 @@ __global__ void __launch_bounds__(TPB, BATCH <= 2 ? 4 : 2) chain_down_kernel(Cha
   }
 }
 
+// Edge statistics of narrow blocks: aggr[r][t] += exp(theta[r][t]) * sum_b G[r][b] X[t][b] with
+// G = flows[r] * exp(mx - mars[r]), X = exp(M[t] - mx).  pcb_dense_edge.cu works in tiles of 128 x 256 outputs, of which
+// a block of 32 latents fills a thirtieth; here a CTA owns 64 x 64 outputs of one block in registers (mma.sync, operands
+// as above) and walks its share of the examples in tiles of 32, the rows of the next tile in flight.  Bound: HBM (four
+// rows per latent and example).  2159 blocks of 32 x 32 at 512 examples: 576 -> 317 us (beside the chain).
+constexpr uint32_t EP = EX + 4;   // pitch of both operand tiles: eight rows x four examples of a fragment in 32 banks
+__global__ void __launch_bounds__(TPB, 2) edge_narrow_kernel(
+    const float* __restrict__ mars, const float* __restrict__ flows, const float* __restrict__ blk_mx,
+    const float* __restrict__ theta, float* __restrict__ aggr, const PcbDenseBlock* __restrict__ blocks, uint32_t ld, uint32_t B,
+    uint32_t rchunks, uint32_t cchunks, uint32_t slices) {
+  __shared__ __align__(16) float gs[2][OUT * EP], xs[2][OUT * EP];
+  const uint32_t slice = blockIdx.x % slices, c2 = blockIdx.x / slices % cchunks, rest = blockIdx.x / (slices * cchunks);
+  const PcbDenseBlock k = blocks[rest / rchunks];
+  const uint32_t r0 = rest % rchunks * OUT, t0 = c2 * OUT;
+  if (r0 >= k.R || t0 >= k.K) return;
+  const uint32_t rows = min(OUT, k.R - r0), cols = min(OUT, k.K - t0);
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = threadIdx.x & 7, g = threadIdx.x >> 3;
+  const uint32_t tiles = (B + EX - 1) / EX;
+  const float* const mxrow = blk_mx + (size_t)k.mx_row * ld;
+  float4 pm[2], pf[2], mc[2], md[2], mx;
+  auto fetch = [&](uint32_t tile) {
+    const uint32_t b = tile * EX + q * 4;
+    mx = ld4(mxrow + b);
+#pragma unroll
+    for (uint32_t u = 0; u < 2; ++u) {
+      const uint32_t r = g + 32 * u;
+      if (r < rows) { pm[u] = ld4(mars + (size_t)(k.p0 + r0 + r) * ld + b); pf[u] = ld4(flows + (size_t)(k.p0 + r0 + r) * ld + b); }
+      if (r < cols) {
+        mc[u] = ld4(mars + (size_t)(k.c0 + t0 + r) * ld + b);
+        md[u] = k.d0 != PCB_NONE ? ld4(mars + (size_t)(k.d0 + t0 + r) * ld + b) : splat(0.0f);
+      }
+    }
+  };
+  float acc[4][4];
+#pragma unroll
+  for (uint32_t j = 0; j < 4; ++j)
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) acc[j][e] = 0.0f;
+  const uint32_t m0 = (warp & 3u) * 16, n0 = (warp >> 2) * 32, hi8 = lane >> 2, lo4 = lane & 3;
+  uint32_t buf = 0;
+  if (slice < tiles) fetch(slice);
+  for (uint32_t tile = slice; tile < tiles; tile += slices, buf ^= 1u) {
+    const uint32_t b = tile * EX + q * 4;
+    // examples past the batch and examples without a possible child count nowhere
+    const bool v0 = b < B && mx.x != -INFINITY, v1 = b + 1 < B && mx.y != -INFINITY, v2 = b + 2 < B && mx.z != -INFINITY,
+               v3 = b + 3 < B && mx.w != -INFINITY;
+#pragma unroll
+    for (uint32_t u = 0; u < 2; ++u) {
+      const uint32_t r = g + 32 * u;
+      float4 y = splat(0.0f), x = splat(0.0f);
+      if (r < rows) {
+        const float4 e = exp4(mx, pm[u]);
+        y = make_float4(v0 ? pf[u].x * e.x : 0.f, v1 ? pf[u].y * e.y : 0.f, v2 ? pf[u].z * e.z : 0.f, v3 ? pf[u].w * e.w : 0.f);
+      }
+      if (r < cols) {
+        const float4 e = exp4(add4(mc[u], md[u]), mx);
+        x = make_float4(v0 ? e.x : 0.f, v1 ? e.y : 0.f, v2 ? e.z : 0.f, v3 ? e.w : 0.f);
+      }
+      st4(&gs[buf][r * EP + q * 4], y);
+      st4(&xs[buf][r * EP + q * 4], x);
+    }
+    if (tile + slices < tiles) fetch(tile + slices);
+    __syncthreads();   // two buffers: a warp that is ahead writes the other one
+    if (m0 < rows && n0 < cols) {
+      const float* const gp = &gs[buf][(m0 + hi8) * EP + lo4];
+      const float* const xp = &xs[buf][(n0 + hi8) * EP + lo4];
+#pragma unroll
+      for (uint32_t e = 0; e < EX; e += 8) {
+        Frag4 a;
+        split(gp[e], a.hi[0], a.lo[0]);
+        split(gp[8 * EP + e], a.hi[1], a.lo[1]);
+        split(gp[e + 4], a.hi[2], a.lo[2]);
+        split(gp[8 * EP + e + 4], a.hi[3], a.lo[3]);
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+          uint32_t bh[2], bl[2];
+          split(xp[8 * j * EP + e], bh[0], bl[0]);
+          split(xp[8 * j * EP + e + 4], bh[1], bl[1]);
+          mma_tf32(acc[j], a.lo, bh[0], bh[1]);
+          mma_tf32(acc[j], a.hi, bl[0], bl[1]);
+          mma_tf32(acc[j], a.hi, bh[0], bh[1]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (uint32_t j = 0; j < 4; ++j)
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) {
+      const uint32_t r = m0 + hi8 + 8 * (e >> 1), t = n0 + 8 * j + 2 * lo4 + (e & 1u);
+      if (r < rows && t < cols) {
+        const size_t p = k.pid0 + (size_t)(r0 + r) * k.K + t0 + t;
+        atomicAdd(aggr + p, __expf(__ldg(theta + p)) * acc[j][e]);
+      }
+    }
+}
+
 // Example tiles shared out over CTAs so that a launch stays about one wave: a CTA keeps its weights over its tiles.
 // `per_tile` CTAs take one tile each; `smem` and `most` (registers) bound the CTAs of an SM.
 uint32_t tile_ctas(uint32_t tiles, uint32_t per_tile, size_t smem, uint32_t most) {
@@ -442,5 +541,23 @@ int32_t pcb_chain_backward(pcb_circuit* c, pcb_workspace* ws, uint32_t step, con
   auto kernel = R <= RSTEP ? chain_down_kernel<1> : R <= 2 * RSTEP ? chain_down_kernel<2> : chain_down_kernel<4>;
   PCB_CUDA(pcb_launch_pdl(kernel, dim3(a.dense_ctas + sparse_ctas), dim3(TPB),
                           smem, st, c->pdl, a, pcb_sparse_down_args(c, ws, hi)));
+  return PCB_OK;
+}
+
+// Edge statistics of dense blocks [o0, o0 + n): true where the narrow kernel takes them.
+bool pcb_edge_narrow_takes(const pcb_circuit* c) {
+  return c->chain && c->max_dense_R <= EDGE_NARROW_DIM && c->max_dense_K <= EDGE_NARROW_DIM;
+}
+
+int32_t pcb_edge_narrow(pcb_circuit* c, pcb_workspace* ws, uint32_t o0, uint32_t n, cudaStream_t st) {
+  const uint32_t rchunks = (c->max_dense_R + OUT - 1) / OUT, cchunks = (c->max_dense_K + OUT - 1) / OUT;
+  const uint32_t tiles = (ws->B + EX - 1) / EX;
+  // two waves of CTAs where the examples allow it
+  const uint32_t slices = std::max(1u, std::min((tiles + 1) / 2, 148 * 4 / std::max(1u, n * rchunks * cchunks)));
+  PCB_REQUIRE((uint64_t)n * rchunks * cchunks * slices <= 0x7fffffffull, "too many dense blocks for one launch");
+  PcbProfScope ps(c, st, PCB_K_DENSE_BWD_EDGE);
+  edge_narrow_kernel<<<n * rchunks * cchunks * slices, TPB, 0, st>>>(ws->mars, ws->flows, ws->blk_mx, c->theta, c->aggr, c->dense + o0,
+                                                                     ws->ld, ws->B, rchunks, cchunks, slices);
+  PCB_CUDA(cudaGetLastError());
   return PCB_OK;
 }

@@ -944,6 +944,7 @@ int32_t pcb_dense_tc_flush_edges(pcb_circuit* c, pcb_workspace* ws, cudaStream_t
     es = c->side;
     c->side_busy = true;
   }
+  if (pcb_edge_narrow_takes(c)) return pcb_edge_narrow(c, ws, o0, n, es);
   if (ws->have_tm) return pcb_dense_edge_launch(c, ws, o0, n, slices, b_per, es);
   for (uint32_t z0 = 0; z0 < n; z0 += 65535) {
     TcArgs a2 = args;

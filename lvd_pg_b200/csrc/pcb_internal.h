@@ -416,6 +416,8 @@ struct PcbHeadInit {
 };
 int32_t pcb_chain_forward(pcb_circuit* c, pcb_workspace* ws, uint32_t step, cudaStream_t st);
 int32_t pcb_chain_backward(pcb_circuit* c, pcb_workspace* ws, uint32_t step, const PcbHeadInit& hi, cudaStream_t st);
+bool pcb_edge_narrow_takes(const pcb_circuit* c);
+int32_t pcb_edge_narrow(pcb_circuit* c, pcb_workspace* ws, uint32_t o0, uint32_t n, cudaStream_t st);
 int32_t pcb_dense_tc_note_edges(pcb_circuit* c, pcb_workspace* ws, uint32_t step, cudaStream_t st);
 int32_t pcb_dense_forward(pcb_circuit* c, pcb_workspace* ws, uint32_t layer, cudaStream_t st);
 int32_t pcb_dense_backward(pcb_circuit* c, pcb_workspace* ws, uint32_t layer, cudaStream_t st);
