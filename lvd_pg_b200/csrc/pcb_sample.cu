@@ -4,8 +4,8 @@
 //    arg-max of key = logp + g(u) (lowest index on ties) picks the edge; a product node passes all
 //    its children on; a leaf does the same arg-max over its categories.  The keys that decide are
 //    fp64 values of the shared host/device routine of include/pcb200_gumbel.h; an fp32 evaluation
-//    with an error bound first removes the entries that cannot win (warp_select64).  One CTA per
-//    sample takes the pending nodes of a round in parallel (sample_hard_cta_kernel); one warp per
+//    with an error bound first removes the entries that cannot win (race, warp_select64).  One CTA per
+//    sample takes the pending edges of a round in parallel (sample_hard_cta_kernel); one warp per
 //    sample with a stack (sample_hard_kernel) serves very wide circuits and the entry point that
 //    allocates nothing.
 //    This is the temperature -> 0 limit of the reference's relaxed sampler
@@ -44,39 +44,25 @@ __device__ __forceinline__ void warp_argmax(double& key, uint32_t& idx) {
   }
 }
 
-// Arg-max of up to 64 Gumbel keys by one warp (entries `lane` and `lane + 32`), with the same result
-// as the fp64 arg-max above, bit for bit, at a fraction of its cost: every key is first evaluated in
-// fp32 together with a bound eps on its distance from the fp64 key; an entry whose upper bound lies
-// below the best lower bound cannot win and drops out.  Almost always a single candidate is left and
-// is the answer; otherwise the fp64 keys of the candidates alone decide (lowest index on ties, as
-// before: an entry that dropped out is strictly below the winner, so it takes no part in a tie).
-// Bound: x = u (1 - 1e-6) + 1e-6 carries a relative error <= 2.4e-7 in fp32, so inner = -log x is off
-// by <= 2.4e-7 (1 + inner) + 1 ulp, g = -log inner by that over inner plus 1 ulp, the sum by 1 ulp more;
-// eps takes four times the total.  Entries whose inner is below 1e-4 (u within 1e-4 of one, where the
-// relative error of inner is no longer small) always stay candidates.
-__device__ __forceinline__ void key32(float lp, float u, float& key, float& eps) {
-  const float x = fmaf(u, 0.999999f, 1e-6f);
-  const float inner = -logf(x);
-  const float g = -logf(inner);
-  key = lp + g;
-  eps = inner < 1e-4f ? INFINITY : 1e-6f * (1.0f / inner + 2.0f + fabsf(g) + fabsf(lp));
-  if (lp == -INFINITY) { key = -INFINITY; eps = 0.0f; }
+// Arg-max of Gumbel keys with the same result as the fp64 arg-max above, bit for bit, at a fraction of its cost.  The
+// key logp - log(-log x) is largest where the race time r = -log x * exp(-logp) is smallest; every entry's r is formed
+// in fp32 with a relative bound eps on its distance from the exact one, and an entry whose lower bound lies above the
+// smallest upper bound cannot win.  Almost always a single candidate is left and is the answer; otherwise the fp64
+// keys of the candidates alone decide (lowest index on ties: an entry that dropped out takes no part in a tie).
+// Bound: x = u (1 - 1e-6) + 1e-6 carries a relative error <= 2.4e-7, __logf an absolute error <= 3.6e-7 on [0.5, 2] and
+// three ulp elsewhere, so inner = -log x is off by 6e-7 / inner + 4e-7; __expf by 2.4e-7 + 1.2e-7 |logp|, the product by
+// 6e-8; eps is four times the sum.  Entries with inner below 1e-4 or exp(-logp) below 1e-30 have no bounds and always
+// stay candidates (lower bound 0, upper bound infinity).
+__device__ __forceinline__ void race(float lp, float u, float& lo, float& hi) {
+  const float inner = -__logf(fmaf(u, 0.999999f, 1e-6f)), inv = __expf(-lp), r = inner * inv;
+  const float eps = __fdividef(2.4e-6f, inner) + 3.2e-6f + 5e-7f * fabsf(lp);
+  const bool none = inner < 1e-4f || inv < 1e-30f;
+  lo = none ? 0.0f : r - r * eps;
+  hi = none ? INFINITY : r + r * eps;
+  if (inv == INFINITY && !none) lo = hi = INFINITY;   // r * eps may be infinite as well: the difference has no value
 }
-__device__ __forceinline__ uint32_t warp_select64(float lp0, float u0, bool v0, float lp1, float u1, bool v1, uint32_t lane,
-                                                  bool exact) {
-  float k0 = -INFINITY, e0 = 0.0f, k1 = -INFINITY, e1 = 0.0f;
-  if (v0) key32(lp0, u0, k0, e0);
-  if (v1) key32(lp1, u1, k1, e1);
-  if (exact) { e0 = INFINITY; e1 = INFINITY; }   // cross-check switch: every entry stays a candidate, fp64 decides
-  // best lower bound over the warp
-  float lo = fmaxf(v0 ? k0 - e0 : -INFINITY, v1 ? k1 - e1 : -INFINITY);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) lo = fmaxf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-  const bool all_impossible = lo == -INFINITY;            // every key is -inf (or unbounded): decide in fp64
-  const bool c0 = v0 && (all_impossible || k0 + e0 >= lo);
-  const bool c1 = v1 && (all_impossible || k1 + e1 >= lo);
-  const uint32_t b0 = __ballot_sync(0xffffffffu, c0), b1 = __ballot_sync(0xffffffffu, c1);
-  if (__popc(b0) + __popc(b1) == 1) return b0 ? (uint32_t)__ffs(b0) - 1u : 32u + (uint32_t)__ffs(b1) - 1u;
+
+__device__ __noinline__ uint32_t warp_exact64(float lp0, float u0, bool c0, float lp1, float u1, bool c1, uint32_t lane) {
   double best = 0.0;
   uint32_t bi = 0xffffffffu;
   if (c0) { best = pcb_gumbel_key(lp0, u0); bi = lane; }
@@ -85,6 +71,53 @@ __device__ __forceinline__ uint32_t warp_select64(float lp0, float u0, bool v0, 
     if (bi == 0xffffffffu || key > best) { best = key; bi = lane + 32; }
   }
   warp_argmax(best, bi);
+  return bi;
+}
+
+// up to 64 entries, `lane` and `lane + 32` (v0, v1: they exist)
+__device__ __forceinline__ uint32_t warp_select64(float lp0, float u0, bool v0, float lp1, float u1, bool v1, uint32_t lane,
+                                                  bool exact) {
+  float lo0 = INFINITY, hi0 = INFINITY, lo1 = INFINITY, hi1 = INFINITY;
+  race(lp0, u0, lo0, hi0);
+  race(lp1, u1, lo1, hi1);
+  // non-negative floats order like their bits; an entry that does not exist, or is not a number, is the largest word
+  const uint32_t best = __reduce_min_sync(0xffffffffu, min(v0 ? __float_as_uint(hi0) : 0xffffffffu, v1 ? __float_as_uint(hi1) : 0xffffffffu));
+  const float top = __uint_as_float(best);
+  bool c0 = v0 && (exact || lo0 <= top), c1 = v1 && (exact || lo1 <= top);
+  uint32_t b0 = __ballot_sync(0xffffffffu, c0), b1 = __ballot_sync(0xffffffffu, c1);
+  if (__popc(b0) + __popc(b1) == 1) return b0 ? (uint32_t)__ffs(b0) - 1u : 32u + (uint32_t)__ffs(b1) - 1u;
+  if (!(b0 | b1)) { c0 = v0; c1 = v1; }   // nothing comparable
+  return warp_exact64(lp0, u0, c0, lp1, u1, c1, lane);
+}
+
+// any number of entries: the bounds are formed twice rather than kept
+template <typename LogP>
+__device__ __forceinline__ uint32_t warp_select(LogP lp, const float* us, uint32_t n, uint32_t lane, bool exact) {
+  uint32_t best = 0xffffffffu;
+  for (uint32_t j = lane; j < n; j += 32) {
+    float lo, hi;
+    race(lp(j), us[j], lo, hi);
+    best = min(best, __float_as_uint(hi));
+  }
+  const float top = __uint_as_float(__reduce_min_sync(0xffffffffu, best));
+  uint32_t left = 0, last = 0;
+  for (uint32_t j = lane; j < n; j += 32) {
+    float lo, hi;
+    race(lp(j), us[j], lo, hi);
+    if (!exact && lo <= top) { ++left; last = j; }
+  }
+  const uint32_t total = __reduce_add_sync(0xffffffffu, left);
+  if (total == 1) return __shfl_sync(0xffffffffu, last, __ffs(__ballot_sync(0xffffffffu, left)) - 1);
+  double key = 0.0;
+  uint32_t bi = 0xffffffffu;
+  for (uint32_t j = lane; j < n; j += 32) {
+    float lo, hi;
+    race(lp(j), us[j], lo, hi);
+    if (total && !(lo <= top)) continue;
+    const double k = pcb_gumbel_key(lp(j), us[j]);
+    if (bi == 0xffffffffu || k > key) { key = k; bi = j; }
+  }
+  warp_argmax(key, bi);
   return bi;
 }
 
@@ -133,8 +166,7 @@ __global__ void sample_hard_kernel(uint32_t S, const float* __restrict__ params,
         off = (uint64_t)lm.x | ((uint64_t)lm.y << 32);
       }
       const float* us = u_leaf + ((size_t)s * V + var) * cmax;
-      double best = 0.0;
-      uint32_t bi = 0xffffffffu;
+      uint32_t bi;
       // fixed leaves keep their log-probs in the circuit, not in the caller's parameter matrix
       if (C <= 64) {
         const bool v0 = lane < C, v1 = lane + 32 < C;
@@ -142,12 +174,7 @@ __global__ void sample_hard_kernel(uint32_t S, const float* __restrict__ params,
         bi = warp_select64(v0 ? lpa(lane) : 0.0f, v0 ? us[lane] : 0.0f, v0, v1 ? lpa(lane + 32) : 0.0f,
                            v1 ? us[lane + 32] : 0.0f, v1, lane, exact);
       } else {
-        for (uint32_t c = lane; c < C; c += 32) {
-          float lp = off < P ? params[ps + pld * (off + c)] : theta[off + c];
-          double key = pcb_gumbel_key(lp, us[c]);
-          if (bi == 0xffffffffu || key > best) { best = key; bi = c; }
-        }
-        warp_argmax(best, bi);
+        bi = warp_select([&](uint32_t c) { return off < P ? params[ps + pld * (off + c)] : theta[off + c]; }, us, C, lane, exact);
       }
       if (lane == 0) x_out[s + (size_t)S * var] = (int32_t)bi;
     } else if (kd == PCB_PRODUCT) {
@@ -174,8 +201,7 @@ __global__ void sample_hard_kernel(uint32_t S, const float* __restrict__ params,
     } else {
       uint32_t e0 = nm.x, cnt = nm.y, pid0 = nm.z;
       const float* us = u_sum + ((size_t)s * R + (nm.w >> 2)) * kmax;
-      double best = 0.0;
-      uint32_t bi = 0xffffffffu;
+      uint32_t bi;
       // the children of this lane's first two edges are fetched with the parameters, not after the
       // arg-max: one dependent load less on the walk's chain
       uint32_t pr0 = PCB_NONE, sb0 = PCB_NONE, pr1 = PCB_NONE, sb1 = PCB_NONE;
@@ -186,11 +212,7 @@ __global__ void sample_hard_kernel(uint32_t S, const float* __restrict__ params,
         bi = warp_select64(v0 ? params[ps + pld * (size_t)(pid0 + lane)] : 0.0f, v0 ? us[lane] : 0.0f, v0,
                            v1 ? params[ps + pld * (size_t)(pid0 + lane + 32)] : 0.0f, v1 ? us[lane + 32] : 0.0f, v1, lane, exact);
       } else {
-        for (uint32_t j = lane; j < cnt; j += 32) {
-          double key = pcb_gumbel_key(params[ps + pld * (size_t)(pid0 + j)], us[j]);
-          if (bi == 0xffffffffu || key > best) { best = key; bi = j; }
-        }
-        warp_argmax(best, bi);
+        bi = warp_select([&](uint32_t j) { return params[ps + pld * (size_t)(pid0 + j)]; }, us, cnt, lane, exact);
       }
       uint32_t pr, sb;
       if (bi < 64) {
@@ -216,18 +238,54 @@ __global__ void sample_hard_kernel(uint32_t S, const float* __restrict__ params,
   }
 }
 
-// The same walk with one CTA per sample: the pending nodes of a sample are roots of sub-circuits over
-// disjoint scopes, so they are independent, and a single warp that visits them one after another
-// spends its time in the dependent loads of each visit (node record -> parameters and noise ->
-// children: ~1.8 us per visit, 1600 visits per sample at 784 variables).  Here the warps of the CTA
-// take the pending nodes of a round in parallel and push what they select to the next round's list
-// (two lists in shared memory, at most one pending node per variable, so V + 2 entries each); the
-// arg-max at a node is the same computation, so the samples are the same bit for bit.
-#ifndef PCB_SAMPLE_CTA_WARPS
-#define PCB_SAMPLE_CTA_WARPS 4
-#endif
-constexpr uint32_t CW = PCB_SAMPLE_CTA_WARPS;   // warps per sample
-__global__ void __launch_bounds__(CW * 32) sample_hard_cta_kernel(
+// The same walk with one CTA per sample: the pending nodes of a sample are roots of sub-circuits over disjoint scopes,
+// so they are independent.  Pending work is a list of EDGES (two lists in shared memory, at most one entry per
+// variable): a warp takes a piece of the round's list with one edge per lane, and the lanes fetch the children and their
+// records together.  Leaves of few categories are decided by their lanes, each on its own; a product's edges go to the
+// next round's list; the sum nodes of the piece are taken one after another by the whole warp, the parameters and noise
+// of the next one on their way, and the edges they select reach the list with one counter update.  The selection is the
+// same computation as in the one-warp walk, so the samples are the same bit for bit.  Bound: instruction issue (two
+// thirds of the slots at 4096 samples).  A warp per node, leaves included, with keys from two logarithms and a maximum
+// by five shuffles: 4096 samples of 784 variables x 64 latents 1573 us, now 450 us; the noise it must read (470 MB) is
+// 72 us of HBM.
+// CW: warps per sample.  One warp fills its lanes best and has nobody to wait for; where the samples alone do not fill
+// the GPU, more warps shorten the walk of each.
+constexpr uint32_t LANE_CATS = 8;               // categories up to which a leaf is decided by one lane
+constexpr uint32_t ROOT_ENTRY = 0xffffffffu;    // the list entry that stands for the root
+
+// one lane's leaf: C categories, at most LANE_CATS
+__device__ __noinline__ uint32_t lane_exact(const float* lp, size_t pld, const float* us, uint32_t C, uint32_t keep) {
+  double best = 0.0;
+  uint32_t bi = 0xffffffffu;
+  for (uint32_t c = 0; c < C; ++c) {
+    if (!((keep >> c) & 1u)) continue;
+    const double key = pcb_gumbel_key(lp[pld * c], us[c]);
+    if (bi == 0xffffffffu || key > best) { best = key; bi = c; }
+  }
+  return bi;
+}
+__device__ __forceinline__ uint32_t lane_select(const float* lp, size_t pld, const float* us, uint32_t C, bool exact) {
+  float lo[LANE_CATS], top = __uint_as_float(0x7f800000u);
+  bool any = false;
+#pragma unroll
+  for (uint32_t c = 0; c < LANE_CATS; ++c) {
+    float hi = INFINITY;
+    lo[c] = INFINITY;
+    if (c < C) {
+      race(lp[pld * c], us[c], lo[c], hi);
+      if (hi <= top) { top = hi; any = true; }
+    }
+  }
+  uint32_t keep = 0;
+#pragma unroll
+  for (uint32_t c = 0; c < LANE_CATS; ++c)
+    if (c < C && (exact || (any && lo[c] <= top))) keep |= 1u << c;
+  if (__popc(keep) == 1) return (uint32_t)__ffs(keep) - 1u;
+  return lane_exact(lp, pld, us, C, keep ? keep : (1u << C) - 1u);
+}
+
+template <uint32_t CW>
+__global__ void __launch_bounds__(CW * 32, CW == 1 ? 32 : 40 / CW) sample_hard_cta_kernel(
     uint32_t S, const float* __restrict__ params, uint32_t Sp, const float* __restrict__ u_sum,
     const float* __restrict__ u_leaf, uint32_t R, uint32_t kmax, uint32_t cmax, uint32_t V, uint32_t N,
     const uint32_t* __restrict__ e_prime, const uint32_t* __restrict__ e_sub, uint64_t P, const float* __restrict__ theta,
@@ -237,97 +295,104 @@ __global__ void __launch_bounds__(CW * 32) sample_hard_cta_kernel(
   __shared__ uint32_t count[2];
   const uint32_t s = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t ps = Sp == 1 ? 0 : s, pld = Sp;
-  for (uint32_t v = threadIdx.x; v < V; v += blockDim.x) x_out[s + (size_t)S * v] = -1;
-  if (threadIdx.x == 0) { lists[0] = N - 1; count[0] = 1; count[1] = 0; }
+  if (threadIdx.x == 0) { lists[0] = ROOT_ENTRY; count[0] = 1; count[1] = 0; }
   __syncthreads();
   uint32_t cur = 0;
   for (uint32_t round = 0;; ++round) {
     const uint32_t n_cur = count[cur];
-    if (n_cur == 0) break;
+    if (n_cur == 0 || n_cur > cap) break;   // more than the list holds: the status word says so
     if (round > N + 8u) {   // a circuit is at most N levels deep
       if (threadIdx.x == 0) atomicMax(status, 2);
       break;
     }
     __syncthreads();                       // every thread has read the count
     if (threadIdx.x == 0) count[cur] = 0;  // this list is the next round's target after the one being filled
-    uint32_t* out = lists + (cur ^ 1u) * cap;
-    uint32_t* out_n = &count[cur ^ 1u];
-    for (uint32_t idx = warp; idx < n_cur; idx += CW) {
-      const uint32_t n = lists[cur * cap + idx];
-      const uint4 nm = s_node[n];
-      const uint8_t kd = (uint8_t)(nm.w & 3u);
-      if (kd == PCB_INPUT) {
-        uint32_t C = nm.y & 0xffffu, var = nm.y >> 16;
-        uint64_t off = nm.x;
-        if (nm.x == 0xffffffffu) {
-          const uint4 lm = s_leaf[nm.z];
-          C = lm.z; var = lm.w;
-          off = (uint64_t)lm.x | ((uint64_t)lm.y << 32);
+    uint32_t* const out = lists + (cur ^ 1u) * cap;
+    uint32_t* const out_n = &count[cur ^ 1u];
+    const uint32_t per = min(32u, (n_cur + CW - 1) / CW);   // edges of a warp's piece
+    for (uint32_t base = warp * per; base < n_cur; base += CW * per) {
+      const bool has = lane < per && base + lane < n_cur;
+      const uint32_t entry = has ? lists[cur * cap + base + lane] : 0u;
+      uint32_t prime = PCB_NONE, sub = PCB_NONE;
+      if (has) {
+        if (entry == ROOT_ENTRY) prime = N - 1;
+        else { prime = e_prime[entry]; sub = e_sub[entry]; }
+      }
+#pragma unroll 1
+      for (uint32_t half = 0; half < 2; ++half) {
+        const uint32_t n = half ? sub : prime;
+        const uint4 nm = n != PCB_NONE ? s_node[n] : make_uint4(0, 0, 0, 3u);
+        const uint32_t kd = nm.w & 3u;
+        if (kd == PCB_INPUT) {
+          uint32_t C = nm.y & 0xffffu, var = nm.y >> 16;
+          uint64_t off = nm.x;
+          if (nm.x == 0xffffffffu) {
+            const uint4 lm = s_leaf[nm.z];
+            C = lm.z; var = lm.w;
+            off = (uint64_t)lm.x | ((uint64_t)lm.y << 32);
+          }
+          if (C <= LANE_CATS) {
+            // fixed leaves keep their log-probs in the circuit, not in the caller's parameter matrix
+            const float* lp = off < P ? params + ps + pld * off : theta + off;
+            x_out[s + (size_t)S * var] = (int32_t)lane_select(lp, off < P ? pld : 1, u_leaf + ((size_t)s * V + var) * cmax, C, exact);
+          }
+        } else if (kd == PCB_PRODUCT) {
+          const uint32_t pos = atomicAdd(out_n, nm.y);
+          if (pos + nm.y > cap) atomicMax(status, 1);
+          else for (uint32_t j = 0; j < nm.y; ++j) out[pos + j] = nm.x + j;
         }
-        const float* us = u_leaf + ((size_t)s * V + var) * cmax;
-        double best = 0.0;
-        uint32_t bi = 0xffffffffu;
-        if (C <= 64) {
-          const bool v0 = lane < C, v1 = lane + 32 < C;
+        // leaves of many categories: a warp each
+        const uint32_t my_cats = kd != PCB_INPUT ? 0u : nm.x == 0xffffffffu ? s_leaf[nm.z].z : nm.y & 0xffffu;
+        for (uint32_t m = __ballot_sync(0xffffffffu, my_cats > LANE_CATS); m; m &= m - 1) {
+          const uint32_t src = (uint32_t)__ffs(m) - 1u;
+          const uint32_t ex = __shfl_sync(0xffffffffu, nm.x, src), ey = __shfl_sync(0xffffffffu, nm.y, src), ez = __shfl_sync(0xffffffffu, nm.z, src);
+          uint32_t C = ey & 0xffffu, var = ey >> 16;
+          uint64_t off = ex;
+          if (ex == 0xffffffffu) {
+            const uint4 lm = s_leaf[ez];
+            C = lm.z; var = lm.w;
+            off = (uint64_t)lm.x | ((uint64_t)lm.y << 32);
+          }
+          const float* us = u_leaf + ((size_t)s * V + var) * cmax;
           auto lpa = [&](uint32_t c) { return off < P ? params[ps + pld * (off + c)] : theta[off + c]; };
-          bi = warp_select64(v0 ? lpa(lane) : 0.0f, v0 ? us[lane] : 0.0f, v0, v1 ? lpa(lane + 32) : 0.0f,
-                             v1 ? us[lane + 32] : 0.0f, v1, lane, exact);
-        } else {
-          for (uint32_t c = lane; c < C; c += 32) {
-            float lp = off < P ? params[ps + pld * (off + c)] : theta[off + c];
-            double key = pcb_gumbel_key(lp, us[c]);
-            if (bi == 0xffffffffu || key > best) { best = key; bi = c; }
-          }
-          warp_argmax(best, bi);
+          const uint32_t bi = warp_select(lpa, us, C, lane, exact);
+          if (lane == 0) x_out[s + (size_t)S * var] = (int32_t)bi;
         }
-        if (lane == 0) x_out[s + (size_t)S * var] = (int32_t)bi;
-      } else if (kd == PCB_PRODUCT) {
-        const uint32_t e0 = nm.x, cnt = nm.y;
-        for (uint32_t j = lane; j < cnt; j += 32) {
-          const uint32_t pr = e_prime[e0 + j], sb = e_sub[e0 + j];
-          const uint32_t np = sb != PCB_NONE ? 2u : 1u;
-          const uint32_t pos = atomicAdd(out_n, np);
-          if (pos + np > cap) { atomicMax(status, 1); continue; }
-          out[pos] = pr;
-          if (sb != PCB_NONE) out[pos + 1] = sb;
-        }
-      } else {
-        const uint32_t e0 = nm.x, cnt = nm.y, pid0 = nm.z;
-        const float* us = u_sum + ((size_t)s * R + (nm.w >> 2)) * kmax;
-        double best = 0.0;
-        uint32_t bi = 0xffffffffu;
-        uint32_t pr0 = PCB_NONE, sb0 = PCB_NONE, pr1 = PCB_NONE, sb1 = PCB_NONE;
-        if (lane < cnt) { pr0 = e_prime[e0 + lane]; sb0 = e_sub[e0 + lane]; }
-        if (lane + 32 < cnt) { pr1 = e_prime[e0 + lane + 32]; sb1 = e_sub[e0 + lane + 32]; }
-        if (cnt <= 64) {
-          const bool v0 = lane < cnt, v1 = lane + 32 < cnt;
-          bi = warp_select64(v0 ? params[ps + pld * (size_t)(pid0 + lane)] : 0.0f, v0 ? us[lane] : 0.0f, v0,
-                             v1 ? params[ps + pld * (size_t)(pid0 + lane + 32)] : 0.0f, v1 ? us[lane + 32] : 0.0f, v1, lane, exact);
-        } else {
-          for (uint32_t j = lane; j < cnt; j += 32) {
-            double key = pcb_gumbel_key(params[ps + pld * (size_t)(pid0 + j)], us[j]);
-            if (bi == 0xffffffffu || key > best) { best = key; bi = j; }
-          }
-          warp_argmax(best, bi);
-        }
-        uint32_t pr, sb;
-        if (bi < 64) {
-          const uint32_t src = bi & 31u;
-          pr = __shfl_sync(0xffffffffu, bi < 32 ? pr0 : pr1, src);
-          sb = __shfl_sync(0xffffffffu, bi < 32 ? sb0 : sb1, src);
-        } else {
-          pr = e_prime[e0 + bi]; sb = e_sub[e0 + bi];
-        }
-        if (lane == 0) {
-          const uint32_t np = sb != PCB_NONE ? 2u : 1u;
-          const uint32_t pos = atomicAdd(out_n, np);
-          if (pos + np > cap) {
-            atomicMax(status, 1);
+        // sum nodes, the operands of the next one in flight
+        uint32_t m = __ballot_sync(0xffffffffu, kd == PCB_SUM);
+        if (!m) continue;
+        const uint32_t sums = m, mine = __popc(m & ((1u << lane) - 1u));
+        uint32_t picked = 0;
+        float lp0 = 0.f, u0 = 0.f, lp1 = 0.f, u1 = 0.f;
+        auto fetch = [&](uint32_t src) {
+          const uint32_t cnt = __shfl_sync(0xffffffffu, nm.y, src), pid = __shfl_sync(0xffffffffu, nm.z, src);
+          const uint32_t reg = __shfl_sync(0xffffffffu, nm.w, src) >> 2;
+          const float* us = u_sum + ((size_t)s * R + reg) * kmax;
+          const float* pp = params + ps + pld * (size_t)pid;
+          if (lane < cnt) { lp0 = pp[pld * lane]; u0 = __ldcs(us + lane); }
+          if (lane + 32 < cnt) { lp1 = pp[pld * (lane + 32)]; u1 = __ldcs(us + lane + 32); }
+        };
+        fetch((uint32_t)__ffs(m) - 1u);
+        while (m) {
+          const uint32_t src = (uint32_t)__ffs(m) - 1u;
+          m &= m - 1;
+          const uint32_t cnt = __shfl_sync(0xffffffffu, nm.y, src);
+          const float a0 = lp0, b0 = u0, a1 = lp1, b1 = u1;
+          if (m) fetch((uint32_t)__ffs(m) - 1u);
+          uint32_t bi;
+          if (cnt <= 64) {
+            bi = warp_select64(a0, b0, lane < cnt, a1, b1, lane + 32 < cnt, lane, exact);
           } else {
-            out[pos] = pr;
-            if (sb != PCB_NONE) out[pos + 1] = sb;
+            const uint32_t pid = __shfl_sync(0xffffffffu, nm.z, src), reg = __shfl_sync(0xffffffffu, nm.w, src) >> 2;
+            bi = warp_select([&](uint32_t j) { return params[ps + pld * (size_t)(pid + j)]; }, u_sum + ((size_t)s * R + reg) * kmax, cnt, lane, exact);
           }
+          if (lane == src) picked = nm.x + bi;
         }
+        uint32_t pos = 0;
+        if (lane == 0) pos = atomicAdd(out_n, (uint32_t)__popc(sums));
+        pos = __shfl_sync(0xffffffffu, pos, 0);
+        if (pos + __popc(sums) > cap) { if (lane == 0) atomicMax(status, 1); }
+        else if ((sums >> lane) & 1u) out[pos + mine] = picked;
       }
     }
     __syncthreads();   // the next list is complete
@@ -335,8 +400,6 @@ __global__ void __launch_bounds__(CW * 32) sample_hard_cta_kernel(
   }
 }
 
-// ---- soft sampling ------------------------------------------------------------------------------
-// unnormalised relaxed edge probabilities and their per-node sums; cum is stored per sum NODE
 // ---- relaxed sampling: exp((log p + gumbel) / T) of every sum edge, normalised per sum node ------------------
 // The keys are formed in fp64 like the reference's (sample.jl:24-54 promotes through its Float64 literals), with
 // logarithm and exponential by table and short polynomial (P. T. P. Tang, ACM TOMS 15 (1989) and 16 (1990)): the
@@ -560,10 +623,19 @@ extern "C" int32_t pcb_sample_hard(pcb_circuit* c, pcb_workspace* ws, const floa
   PCB_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), st));
   if (cta_walk) {
     // one CTA per sample, its warps sharing the rounds of pending nodes
+    PCB_CUDA(cudaMemsetAsync(x_out_dev, 0xff, (size_t)S * c->V * sizeof(int32_t), st));   // -1: a variable the walk does not reach
     ++c->prof.launches[PCB_K_SAMPLE];
-    sample_hard_cta_kernel<<<S, CW * 32, (size_t)2 * ws->stack_cap * 4, st>>>(
-        S, params_dev, Sp, u_sum_dev, u_leaf_dev, c->n_regions, c->max_group, c->max_cats, c->V, c->N, c->e_prime, c->e_sub,
-        c->P, c->theta, ws->stack_cap, x_out_dev, status, c->s_node, c->s_leaf, c->sample_exact_keys);
+    auto walk = [&](auto* kernel, uint32_t warps) {
+      kernel<<<S, warps * 32, (size_t)2 * ws->stack_cap * 4, st>>>(
+          S, params_dev, Sp, u_sum_dev, u_leaf_dev, c->n_regions, c->max_group, c->max_cats, c->V, c->N, c->e_prime, c->e_sub,
+          c->P, c->theta, ws->stack_cap, x_out_dev, status, c->s_node, c->s_leaf, c->sample_exact_keys);
+    };
+    // warps per sample, 784 variables x 64 latents, us with 1 / 2 / 4 / 8: 4096 samples 512 / 629 / 664 / 912, 2048 samples
+    // 412 / 367 / 407 / 494, 1024 samples 396 / 295 / 243 / 320, 512 samples 376 / 269 / 199 / 187
+    if (S >= 148 * 16) walk(sample_hard_cta_kernel<1>, 1);
+    else if (S >= 148 * 10) walk(sample_hard_cta_kernel<2>, 2);
+    else if (S >= 148 * 5) walk(sample_hard_cta_kernel<4>, 4);
+    else walk(sample_hard_cta_kernel<8>, 8);
     PCB_CUDA(cudaGetLastError());
     int32_t h0 = 0;
     PCB_CUDA(cudaMemcpyAsync(&h0, status, sizeof(int32_t), cudaMemcpyDeviceToHost, st));

@@ -1,0 +1,33 @@
+"""Hard samples bit for bit against the oracle for every number of warps per sample, leaves that a lane or a warp decides,
+nodes of more edges than a warp holds, one parameter set and one per sample, and parameters without bounds."""
+import numpy as np
+import pytest
+
+from tests.helpers import random_hclt
+from tests.test_gpu_kld_sample import _cuda, _param_sets
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("v,k,c,S,per_sample", [
+    (12, 16, 2, 1, False), (40, 20, 8, 800, False), (30, 17, 9, 1500, False), (9, 70, 70, 2400, False), (5, 150, 3, 300, False),
+    (7, 64, 300, 40, False), (12, 33, 4, 50, True)])
+@pytest.mark.parametrize("extreme", [False, True])
+def test_samples_equal_the_oracle(oracle, v, k, c, S, per_sample, extreme):
+    torch, api = _cuda()
+    fc = random_hclt(v, k, c, v + k)
+    m = api.CuMetaBitsProbCircuit(fc)
+    p = _param_sets(oracle, fc, S if per_sample else 1, 1)
+    rng = np.random.default_rng(k)
+    shp = api.noise_shapes(m, S)
+    u_sum, u_leaf = rng.random(shp[0], dtype=np.float32), rng.random(shp[1], dtype=np.float32)
+    if extreme:   # certain and impossible edges, tiny and huge weights, noise at both ends and ties
+        p.reshape(-1)[::7] = -np.inf
+        p.reshape(-1)[::11] = -100.0
+        p.reshape(-1)[::13] = 80.0
+        for u in (u_sum, u_leaf):
+            u.reshape(-1)[::5] = 1 - 2.0 ** -24
+            u.reshape(-1)[::6] = 0.0
+            u.reshape(-1)[::3] = 0.5
+    x = api.sample(m, p if per_sample else p[0], u_sum, u_leaf).cpu().numpy()
+    assert np.array_equal(x, oracle.sample_hard(fc, p if per_sample else p[0], u_sum, u_leaf, S))
