@@ -278,7 +278,7 @@ int32_t compile(const pcb_circuit_desc* d, pcb_circuit* c) {
   c->h_dense_off[c->L + 1] = (uint32_t)c->h_dense.size();
   c->n_dense = (uint32_t)c->h_dense.size();
 
-  // ---- the steps of an EM pass ----------------------------------------------------------------
+  // ---- the steps of a pass ----------------------------------------------------------------
   // The up layers count a product layer below every block of sums, but a block whose prime children are products of
   // consecutive, exclusive runs of nodes can form those products itself (their values are sums of the runs' values,
   // and their flows are the runs' flows).  Without these fused products a circuit has about half as many dependent
@@ -329,10 +329,6 @@ int32_t compile(const pcb_circuit_desc* d, pcb_circuit* c) {
       step[n] = fused[n] ? top : top + 1;
       c->n_steps = std::max(c->n_steps, step[n]);
     }
-  // blocks by up layer for the passes over parameter sets, by step for the EM passes
-  std::vector<PcbDenseBlock> by_layer_blocks = c->h_dense;
-  c->h_layer_dense = by_layer_blocks;
-  c->h_layer_dense_off = c->h_dense_off;
   std::stable_sort(c->h_dense.begin(), c->h_dense.end(),
                    [&](const PcbDenseBlock& x, const PcbDenseBlock& y) { return step[x.p0] < step[y.p0]; });
   const uint32_t T = c->n_steps;
@@ -384,47 +380,21 @@ int32_t compile(const pcb_circuit_desc* d, pcb_circuit* c) {
   flatten(sources, st_src, c->h_st_src_off);
 
   // ---- layer lists --------------------------------------------------------------------------
-  std::vector<uint32_t> up_all, up_sparse, down_all, down_sparse;
-  c->h_up_all_off.assign(c->L + 1, 0); c->h_up_sparse_off.assign(c->L + 1, 0);
+  std::vector<uint32_t> up_all, down_all;
+  c->h_up_all_off.assign(c->L + 1, 0);
   for (uint32_t lay = 1; lay <= c->L; ++lay) {
     c->h_up_all_off[lay - 1] = (uint32_t)up_all.size();
-    c->h_up_sparse_off[lay - 1] = (uint32_t)up_sparse.size();
-    for (uint32_t n : layer_nodes[lay]) { up_all.push_back(n); if (!in_dense[n]) up_sparse.push_back(n); }
+    for (uint32_t n : layer_nodes[lay]) up_all.push_back(n);
   }
   c->h_up_all_off[c->L] = (uint32_t)up_all.size();
-  c->h_up_sparse_off[c->L] = (uint32_t)up_sparse.size();
-  // Chunks of eight consecutive nodes of a layer list whose edges lead to the same children in the
-  // same order (the k sums of one HCLT variable do): a top-down pass that pushes to the children
-  // adds the eight contributions in shared memory first.
-  std::vector<uint8_t> up_same;
-  c->h_up_chunk_off.assign(c->L + 1, 0);
-  for (uint32_t lay = 1; lay <= c->L; ++lay) {
-    c->h_up_chunk_off[lay - 1] = (uint32_t)up_same.size();
-    const uint32_t o0 = c->h_up_all_off[lay - 1], o1 = c->h_up_all_off[lay];
-    for (uint32_t b = o0; b < o1; b += 8) {
-      const uint32_t first = up_all[b];
-      bool same = kind[first] == PCB_SUM && ecount[first] <= 256;
-      for (uint32_t i = b + 1; same && i < std::min(o1, b + 8); ++i) {
-        const uint32_t n = up_all[i];
-        same = kind[n] == PCB_SUM && ecount[n] == ecount[first] &&
-               !memcmp(&d->up_prime[estart[n]], &d->up_prime[estart[first]], ecount[n] * sizeof(uint32_t)) &&
-               !memcmp(&d->up_sub[estart[n]], &d->up_sub[estart[first]], ecount[n] * sizeof(uint32_t));
-      }
-      up_same.push_back(same ? 1 : 0);
-    }
-  }
-  c->h_up_chunk_off[c->L] = (uint32_t)up_same.size();
-  if (up_same.empty()) up_same.push_back(0);
   std::vector<std::vector<uint32_t>> by_layer(c->L + 1);
   for (uint32_t n = 0; n < N; ++n) by_layer[layer[n]].push_back(n);
-  c->h_down_all_off.assign(c->L + 2, 0); c->h_down_sparse_off.assign(c->L + 2, 0);
+  c->h_down_all_off.assign(c->L + 2, 0);
   for (uint32_t lay = 0; lay <= c->L; ++lay) {
     c->h_down_all_off[lay] = (uint32_t)down_all.size();
-    c->h_down_sparse_off[lay] = (uint32_t)down_sparse.size();
-    for (uint32_t n : by_layer[lay]) { down_all.push_back(n); if (!dense_child[n]) down_sparse.push_back(n); }
+    for (uint32_t n : by_layer[lay]) down_all.push_back(n);
   }
   c->h_down_all_off[c->L + 1] = (uint32_t)down_all.size();
-  c->h_down_sparse_off[c->L + 1] = (uint32_t)down_sparse.size();
 
   // ---- upload ---------------------------------------------------------------------------------
   std::vector<uint32_t> e_prime(E), e_sub(E);
@@ -475,10 +445,7 @@ int32_t compile(const pcb_circuit_desc* d, pcb_circuit* c) {
   PCB_TRY(upload(&c->n_head, node_head, &bytes));
   PCB_TRY(upload(&c->head_roots, c->h_head_roots, &bytes));
   PCB_TRY(upload(&c->up_all, up_all, &bytes));
-  PCB_TRY(upload(&c->up_same, up_same, &bytes));
-  PCB_TRY(upload(&c->up_sparse, up_sparse, &bytes));
   PCB_TRY(upload(&c->down_all, down_all, &bytes));
-  PCB_TRY(upload(&c->down_sparse, down_sparse, &bytes));
   PCB_TRY(upload(&c->in_off, in_off, &bytes));
   PCB_TRY(upload(&c->in_ent, in_ent, &bytes));
   PCB_TRY(upload(&c->dense, c->h_dense, &bytes));
@@ -493,14 +460,13 @@ int32_t compile(const pcb_circuit_desc* d, pcb_circuit* c) {
       if (bytes_of) memcpy(pack.data() + at, src, bytes_of);
       return at;
     };
-    const size_t o_ld = put(c->h_layer_dense.data(), c->h_layer_dense.size() * sizeof(PcbDenseBlock));
     const size_t o_th = put(c->h_thin.data(), c->h_thin.size() * sizeof(PcbDenseBlock));
     const size_t o_sl = put(src_list.data(), src_list.size() * 4), o_up = put(st_up.data(), st_up.size() * 4);
     const size_t o_dn = put(st_down.data(), st_down.size() * 4), o_pr = put(st_prod.data(), st_prod.size() * 4);
     const size_t o_sr = put(st_src.data(), st_src.size() * 4), o_lo = put(loose.data(), loose.size() * 4);
     PCB_TRY(upload(&c->step_tables, pack, &bytes));
     uint32_t* const t = c->step_tables;
-    c->layer_dense = reinterpret_cast<PcbDenseBlock*>(t + o_ld); c->thin = reinterpret_cast<PcbDenseBlock*>(t + o_th);
+    c->thin = reinterpret_cast<PcbDenseBlock*>(t + o_th);
     c->src_list = t + o_sl; c->st_up = t + o_up; c->st_down = t + o_dn; c->st_prod = t + o_pr; c->st_src = t + o_sr;
     c->grp_loose = t + o_lo;
   }
@@ -586,9 +552,9 @@ namespace {
 void free_circuit(pcb_circuit* c) {
   void* ptrs[] = {c->theta, c->aggr, c->kind, c->n_estart, c->n_ecount, c->n_pid0, c->n_region, c->e_prime,
                   c->e_sub, c->in_node, c->in_var, c->in_cats, c->in_poff, c->in_foff, c->node2input,
-                  c->up_all, c->up_sparse, c->down_all, c->down_sparse, c->in_off, c->in_ent, c->dense,
+                  c->up_all, c->down_all, c->in_off, c->in_ent, c->dense,
                   c->grp_node, c->step_tables, c->lchunk_var, c->lchunk_off, c->lchunk_inputs, c->status, c->w_img, c->dense_img, c->w_img16, c->dense_img16,
-                  c->lgrp_var, c->lgrp_off, c->s_node, c->s_leaf, c->n_head, c->head_roots, c->up_same, c->var_cats, c->check_word};
+                  c->lgrp_var, c->lgrp_off, c->s_node, c->s_leaf, c->n_head, c->head_roots, c->var_cats, c->check_word};
   for (void* p : ptrs) if (p) cudaFree(p);
   if (c->ev_g0) cudaEventDestroy(c->ev_g0);
   if (c->ev_g1) cudaEventDestroy(c->ev_g1);

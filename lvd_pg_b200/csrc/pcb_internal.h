@@ -125,21 +125,16 @@ struct pcb_circuit {
   uint32_t* lgrp_var = nullptr;
   uint32_t* lgrp_off = nullptr;
   uint32_t n_lgrps = 0;
-  // layer lists: all inner nodes by layer / only those outside dense blocks
+  // layer lists: all inner nodes by layer, every node by layer
   uint32_t* up_all = nullptr;     // [n_inner_nodes]
-  uint8_t* up_same = nullptr;     // per chunk of 8 entries of a layer of up_all: same children in the same order
-  std::vector<uint32_t> h_up_chunk_off;   // [L+1] first chunk of a layer (index = layer-1)
-  uint32_t* up_sparse = nullptr;
   uint32_t* down_all = nullptr;   // [N] every node, by layer
-  uint32_t* down_sparse = nullptr;
   uint32_t* in_off = nullptr;     // [N+1] CSR by child
   PcbInEntry* in_ent = nullptr;
   PcbDenseBlock* dense = nullptr; // sorted by step
-  PcbDenseBlock* layer_dense = nullptr;   // the same sorted by parent layer
-  // the steps of an EM pass (1 .. n_steps): blocks with their fused products, thin blocks (single sum nodes over
+  // the steps of a pass (1 .. n_steps): blocks with their fused products, thin blocks (single sum nodes over
   // consecutive children, upward only) and nodes taken one by one
   uint32_t n_steps = 0;
-  uint32_t* step_tables = nullptr;   // the allocation that holds the tables below, layer_dense and grp_loose
+  uint32_t* step_tables = nullptr;   // the allocation that holds the tables below and grp_loose
   PcbDenseBlock* thin = nullptr;
   uint32_t* src_list = nullptr;   // [count, runs ...] per fused block
   uint32_t* st_up = nullptr;      // nodes a step computes one by one (thin blocks' nodes last)
@@ -151,12 +146,11 @@ struct pcb_circuit {
   uint32_t n_grp_loose = 0;
 
   // ---- host copies of the small per-layer tables ----
-  std::vector<uint32_t> h_up_all_off, h_up_sparse_off;      // [L+1] (index = layer-1)
-  std::vector<uint32_t> h_down_all_off, h_down_sparse_off;  // [L+2] (index = layer)
+  std::vector<uint32_t> h_up_all_off;      // [L+1] (index = layer-1)
+  std::vector<uint32_t> h_down_all_off;  // [L+2] (index = layer)
   std::vector<uint32_t> h_dense_off;                        // [n_steps+2] blocks by step
   std::vector<PcbDenseBlock> h_dense;
-  std::vector<uint32_t> h_layer_dense_off;                  // [L+2] blocks by parent layer
-  std::vector<PcbDenseBlock> h_layer_dense, h_thin;
+  std::vector<PcbDenseBlock> h_thin;
   std::vector<uint32_t> h_st_up_off, h_st_down_off, h_st_prod_off, h_st_src_off, h_st_thin_off;   // [n_steps+2]
   uint64_t chain_macs = 0;      // PCB_CHAIN_MACS: cost limit of the fp32 chain kernels (0: the built-in rule, ~0: always)
   bool chain = true;            // PCB_CHAIN=0: dense blocks always on the tensor cores
@@ -389,13 +383,13 @@ __device__ __forceinline__ void pcb_copy16_async(float* dst, const float* src) {
 __device__ __forceinline__ void pcb_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 #endif
 
-// the dense blocks whose parents lie in layer `lay`, and the largest row and child count over them
-static inline uint32_t pcb_layer_blocks(const pcb_circuit* c, uint32_t lay) {
-  return lay >= 1 && lay <= c->L ? c->h_layer_dense_off[lay + 1] - c->h_layer_dense_off[lay] : 0;
+// the dense blocks of a step, and the largest row and child count over them
+static inline uint32_t pcb_step_blocks(const pcb_circuit* c, uint32_t t) {
+  return t >= 1 && t <= c->n_steps ? c->h_dense_off[t + 1] - c->h_dense_off[t] : 0;
 }
-static inline void pcb_layer_extent(const pcb_circuit* c, uint32_t lay, uint32_t& R, uint32_t& K) {
-  for (uint32_t i = 0; i < pcb_layer_blocks(c, lay); ++i) {
-    const PcbDenseBlock& b = c->h_layer_dense[c->h_layer_dense_off[lay] + i];
+static inline void pcb_step_extent(const pcb_circuit* c, uint32_t t, uint32_t& R, uint32_t& K) {
+  for (uint32_t i = 0; i < pcb_step_blocks(c, t); ++i) {
+    const PcbDenseBlock& b = c->h_dense[c->h_dense_off[t] + i];
     R = b.R > R ? b.R : R; K = b.K > K ? b.K : K;
   }
 }

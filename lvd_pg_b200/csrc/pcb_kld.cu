@@ -123,14 +123,19 @@ __global__ void __launch_bounds__(256) param_columns_kernel(float* __restrict__ 
 // in flight, the widest layer ran at 1.6 TB/s).  The values of the neighbouring layer are staged for the whole CTA
 // in one batch of loads after the wait, so a small layer costs one L2 round trip.  Dense blocks
 // (children c0.., d0.. consecutive) need no edge list; the other nodes of the layer ride in the same launch.
-// 784 variables x 64 latents x 24 sets: upward 1164 -> 185 us, downward 1726 -> 207 us (19 layers each).
+// The launches follow the steps of the EM passes: a fused product is read as the sum of its sources by the block above
+// it (three of them in flight; one at a time the upward pass took 236 us), so the chain has 11 launches instead of 19.
+// 784 variables x 64 latents x 24 sets: upward 1164 -> 185 us over layers, 194 over steps; downward 1726 -> 207 -> 187 us.
+// One set, both passes: 180 -> 155 us.
 constexpr uint32_t KLD_THREADS = 256, KLD_SLOTS = 32;   // steps parked per thread; further ones are read directly
 constexpr uint32_t KLD_STAGE = 8 * KLD_THREADS;         // staged values of the neighbouring layer (floats)
 
 struct KldLayer {
   float* klds; float* grads; const float* p1; const float* p2; float* g1; float* g2;
   uint32_t ld, S, St;                    // sets, sets per tile (blockIdx.y)
-  const PcbDenseBlock* blk; uint32_t per_blk, dense_ctas, rows;   // CTAs per block; rows (up) / children (down) of one
+  const PcbDenseBlock* blk; const PcbDenseBlock* thin; uint32_t nblk;   // thin: single sum nodes (up only), after the blocks
+  const uint32_t* src_list;
+  uint32_t per_blk, dense_ctas, rows;    // CTAs per block; rows (up) / children (down) of one
   uint32_t slots;
   const uint32_t* nodes; uint32_t count; // nodes outside dense blocks
   const uint8_t* kind; const uint32_t* n_estart; const uint32_t* n_ecount; const uint32_t* n_pid0;
@@ -141,12 +146,17 @@ struct KldLayer {
 __global__ void __launch_bounds__(KLD_THREADS) kld_up_layer_kernel(KldLayer a) {
   extern __shared__ float park[];   // [slots][p1 | p2][threads], then the staged values
   __shared__ float red[KLD_THREADS];
+  __shared__ uint32_t src[PCB_MAX_SOURCES];
   pcb_grid_dep_launch();
   const uint32_t s0 = blockIdx.y * a.St, St = min(a.St, a.S - s0), J = KLD_THREADS / a.St;
   const uint32_t q = threadIdx.x / a.St, s = threadIdx.x % a.St;
   if (blockIdx.x < a.dense_ctas) {
-    const PcbDenseBlock b = a.blk[blockIdx.x / a.per_blk];
+    const uint32_t bi = blockIdx.x / a.per_blk;
+    const PcbDenseBlock b = bi < a.nblk ? a.blk[bi] : a.thin[bi - a.nblk];
     const uint32_t i0 = blockIdx.x % a.per_blk * a.rows, JG = J / a.rows;
+    if (i0 >= b.R) return;
+    const uint32_t nsrc = b.src != PCB_NONE ? a.src_list[b.src] : 0;
+    if (threadIdx.x < nsrc) src[threadIdx.x] = a.src_list[b.src + 1 + threadIdx.x];
     const uint32_t r = q / JG, jg = q % JG, i = i0 + r;
     const bool on = q < JG * a.rows && s < St && i < b.R;
     float* const stage = park + (size_t)a.slots * 2 * KLD_THREADS;
@@ -157,13 +167,14 @@ __global__ void __launch_bounds__(KLD_THREADS) kld_up_layer_kernel(KldLayer a) {
         pcb_copy4_async(mine + (2 * m) * KLD_THREADS, a.p1 + base + (size_t)j * a.S);
         pcb_copy4_async(mine + (2 * m + 1) * KLD_THREADS, a.p2 + base + (size_t)j * a.S);
       }
+    __syncthreads();   // src is complete
     pcb_grid_dep_wait();
     const uint32_t cj = KLD_STAGE / a.St;
     float acc = 0.0f;
     uint32_t j = jg, m = 0;
     for (uint32_t c0 = 0; c0 < b.K; c0 += cj) {
       const uint32_t n = min(cj, b.K - c0);
-      const float* kc = a.klds + (size_t)(b.c0 + c0) * a.ld + s0 + s;
+      const float* kc = a.klds + (size_t)((nsrc ? src[0] : b.c0) + c0) * a.ld + s0 + s;
       const float* kd = a.klds + (size_t)((b.d0 != PCB_NONE ? b.d0 : b.c0) + c0) * a.ld + s0 + s;
       float v0[8], v1[8];
       for (uint32_t g0 = q; g0 < n; g0 += 8 * J) {
@@ -173,6 +184,23 @@ __global__ void __launch_bounds__(KLD_THREADS) kld_up_layer_kernel(KldLayer a) {
           v0[u] = in ? kc[(size_t)(g0 + u * J) * a.ld] : 0.0f;
           v1[u] = in && b.d0 != PCB_NONE ? kd[(size_t)(g0 + u * J) * a.ld] : 0.0f;
         }
+        for (uint32_t x = 1; x < nsrc; x += 3) {   // the other nodes that a fused product adds up, three of them in flight
+          float y[3][8];
+#pragma unroll
+          for (uint32_t k = 0; k < 3; ++k) {
+            const float* ks = a.klds + (size_t)(src[min(x + k, nsrc - 1)] + c0) * a.ld + s0 + s;
+#pragma unroll
+            for (uint32_t u = 0; u < 8; ++u) y[k][u] = x + k < nsrc && q < J && s < St && g0 + u * J < n ? ks[(size_t)(g0 + u * J) * a.ld] : 0.0f;
+          }
+#pragma unroll
+          for (uint32_t k = 0; k < 3; ++k)
+#pragma unroll
+            for (uint32_t u = 0; u < 8; ++u) v0[u] += y[k][u];
+        }
+        if (nsrc && i0 == 0)   // the products' own values: the way down and the accessors read them
+#pragma unroll
+          for (uint32_t u = 0; u < 8; ++u)
+            if (q < J && s < St && g0 + u * J < n) a.klds[(size_t)(b.c0 + c0 + g0 + u * J) * a.ld + s0 + s] = v0[u];
 #pragma unroll
         for (uint32_t u = 0; u < 8; ++u)
           if (q < J && s < St && g0 + u * J < n) stage[(g0 + u * J) * a.St + s] = v0[u] + v1[u];
@@ -244,77 +272,98 @@ __global__ void __launch_bounds__(KLD_THREADS) kld_up_layer_kernel(KldLayer a) {
   }
 }
 
-// The same with one warp per (node, set): lanes over the node's edges.  With a handful of parameter
-// sets the (set, node) layout above leaves every thread a serial loop over up to k edges; a layer
-// of a single-set call then takes tens of microseconds instead of a few.  Such a call is a chain of
-// short dependent launches, so everything that does not depend on the layer below (the edge lists,
-// both parameters of the first 64 edges and exp of one) is fetched BEFORE the wait on the preceding
-// launch; after it only the children's values are gathered.
+// One or two sets: one warp per (sum node, set), lanes over the node's edges.  Such a call is a chain of short dependent
+// launches, so everything that does not depend on the step below (the run of children or the edge list, both parameters
+// of the first 64 edges and exp of one) is fetched BEFORE the wait on the preceding launch; after it only the children's
+// values are gathered, all of them in flight at once, so a step costs one round trip to L2.
+// Blocks of threads: eight rows of a dense block each, then eight of the other nodes.
 constexpr int KLD_PRE = 2;   // edges per lane held across the wait
-__global__ void kld_up_warp_kernel(float* __restrict__ klds, uint32_t ld, uint32_t S, const float* __restrict__ p1,
-                                   const float* __restrict__ p2, const uint32_t* __restrict__ nodes, uint32_t count,
-                                   const uint8_t* __restrict__ kind, const uint32_t* __restrict__ n_estart,
-                                   const uint32_t* __restrict__ n_ecount, const uint32_t* __restrict__ n_pid0,
-                                   const uint32_t* __restrict__ e_prime, const uint32_t* __restrict__ e_sub,
-                                   uint32_t root, float* __restrict__ root_out) {
+__global__ void __launch_bounds__(256) kld_up_warp_kernel(KldLayer a) {
+  __shared__ uint32_t src[PCB_MAX_SOURCES];
   pcb_grid_dep_launch();
   KLD_T_ENTER();
-  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= count * S) return;
-  const uint32_t i = w / S, s = w % S;
-  const uint32_t n = nodes[i];
-  const uint32_t e0 = n_estart[n], cnt = n_ecount[n];
-  const bool issum = kind[n] == PCB_SUM;
-  const uint32_t pid0 = n_pid0[n];
-  uint32_t pr[KLD_PRE], sb[KLD_PRE];
-  float wgt[KLD_PRE], dif[KLD_PRE];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, s = blockIdx.y, S = a.S;
+  float* const klds = a.klds + s;
+  const size_t ld = a.ld;
+  if (blockIdx.x < a.dense_ctas) {
+    const uint32_t bi = blockIdx.x / a.per_blk;
+    const PcbDenseBlock b = bi < a.nblk ? a.blk[bi] : a.thin[bi - a.nblk];
+    const uint32_t i = blockIdx.x % a.per_blk * 8 + warp;
+    if (blockIdx.x % a.per_blk * 8 >= b.R) return;
+    uint32_t nsrc = b.src != PCB_NONE ? a.src_list[b.src] : 0;
+    if (threadIdx.x < nsrc) src[threadIdx.x] = a.src_list[b.src + 1 + threadIdx.x];
+    const size_t base = s + (size_t)S * (b.pid0 + (size_t)(i < b.R ? i : 0) * b.K);
+    float wgt[KLD_PRE], dif[KLD_PRE];
 #pragma unroll
-  for (int r = 0; r < KLD_PRE; ++r) {
-    const uint32_t j = lane + 32 * r;
-    pr[r] = sb[r] = PCB_NONE; wgt[r] = 1.0f; dif[r] = 0.0f;
-    if (j < cnt) {
-      pr[r] = e_prime[e0 + j];
-      sb[r] = e_sub[e0 + j];
-      if (issum) {
-        const float a = p1[s + (size_t)S * (pid0 + j)], b = p2[s + (size_t)S * (pid0 + j)];
-        wgt[r] = expf(a);
-        dif[r] = a - b;
+    for (int r = 0; r < KLD_PRE; ++r) {
+      const uint32_t j = lane + 32 * r;
+      wgt[r] = dif[r] = 0.0f;
+      if (j < b.K) {
+        const float x = a.p1[base + (size_t)S * j], y = a.p2[base + (size_t)S * j];
+        wgt[r] = expf(x);
+        dif[r] = x - y;
       }
+      keep(wgt[r]); keep(dif[r]);
     }
-    keep(pr[r]); keep(sb[r]); keep(wgt[r]); keep(dif[r]);
-  }
-  pcb_grid_dep_wait();   // everything above is static circuit data or this call's parameters
-  KLD_T_WAITED();
-  // all gathers of the held edges are issued back to back (an edge without a second child reads
-  // the first one again), so the layer costs one round trip to L2, not one per operand
-  float k0[KLD_PRE], k1[KLD_PRE];
+    keep(nsrc);
+    __syncthreads();
+    pcb_grid_dep_wait();
+    KLD_T_WAITED();
+    const uint32_t first = nsrc ? src[0] : b.c0, second = nsrc > 1 ? src[1] : first, sub = b.d0 != PCB_NONE ? b.d0 : first;
+    auto value = [&](uint32_t j, float& product) {
+      const float k0 = klds[(size_t)(first + j) * ld], k1 = klds[(size_t)(second + j) * ld], k2 = klds[(size_t)(sub + j) * ld];
+      product = k0 + (nsrc > 1 ? k1 : 0.0f);
+      for (uint32_t x = 2; x < nsrc; x += 4) {
+        float y[4];
 #pragma unroll
-  for (int r = 0; r < KLD_PRE; ++r) {
-    const uint32_t a0 = pr[r] != PCB_NONE ? pr[r] : n, a1 = sb[r] != PCB_NONE ? sb[r] : a0;
-    k0[r] = klds[(size_t)a0 * ld + s];
-    k1[r] = klds[(size_t)a1 * ld + s];
+        for (uint32_t k = 0; k < 4; ++k) y[k] = x + k < nsrc ? klds[(size_t)(src[x + k] + j) * ld] : 0.0f;
+        product += (y[0] + y[1]) + (y[2] + y[3]);
+      }
+      return product + (b.d0 != PCB_NONE ? k2 : 0.0f);
+    };
+    float k[KLD_PRE], pr[KLD_PRE], acc = 0.0f;
+#pragma unroll
+    for (int r = 0; r < KLD_PRE; ++r) k[r] = lane + 32 * r < b.K ? value(lane + 32 * r, pr[r]) : 0.0f;
+#pragma unroll
+    for (int r = 0; r < KLD_PRE; ++r) {
+      acc += wgt[r] * (k[r] + dif[r]);
+      if (nsrc && i == 0 && lane + 32 * r < b.K) klds[(size_t)(b.c0 + lane + 32 * r) * ld] = pr[r];   // the products' own values
+    }
+    for (uint32_t j = lane + 32 * KLD_PRE; j < b.K; j += 32) {
+      float product;
+      const float v = value(j, product), x = a.p1[base + (size_t)S * j], y = a.p2[base + (size_t)S * j];
+      acc += expf(x) * (v + x - y);
+      if (nsrc && i == 0) klds[(size_t)(b.c0 + j) * ld] = product;
+    }
+    acc = warp_sum(acc);
+    if (lane == 0 && i < b.R) {
+      klds[(size_t)(b.p0 + i) * ld] = acc;
+      if (a.root_out && b.p0 + i == a.root) a.root_out[s] = acc;
+    }
+    KLD_T_EXIT();
+    return;
   }
+  const uint32_t i = (blockIdx.x - a.dense_ctas) * 8 + warp;
+  if (i >= a.count) return;
+  const uint32_t n = a.nodes[i], e0 = a.n_estart[n], cnt = a.n_ecount[n], pid0 = a.n_pid0[n];
+  const bool issum = a.kind[n] == PCB_SUM;
+  pcb_grid_dep_wait();
   float acc = 0.0f;
-#pragma unroll
-  for (int r = 0; r < KLD_PRE; ++r) {
-    const float k = k0[r] + (sb[r] != PCB_NONE ? k1[r] : 0.0f);
-    const float term = issum ? wgt[r] * (k + dif[r]) : k;
-    acc += pr[r] != PCB_NONE ? term : 0.0f;
-  }
-  for (uint32_t j = lane + 32 * KLD_PRE; j < cnt; j += 32) {
-    float k = klds[(size_t)e_prime[e0 + j] * ld + s];
-    uint32_t sb2 = e_sub[e0 + j];
-    if (sb2 != PCB_NONE) k += klds[(size_t)sb2 * ld + s];
+#pragma unroll 2
+  for (uint32_t j = lane; j < cnt; j += 32) {
+    float k = klds[(size_t)a.e_prime[e0 + j] * ld];
+    const uint32_t sb = a.e_sub[e0 + j];
+    if (sb != PCB_NONE) k += klds[(size_t)sb * ld];
     if (issum) {
-      float a = p1[s + (size_t)S * (pid0 + j)], b = p2[s + (size_t)S * (pid0 + j)];
-      k = expf(a) * (k + a - b);
+      const float x = a.p1[s + (size_t)S * (pid0 + j)], y = a.p2[s + (size_t)S * (pid0 + j)];
+      k = expf(x) * (k + x - y);
     }
     acc += k;
   }
   acc = warp_sum(acc);
   if (lane == 0) {
-    klds[(size_t)n * ld + s] = acc;
-    if (root_out && n == root) root_out[s] = acc;
+    klds[(size_t)n * ld] = acc;
+    if (a.root_out && n == a.root) a.root_out[s] = acc;
   }
   KLD_T_EXIT();
 }
@@ -359,6 +408,7 @@ __global__ void __launch_bounds__(KLD_THREADS) kld_down_layer_kernel(KldLayer a)
   if (blockIdx.x < a.dense_ctas) {
     const PcbDenseBlock b = a.blk[blockIdx.x / a.per_blk];
     const uint32_t JC = a.rows, IG = J / JC;
+    const uint32_t nsrc = b.src != PCB_NONE ? a.src_list[b.src] : 0;
     const uint32_t jj = q % JC, ig = q / JC, j = blockIdx.x % a.per_blk * JC + jj;
     const bool on = ig < IG && s < St && j < b.K;
     const size_t base = ((size_t)b.pid0 + (on ? j : 0)) * a.S + s0 + (on ? s : 0), step = (size_t)b.K * a.S;
@@ -416,7 +466,8 @@ __global__ void __launch_bounds__(KLD_THREADS) kld_down_layer_kernel(KldLayer a)
     if (on && ig == 0) {
       float t = 0.0f;
       for (uint32_t g = 0; g < IG; ++g) t += red[threadIdx.x + g * JC * a.St];
-      a.grads[(size_t)(b.c0 + j) * a.ld + s0 + s] = t;
+      if (!nsrc) a.grads[(size_t)(b.c0 + j) * a.ld + s0 + s] = t;
+      for (uint32_t x = 0; x < nsrc; ++x) a.grads[(size_t)(a.src_list[b.src + 1 + x] + j) * a.ld + s0 + s] = t;   // what the product hands on
       if (b.d0 != PCB_NONE) a.grads[(size_t)(b.d0 + j) * a.ld + s0 + s] = t;
     }
     return;
@@ -616,17 +667,28 @@ __global__ void renorm_kernel(float* __restrict__ theta, uint32_t n_groups, cons
 // with the caller's copies: two sets 240 against 264 us, four sets 397 against 228 us).
 constexpr uint32_t KLD_WARP_SETS = 2;
 
-KldLayer kld_layer(pcb_circuit* c, pcb_workspace* ws, const float* p1, const float* p2, uint32_t S, uint32_t lay) {
+// what the kernels of step t need; the caller adds the loose nodes and the shares of a CTA
+KldLayer kld_layer(pcb_circuit* c, pcb_workspace* ws, const float* p1, const float* p2, uint32_t S, uint32_t t) {
   KldLayer a;
   memset(&a, 0, sizeof(a));
   a.klds = ws->klds; a.grads = ws->grads; a.p1 = p1; a.p2 = p2; a.ld = ws->ldS; a.S = S; a.St = std::min(S, 32u);
-  if (pcb_layer_blocks(c, lay)) a.blk = c->layer_dense + c->h_layer_dense_off[lay];
+  a.nblk = pcb_step_blocks(c, t);
+  if (a.nblk) a.blk = c->dense + c->h_dense_off[t];
+  a.src_list = c->src_list;
   a.kind = c->kind; a.n_estart = c->n_estart; a.n_ecount = c->n_ecount; a.n_pid0 = c->n_pid0;
   a.e_prime = c->e_prime; a.e_sub = c->e_sub; a.in_off = c->in_off; a.in_ent = c->in_ent; a.root = c->N - 1;
   return a;
 }
+// the upward work of step t: thin blocks and the nodes taken one by one; returns the number of blocks
+uint32_t kld_up_work(pcb_circuit* c, KldLayer& a, uint32_t t) {
+  const uint32_t thin = c->h_st_thin_off[t + 1] - c->h_st_thin_off[t];
+  a.thin = c->thin + c->h_st_thin_off[t];
+  a.nodes = c->st_up + c->h_st_up_off[t];
+  a.count = c->h_st_up_off[t + 1] - c->h_st_up_off[t] - thin;
+  return a.nblk + thin;
+}
 
-cudaError_t kld_launch_layer(pcb_circuit* c, void (*kernel)(KldLayer), KldLayer& a, uint32_t lay, bool chained,
+cudaError_t kld_launch_layer(pcb_circuit* c, void (*kernel)(KldLayer), KldLayer& a, uint32_t blocks, bool chained,
                              cudaStream_t st) {
   static PcbPerDeviceOnce once;
   const size_t most = (2 * KLD_SLOTS * KLD_THREADS + KLD_STAGE) * sizeof(float);
@@ -636,11 +698,21 @@ cudaError_t kld_launch_layer(pcb_circuit* c, void (*kernel)(KldLayer), KldLayer&
   });
   if (e != cudaSuccess) return e;
   const uint32_t J = KLD_THREADS / a.St;
-  a.dense_ctas = pcb_layer_blocks(c, lay) * a.per_blk;
+  a.dense_ctas = blocks * a.per_blk;
   const uint32_t ctas = a.dense_ctas + (a.count + J - 1) / J;
   ++c->prof.launches[PCB_K_KLD];
   return pcb_launch_pdl(kernel, dim3(ctas, (a.S + a.St - 1) / a.St), dim3(KLD_THREADS),
                         a.dense_ctas ? (2 * a.slots * KLD_THREADS + KLD_STAGE) * sizeof(float) : 0, st, c->pdl && chained, a);
+}
+
+// a warp per sum node or loose node (kld_up_warp_kernel, kld1_push_kernel)
+cudaError_t kld_launch_warps(pcb_circuit* c, void (*kernel)(KldLayer), KldLayer& a, uint32_t blocks, uint32_t R, cudaStream_t st) {
+  a.per_blk = (R + 7) / 8;
+  a.dense_ctas = blocks * a.per_blk;
+  const uint32_t ctas = a.dense_ctas + (a.count + 7) / 8;
+  if (!ctas) return cudaSuccess;
+  ++c->prof.launches[PCB_K_KLD];
+  return pcb_launch_pdl(kernel, dim3(ctas, a.S), dim3(256), 0, st, c->pdl, a);
 }
 
 }  // namespace
@@ -672,28 +744,23 @@ extern "C" int32_t pcb_kld(pcb_circuit* c, pcb_workspace* ws, const float* param
                                                   c->in_node, c->in_cats, c->in_poff, ws->kld_bump,
                                                   ws->kld_bump ? ws->grads : nullptr, c->N);
   }
-  for (uint32_t lay = 1; lay <= c->L; ++lay) {
-    uint32_t o0 = c->h_up_all_off[lay - 1], o1 = c->h_up_all_off[lay];
-    if (o1 == o0) continue;
+  for (uint32_t t = 1; t <= c->n_steps; ++t) {
+    KldLayer a = kld_layer(c, ws, params1_dev, params2_dev, S, t);
+    const uint32_t blocks = kld_up_work(c, a, t);
+    a.root_out = kld_out_dev;
+    uint32_t R = 1, K = 1;
+    pcb_step_extent(c, t, R, K);
+    for (uint32_t i = c->h_st_thin_off[t]; i < c->h_st_thin_off[t + 1]; ++i) K = std::max(K, c->h_thin[i].K);
     if (S <= KLD_WARP_SETS) {
-      ++c->prof.launches[PCB_K_KLD];
-      PCB_CUDA(pcb_launch_pdl(kld_up_warp_kernel, dim3((uint32_t)(((uint64_t)(o1 - o0) * S + 7) / 8)), dim3(256), 0, st, c->pdl,
-                              ws->klds, ld, S, params1_dev, params2_dev, c->up_all + o0, o1 - o0, c->kind, c->n_estart,
-                              c->n_ecount, c->n_pid0, c->e_prime, c->e_sub, c->N - 1, kld_out_dev));
+      PCB_CUDA(kld_launch_warps(c, kld_up_warp_kernel, a, blocks, R, st));
       continue;
     }
-    KldLayer a = kld_layer(c, ws, params1_dev, params2_dev, S, lay);
-    a.nodes = c->up_sparse + c->h_up_sparse_off[lay - 1];
-    a.count = c->h_up_sparse_off[lay] - c->h_up_sparse_off[lay - 1];
-    a.root_out = kld_out_dev;
-    uint32_t R = 0, K = 1;
-    pcb_layer_extent(c, lay, R, K);
     // a thread should have about twelve edges (24 KB of parameters in flight per CTA): rows that share a CTA
     const uint32_t J = KLD_THREADS / a.St;
-    a.rows = R ? std::min({std::max(1u, (J * 12 + K / 2) / K), J, R}) : 1;
+    a.rows = std::min({std::max(1u, (J * 12 + K / 2) / K), J, R});
     a.per_blk = (R + a.rows - 1) / a.rows;
     a.slots = std::min(KLD_SLOTS, (K + J / a.rows - 1) / (J / a.rows));
-    PCB_CUDA(kld_launch_layer(c, kld_up_layer_kernel, a, lay, true, st));
+    PCB_CUDA(kld_launch_layer(c, kld_up_layer_kernel, a, blocks, true, st));
   }
   if (kld_out_dev && c->L == 0)   // the layer kernels write the root's value themselves
     ++c->prof.launches[PCB_K_KLD], copy_root_kernel<<<(S + 127) / 128, 128, 0, st>>>(ws->klds + (size_t)(c->N - 1) * ld, S, kld_out_dev);
@@ -714,30 +781,33 @@ extern "C" int32_t pcb_kld_backward(pcb_circuit* c, pcb_workspace* ws, const flo
   cudaStream_t st = (cudaStream_t)s;
   const uint32_t ld = ws->ldS;
   bool chained = false;   // the first launch of the pass waits for whatever the caller's stream holds before it
-  for (int64_t lay = c->L; lay >= 0; --lay) {
-    uint32_t o0 = c->h_down_all_off[lay], o1 = c->h_down_all_off[lay + 1];
-    if (S <= KLD_WARP_SETS) {
+  if (S <= KLD_WARP_SETS) {
+    for (int64_t lay = c->L; lay >= 0; --lay) {
+      const uint32_t o0 = c->h_down_all_off[lay], o1 = c->h_down_all_off[lay + 1];
       if (o1 == o0) continue;
       ++c->prof.launches[PCB_K_KLD];
-      PCB_CUDA(pcb_launch_pdl(kld_down_warp_kernel, dim3((uint32_t)(((uint64_t)(o1 - o0) * S + 7) / 8)), dim3(256), 0, st, c->pdl,
-                              ws->grads, (const float*)ws->klds, ld, S, params1_dev, params2_dev, c->down_all + o0, o1 - o0,
-                              c->N - 1, c->in_off, c->in_ent, grads1_dev, grads2_dev));
-      continue;
+      PCB_CUDA(pcb_launch_pdl(kld_down_warp_kernel, dim3((uint32_t)(((uint64_t)(o1 - o0) * S + 7) / 8)), dim3(256), 0, st,
+                              c->pdl && chained, ws->grads, (const float*)ws->klds, ld, S, params1_dev, params2_dev, c->down_all + o0,
+                              o1 - o0, c->N - 1, c->in_off, c->in_ent, grads1_dev, grads2_dev));
+      chained = true;
     }
-    KldLayer a = kld_layer(c, ws, params1_dev, params2_dev, S, (uint32_t)lay + 1);
-    a.g1 = grads1_dev; a.g2 = grads2_dev;
-    a.nodes = c->down_sparse + c->h_down_sparse_off[lay];
-    a.count = c->h_down_sparse_off[lay + 1] - c->h_down_sparse_off[lay];
-    uint32_t R = 0, K = 1;
-    pcb_layer_extent(c, (uint32_t)lay + 1, R, K);
-    // children of a CTA: whole 256-byte runs of parameters; the rest of the threads split the rows
-    const uint32_t J = KLD_THREADS / a.St;
-    a.rows = std::min({std::max(1u, 64 / a.St), J, K});
-    a.per_blk = (K + a.rows - 1) / a.rows;
-    a.slots = std::min(KLD_SLOTS, ((R ? R : 1) + J / a.rows - 1) / (J / a.rows));
-    if (!a.count && !pcb_layer_blocks(c, (uint32_t)lay + 1)) continue;
-    PCB_CUDA(kld_launch_layer(c, kld_down_layer_kernel, a, (uint32_t)lay + 1, chained, st));
-    chained = true;
+  } else {
+    for (int64_t t = c->n_steps; t >= 0; --t) {   // the blocks of step t + 1 and the other nodes of step t
+      KldLayer a = kld_layer(c, ws, params1_dev, params2_dev, S, (uint32_t)t + 1);
+      a.g1 = grads1_dev; a.g2 = grads2_dev;
+      a.nodes = c->st_down + c->h_st_down_off[t];
+      a.count = c->h_st_down_off[t + 1] - c->h_st_down_off[t];
+      if (!a.count && !a.nblk) continue;
+      uint32_t R = 1, K = 1;
+      pcb_step_extent(c, (uint32_t)t + 1, R, K);
+      // children of a CTA: whole 256-byte runs of parameters; the rest of the threads split the rows
+      const uint32_t J = KLD_THREADS / a.St;
+      a.rows = std::min({std::max(1u, 64 / a.St), J, K});
+      a.per_blk = (K + a.rows - 1) / a.rows;
+      a.slots = std::min(KLD_SLOTS, (R + J / a.rows - 1) / (J / a.rows));
+      PCB_CUDA(kld_launch_layer(c, kld_down_layer_kernel, a, a.nblk, chained, st));
+      chained = true;
+    }
   }
   if (c->n_inputs) {
     Shape2 sh = shape_for(S, c->n_inputs);
@@ -810,75 +880,68 @@ namespace {
 __global__ void set_step_kernel(int* __restrict__ t, int value) { *t = value; }
 
 // ---- the fused single-set step: node gradients pushed down by the parents -------------------------
-// One warp per node of an up layer, layers from the root down: every parent of the node lies in a
-// higher layer, so its gradient is complete.  A sum edge hands pg * exp(theta) to both children, a
-// product edge hands pg.  Lanes run over the edges of the node, so the parameters are read
-// contiguously (the pull form reads them with the stride of the fan-in).  The eight nodes of a block
-// usually have the same children (up_same): their contributions are added in shared memory and reach
-// memory as one atomic per child; otherwise every edge adds its own.  The sums are floating-point
-// atomics, like the reference's CUDA.@atomic on partially owned nodes (queries/kld.jl:258-300): the
-// order of the additions, and with it the last bits, can differ from run to run.
-__global__ void __launch_bounds__(256) kld1_push_kernel(float* __restrict__ grads, const float* __restrict__ p1,
-                                                        const uint32_t* __restrict__ nodes, uint32_t count,
-                                                        const uint4* __restrict__ s_node,
-                                                        const uint32_t* __restrict__ e_prime,
-                                                        const uint32_t* __restrict__ e_sub,
-                                                        const uint8_t* __restrict__ same_flags, uint32_t ld) {
+// Steps from the root down: every parent of a step's nodes lies in a higher step, so their gradients are complete.  A
+// block of threads takes eight rows of a dense block: a warp per row, lanes over the edges, so the parameters are read
+// contiguously (the pull form reads them with the stride of the fan-in); pg * exp(theta) of the eight rows is added in
+// shared memory and reaches the children (and the nodes that fused products multiply) as one atomic each.  The other
+// nodes push edge by edge.  The sums are floating-point atomics, like the reference's CUDA.@atomic on partially owned
+// nodes (queries/kld.jl:258-300): the order of the additions, and with it the last bits, can differ from run to run.
+__global__ void __launch_bounds__(256) kld1_push_kernel(KldLayer a) {
   __shared__ float red[8][256];
+  __shared__ uint32_t src[PCB_MAX_SOURCES];
   pcb_grid_dep_launch();
   KLD_T_ENTER();
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t i = blockIdx.x * 8 + warp;
-  const bool valid = i < count;
-  const uint32_t n = nodes[valid ? i : blockIdx.x * 8];
-  const uint4 sn = s_node[n];                     // edge start, edge count, first parameter, kind | region << 2
-  const uint32_t e0 = sn.x, cnt = sn.y, pid0 = sn.z;
-  const bool issum = (sn.w & 3u) == PCB_SUM;
-  const bool same = same_flags[blockIdx.x] != 0;   // then every warp of the block sees the same e0-relative children
-  float wgt[KLD_PRE];
-  uint32_t pr[KLD_PRE], sb[KLD_PRE];
+  float* const grads = a.grads;
+  const size_t ld = a.ld;
+  if (blockIdx.x < a.dense_ctas) {
+    const PcbDenseBlock b = a.blk[blockIdx.x / a.per_blk];
+    const uint32_t i0 = blockIdx.x % a.per_blk * 8, i = i0 + warp;
+    if (i0 >= b.R) return;
+    uint32_t nsrc = b.src != PCB_NONE ? a.src_list[b.src] : 0;
+    if (threadIdx.x < nsrc) src[threadIdx.x] = a.src_list[b.src + 1 + threadIdx.x];
+    const float* const p = a.p1 + b.pid0 + (size_t)(i < b.R ? i : 0) * b.K;
+    float wgt[KLD_PRE];
 #pragma unroll
-  for (int r = 0; r < KLD_PRE; ++r) {
-    const uint32_t j = lane + 32 * r;
-    wgt[r] = 0.0f; pr[r] = sb[r] = PCB_NONE;
-    if (j < cnt) {
-      wgt[r] = issum ? expf(p1[pid0 + j]) : 1.0f;
-      if (!same) { pr[r] = e_prime[e0 + j]; sb[r] = e_sub[e0 + j]; }
+    for (int r = 0; r < KLD_PRE; ++r) {
+      wgt[r] = lane + 32 * r < b.K ? expf(p[lane + 32 * r]) : 0.0f;
+      keep(wgt[r]);
     }
-    keep(wgt[r]); keep(pr[r]); keep(sb[r]);
-  }
-  // the threads that will add a column of the block: its two children
-  uint32_t cpr = PCB_NONE, csb = PCB_NONE;
-  if (same && threadIdx.x < cnt) { cpr = e_prime[e0 + threadIdx.x]; csb = e_sub[e0 + threadIdx.x]; }
-  keep(cpr); keep(csb);
-  pcb_grid_dep_wait();   // everything above is static circuit data or this call's parameters
-  KLD_T_WAITED();
-  const float pg = valid ? grads[(size_t)n * ld] : 0.0f;
-  if (same) {
+    keep(nsrc);
+    pcb_grid_dep_wait();   // everything above is static circuit data or this call's parameters
+    KLD_T_WAITED();
+    const float pg = i < b.R ? grads[(size_t)(b.p0 + i) * ld] : 0.0f;
+    for (uint32_t j0 = 0; j0 < b.K; j0 += 256) {   // the rows' shares of up to 256 children at a time
+      if (j0) __syncthreads();
 #pragma unroll
-    for (int r = 0; r < KLD_PRE; ++r)
-      if (lane + 32 * r < cnt) red[warp][lane + 32 * r] = pg * wgt[r];
-    for (uint32_t j = lane + 32 * KLD_PRE; j < cnt; j += 32) red[warp][j] = pg * expf(p1[pid0 + j]);
-    __syncthreads();
-    if (threadIdx.x < cnt) {
-      float v = 0.0f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) v += red[w][threadIdx.x];
-      atomicAdd(grads + (size_t)cpr * ld, v);
-      if (csb != PCB_NONE) atomicAdd(grads + (size_t)csb * ld, v);
-    }
-  } else if (valid) {
-#pragma unroll
-    for (int r = 0; r < KLD_PRE; ++r)
-      if (pr[r] != PCB_NONE) {
-        atomicAdd(grads + (size_t)pr[r] * ld, pg * wgt[r]);
-        if (sb[r] != PCB_NONE) atomicAdd(grads + (size_t)sb[r] * ld, pg * wgt[r]);
+      for (int r = 0; r < 8; ++r) {
+        const uint32_t j = lane + 32 * r;
+        if (j0 + j < b.K) red[warp][j] = pg * (j0 == 0 && r < KLD_PRE ? wgt[r < KLD_PRE ? r : 0] : expf(p[j0 + j]));
       }
-    for (uint32_t j = lane + 32 * KLD_PRE; j < cnt; j += 32) {
-      const float eg = issum ? pg * expf(p1[pid0 + j]) : pg;
-      atomicAdd(grads + (size_t)e_prime[e0 + j] * ld, eg);
-      if (e_sub[e0 + j] != PCB_NONE) atomicAdd(grads + (size_t)e_sub[e0 + j] * ld, eg);
+      __syncthreads();
+      const uint32_t j = j0 + threadIdx.x;
+      if (j < b.K) {
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v += red[w][threadIdx.x];
+        if (!nsrc) atomicAdd(grads + (size_t)(b.c0 + j) * ld, v);
+        for (uint32_t x = 0; x < nsrc; ++x) atomicAdd(grads + (size_t)(src[x] + j) * ld, v);
+        if (b.d0 != PCB_NONE) atomicAdd(grads + (size_t)(b.d0 + j) * ld, v);
+      }
     }
+    KLD_T_EXIT();
+    return;
+  }
+  const uint32_t i = (blockIdx.x - a.dense_ctas) * 8 + warp;
+  if (i >= a.count) return;
+  const uint32_t n = a.nodes[i], e0 = a.n_estart[n], cnt = a.n_ecount[n], pid0 = a.n_pid0[n];
+  const bool issum = a.kind[n] == PCB_SUM;
+  pcb_grid_dep_wait();
+  const float pg = grads[(size_t)n * ld];
+  for (uint32_t j = lane; j < cnt; j += 32) {
+    const float eg = issum ? pg * expf(a.p1[pid0 + j]) : pg;
+    atomicAdd(grads + (size_t)a.e_prime[e0 + j] * ld, eg);
+    if (a.e_sub[e0 + j] != PCB_NONE) atomicAdd(grads + (size_t)a.e_sub[e0 + j] * ld, eg);
   }
   KLD_T_EXIT();
 }
@@ -1053,14 +1116,13 @@ static int32_t kld_adam_body(pcb_circuit* c, pcb_workspace* ws, float* theta_q, 
   int32_t r = pcb_kld(c, ws, theta_q, theta_p, 1, kld_out, s);
   ws->kld_bump = nullptr;
   if (r != PCB_OK) return r;
-  for (int64_t lay = c->L; lay >= 1; --lay) {
-    const uint32_t o0 = c->h_up_all_off[lay - 1], o1 = c->h_up_all_off[lay];
-    if (o1 == o0) continue;
-    ++c->prof.launches[PCB_K_KLD];
-    PCB_CUDA(pcb_launch_pdl(kld1_push_kernel, dim3((o1 - o0 + 7) / 8), dim3(256), 0, st, c->pdl, ws->grads,
-                            (const float*)theta_q, (const uint32_t*)(c->up_all + o0), o1 - o0, (const uint4*)c->s_node,
-                            (const uint32_t*)c->e_prime, (const uint32_t*)c->e_sub,
-                            (const uint8_t*)(c->up_same + c->h_up_chunk_off[lay - 1]), ws->ldS));
+  for (uint32_t t = c->n_steps; t >= 1; --t) {
+    KldLayer a = kld_layer(c, ws, theta_q, theta_p, 1, t);
+    a.nodes = c->st_up + c->h_st_up_off[t];
+    a.count = c->h_st_up_off[t + 1] - c->h_st_up_off[t];
+    uint32_t R = 1, K = 1;
+    pcb_step_extent(c, t, R, K);
+    PCB_CUDA(kld_launch_warps(c, kld1_push_kernel, a, a.nblk, R, st));
   }
   if (c->P) {
     AdamArgs a;

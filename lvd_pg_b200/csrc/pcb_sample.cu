@@ -506,17 +506,17 @@ __global__ void __launch_bounds__(SOFT_THREADS, 4) soft_params_kernel(
   }
 }
 
-// One launch per layer, from the root down: the dense blocks with parents in the layer above hand their probability
-// to their children, the other nodes of the layer pull from their parents (all parents were completed by earlier
+// One launch per step, from the root down: the dense blocks of the step above hand their probability to their children
+// (and to the nodes that fused products multiply), the other nodes of the step pull from their parents (all parents were completed by earlier
 // launches).  The weights of a CTA are copied into shared memory before the wait on the preceding launch, one private
 // slot per thread and row; after it the parents' values are staged in one batch.  784 variables x 64 latents x 24
-// samples: 993 -> 155 us over the 20 layers (one thread walked all parents of a child before).
+// samples: 993 -> 155 us over 20 layers (one thread walked all parents of a child before); 139 us over the 12 steps.
 constexpr uint32_t SOFT_SLOTS = 40, SOFT_STAGE = 8 * SOFT_THREADS;
 
 struct SoftLayer {
   float* td; const float* w;
   uint32_t ld, S, St, JC, per_blk, dense_ctas, slots;
-  const PcbDenseBlock* blk;
+  const PcbDenseBlock* blk; const uint32_t* src_list;
   const uint32_t* nodes; uint32_t count, root;
   const uint32_t* in_off; const PcbInEntry* in_ent;
 };
@@ -565,7 +565,9 @@ __global__ void __launch_bounds__(SOFT_THREADS) soft_down_kernel(SoftLayer a) {
     if (on && ig == 0) {
       float t = 0.0f;
       for (uint32_t k = 0; k < IG; ++k) t += red[threadIdx.x + k * JC * a.St];
-      a.td[(size_t)(b.c0 + j) * a.ld + s0 + s] = t;
+      const uint32_t nsrc = b.src != PCB_NONE ? a.src_list[b.src] : 0;
+      if (!nsrc) a.td[(size_t)(b.c0 + j) * a.ld + s0 + s] = t;
+      for (uint32_t x = 0; x < nsrc; ++x) a.td[(size_t)(a.src_list[b.src + 1 + x] + j) * a.ld + s0 + s] = t;   // what the product hands on
       if (b.d0 != PCB_NONE) a.td[(size_t)(b.d0 + j) * a.ld + s0 + s] = t;
     }
     return;
@@ -695,14 +697,15 @@ extern "C" int32_t pcb_sample_soft(pcb_circuit* c, pcb_workspace* ws, const floa
   bool chained = false;   // the first launch waits for the weights in full, the others for the launch before them
   SoftLayer a;
   a.td = td; a.w = ws->eprob; a.ld = ld; a.S = S; a.St = St; a.root = c->N - 1; a.in_off = c->in_off; a.in_ent = c->in_ent;
-  for (int64_t lay = c->L; lay >= 0; --lay) {
-    const uint32_t blocks = pcb_layer_blocks(c, (uint32_t)lay + 1);
-    a.blk = blocks ? c->layer_dense + c->h_layer_dense_off[lay + 1] : nullptr;
-    a.nodes = c->down_sparse + c->h_down_sparse_off[lay];
-    a.count = c->h_down_sparse_off[lay + 1] - c->h_down_sparse_off[lay];
+  a.src_list = c->src_list;
+  for (int64_t t = c->n_steps; t >= 0; --t) {   // the blocks of step t + 1 and the other nodes of step t
+    const uint32_t blocks = pcb_step_blocks(c, (uint32_t)t + 1);
+    a.blk = blocks ? c->dense + c->h_dense_off[t + 1] : nullptr;
+    a.nodes = c->st_down + c->h_st_down_off[t];
+    a.count = c->h_st_down_off[t + 1] - c->h_st_down_off[t];
     if (!blocks && !a.count) continue;
     uint32_t R = 1, K = 1;
-    pcb_layer_extent(c, (uint32_t)lay + 1, R, K);
+    pcb_step_extent(c, (uint32_t)t + 1, R, K);
     a.JC = std::min({std::max(1u, 64 / St), J, K});   // children of a CTA: runs of 256 bytes of weights
     a.per_blk = (K + a.JC - 1) / a.JC;
     a.slots = std::min(SOFT_SLOTS, (R + J / a.JC - 1) / (J / a.JC));
