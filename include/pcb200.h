@@ -277,6 +277,10 @@ int32_t pcb_sample_hard_static(pcb_circuit* c, const float* params_dev, uint32_t
 int32_t pcb_sample_soft(pcb_circuit* c, pcb_workspace* ws, const float* params_dev, uint32_t Sp,
                         const float* u_dev, float temperature, uint32_t S, float* out_dev,
                         pcb_stream s);
+/* The same with the sets and the uniforms row-major ([Sp, P] and [S, num_inner_params], last index fastest); at most
+ * 256 edges per sum node. */
+int32_t pcb_sample_soft_rows(pcb_circuit* c, pcb_workspace* ws, const float* params_dev, uint32_t Sp, const float* u_dev,
+                             float temperature, uint32_t S, float* out_dev, pcb_stream s);
 
 /* conditioned_td_prob(mbpc, marked_pc_idx1, marked_pc_idx2, node_probs, input_aggr_params)
  * (queries/td_prob.jl:161-291): top-down probabilities with the circuit's own weights in which

@@ -628,6 +628,12 @@ def _params_matrix(mbpc, p: ArrayLike) -> torch.Tensor:
     return _columns(mbpc, p.to(mbpc.device))
 
 
+def _row_major(mbpc, p, columns: int) -> bool:
+    """Several rows of `columns` values on the circuit's device, one contiguous row after the other."""
+    return isinstance(p, torch.Tensor) and p.dim() == 2 and p.shape[0] > 1 and p.shape[1] == columns \
+        and p.dtype == torch.float32 and p.device == mbpc.device and p.is_contiguous()
+
+
 def _columns(mbpc, p: torch.Tensor) -> torch.Tensor:
     """`p.t().contiguous()`; a row-major float32 matrix of several rows goes through the library's own kernel."""
     if p.dim() == 2 and p.dtype == torch.float32 and p.is_contiguous() and 1 < p.shape[0] < 32 * 65535 and p.shape[1] > 1 \
@@ -812,16 +818,19 @@ def gumbel_sample(mbpc: CuMetaBitsProbCircuit, params: ArrayLike, num_vars: int,
     """Relaxed top-down sampling: returns input_aggr_params [S, num_vars, par_buffer_size].
     The reference draws its noise in-kernel; here `u` ([S, num_inner_params] uniforms) is passed
     in, or no_gumbel=True selects the noise-free variant."""
-    p = _params_matrix(mbpc, params)
-    Sp = int(p.shape[1])
+    # row-major sets and uniforms of the exact shapes go in as they are, anything else as the column-major matrices of the C ABI
+    rows = _row_major(mbpc, params, num_parameters(mbpc)) and int(mbpc.info.max_group_size) <= 256 \
+        and S in (None, params.shape[0]) and (no_gumbel or (_row_major(mbpc, u, mbpc.num_inner_params) and u.shape[0] == params.shape[0]))
+    p = params if rows else _params_matrix(mbpc, params)
+    Sp = int(p.shape[0 if rows else 1])
     S = S or Sp
     assert num_vars == mbpc.fc.num_vars and par_buffer_size == int(mbpc.info.max_num_cats)
     ud = None
     if not no_gumbel:
         assert u is not None, "pass uniforms `u` or no_gumbel=True"
-        ud = _columns(mbpc, torch.as_tensor(u, dtype=torch.float32).to(mbpc.device))
+        ud = u if rows else _columns(mbpc, torch.as_tensor(u, dtype=torch.float32).to(mbpc.device))
     ws = mbpc.workspace(1)
     out = torch.empty(par_buffer_size, num_vars, S, dtype=torch.float32, device=mbpc.device)
-    _lib.check(mbpc.lib.pcb_sample_soft(mbpc.handle, ws, _ptr(p), Sp, _ptr(ud), temperature, S, _ptr(out),
-                                        _stream(mbpc.device)))
+    call = mbpc.lib.pcb_sample_soft_rows if rows else mbpc.lib.pcb_sample_soft
+    _lib.check(call(mbpc.handle, ws, _ptr(p), Sp, _ptr(ud), temperature, S, _ptr(out), _stream(mbpc.device)))
     return out.permute(2, 1, 0)

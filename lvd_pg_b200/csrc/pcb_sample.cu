@@ -403,60 +403,77 @@ __global__ void __launch_bounds__(CW * 32, CW == 1 ? 32 : 40 / CW) sample_hard_c
 // ---- relaxed sampling: exp((log p + gumbel) / T) of every sum edge, normalised per sum node ------------------
 // The keys are formed in fp64 like the reference's (sample.jl:24-54 promotes through its Float64 literals), with
 // logarithm and exponential by table and short polynomial (P. T. P. Tang, ACM TOMS 15 (1989) and 16 (1990)): the
-// result is rounded to fp32 (6e-8), a hundred times the error of these series, and eight fp64 operations per logarithm
-// replace the forty or more of one that is exact to the last bit.  Arguments outside the tables'
-// range (u outside (0, 1), |z| >= 600, NaN) take the CUDA functions.  fp64 units and HBM are the bounds: 24 x 1.7 M
-// edges 462 -> 285 us, now with the division by the node's sum that the top-down pass made before.
+// result is rounded to fp32 (6e-8), a hundred times the error of these series, and ten fp64 operations per logarithm
+// replace the forty or more of one that is exact to the last bit.  Arguments outside the tables' range (u outside
+// [0, 1), |z| >= 600, NaN) take the CUDA functions.  Instruction issue is the bound (66% of the slots, fp64 units at a
+// fifth): the checks of a pair of edges share one branch, the noise-free variant is a kernel of its own.
 constexpr uint32_t SOFT_THREADS = 256;
+// Every entry is there once for each lane of a half warp, so that lanes with different entries meet no bank twice (with
+// one copy a lookup of 128 and 256 entries took three times the passes): 32 entries, and two more terms of the series.
+constexpr uint32_t SOFT_COPIES = 16;
 struct SoftTables {
-  double2 lg[128];     // 1/c and log c of 128 intervals of [sqrt(1/2), sqrt 2)
-  double ex[256];      // 2^(i/256)
+  double rc[32][SOFT_COPIES], lg[32][SOFT_COPIES];   // 1/c and log c of 32 intervals of [sqrt(1/2), sqrt 2)
+  double ex[32][SOFT_COPIES];                        // 2^(i/32)
 };
 
 __device__ __forceinline__ void soft_tables_fill(SoftTables* t) {
-  for (uint32_t i = threadIdx.x; i < 128; i += blockDim.x) {
-    const double mid = __hiloint2double((int)(0x3fe6a09eu + (i << 13) + (1u << 12)), 0);
-    // the two intervals around one keep c = 1: log x is then the polynomial in x - 1 alone, relatively exact there
-    const double rcp = (i == 74 || i == 75) ? 1.0 : 1.0 / mid;
-    t->lg[i] = make_double2(rcp, -log(rcp));
-  }
-  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) t->ex[i] = exp2((double)i / 256.0);
+  const uint32_t i = threadIdx.x & 31;
+  const double mid = __hiloint2double((int)(0x3fe6a09eu + (i << 15) + (1u << 14)), 0);
+  // the interval around one keeps c = 1: log x is then the polynomial in x - 1 alone, relatively exact there
+  const double rcp = i == 18 ? 1.0 : 1.0 / mid, lg = -log(rcp), ex = exp2((double)i / 32.0);
+  for (uint32_t k = threadIdx.x >> 5; k < SOFT_COPIES; k += blockDim.x >> 5) { t->rc[i][k] = rcp; t->lg[i][k] = lg; t->ex[i][k] = ex; }
   __syncthreads();
 }
 
-// log of a positive normal double: |r| <= 2^-7 and the series ends after r^4, a relative 7e-10 at most
+// log of a positive normal double: |r| <= 2^-6 and the series ends after r^5, a relative 2e-10 at most
 __device__ __forceinline__ double soft_log(double x, const SoftTables* t) {
   const int hi = __double2hiint(x), tmp = hi - 0x3fe6a09e, e = tmp >> 20;
   const double m = __hiloint2double(hi - (e << 20), __double2loint(x));
-  const double2 c = t->lg[(tmp >> 13) & 127];
-  const double r = fma(m, c.x, -1.0);
-  const double q = fma(r, fma(r, fma(r, -0.25, 1.0 / 3.0), -0.5), 1.0);
+  const uint32_t i = (tmp >> 15) & 31, copy = threadIdx.x % SOFT_COPIES;
+  const double r = fma(m, t->rc[i][copy], -1.0);
+  const double q = fma(r, fma(r, fma(r, fma(r, 0.2, -0.25), 1.0 / 3.0), -0.5), 1.0);
   const double ed = __hiloint2double(0x43300000, e ^ (int)0x80000000) - (4503599627370496.0 + 2147483648.0);   // (double)e
-  return fma(ed, 0.69314718055994530942, fma(r, q, c.y));
+  return fma(ed, 0.69314718055994530942, fma(r, q, t->lg[i][copy]));
 }
 
-// exp(z) rounded to fp32, |z| < 600: |r| <= ln2 / 512, the series ends after r^2, a relative 4e-10
+// exp(z) rounded to fp32, |z| < 600: |r| <= ln2 / 64, the series ends after r^4, a relative 2e-12
 __device__ __forceinline__ float soft_exp(double z, const SoftTables* t) {
   const double shift = 6755399441055744.0;   // 1.5 * 2^52: the sum's low word is the rounded integer
-  const double s = fma(z, 256.0 / 0.69314718055994530942, shift);
+  const double s = fma(z, 32.0 / 0.69314718055994530942, shift);
   const int n = __double2loint(s);
-  const double r = fma(s - shift, -0.69314718055994530942 / 256.0, z);
-  const double p = fma(fma(r, 0.5, 1.0), r, 1.0) * t->ex[n & 255];
-  return (float)__hiloint2double(__double2hiint(p) + ((n >> 8) << 20), __double2loint(p));
+  const double r = fma(s - shift, -0.69314718055994530942 / 32.0, z);
+  const double p = fma(fma(fma(fma(r, 1.0 / 24.0, 1.0 / 6.0), r, 0.5), r, 1.0), r, 1.0) * t->ex[n & 31][threadIdx.x % SOFT_COPIES];
+  return (float)__hiloint2double(__double2hiint(p) + ((n >> 5) << 20), __double2loint(p));
 }
 
-__device__ __forceinline__ float soft_weight(float logp, float u, bool noise, double inv_t, const SoftTables* t) {
+// the tables serve u in [0, 1) and |z| < 600; `ok` is cleared for anything else
+template <bool NOISE>
+__device__ __forceinline__ float soft_weight_fast(float logp, float u, double inv_t, const SoftTables* t, bool& ok) {
   double g = 0.0;
-  if (noise) {
-    const double x = fma((double)u, 1.0 - 1e-6, 1e-6);
-    g = u > 0.0f && u < 1.0f ? -soft_log(-soft_log(x, t), t) : -log(-log(x));
+  if (NOISE) {
+    g = -soft_log(-soft_log(fma((double)u, 1.0 - 1e-6, 1e-6), t), t);
+    ok = ok && __float_as_uint(u) < 0x3f800000u;
   }
   const double z = ((double)logp + g) * inv_t;
-  return fabs(z) < 600.0 ? soft_exp(z, t) : (float)exp(z);
+  ok = ok && fabs(z) < 600.0;
+  return soft_exp(z, t);
+}
+template <bool NOISE>
+__device__ __noinline__ float soft_weight_any(float logp, float u, double inv_t) {
+  double g = 0.0;
+  if (NOISE) g = -log(-log(fma((double)u, 1.0 - 1e-6, 1e-6)));
+  return (float)exp(((double)logp + g) * inv_t);
+}
+template <bool NOISE>
+__device__ __forceinline__ float soft_weight(float logp, float u, double inv_t, const SoftTables* t) {
+  bool ok = true;
+  const float e = soft_weight_fast<NOISE>(logp, u, inv_t, t, ok);
+  return ok ? e : soft_weight_any<NOISE>(logp, u, inv_t);
 }
 
 // Threads are laid out (set, edge) with the set fastest, `rows` sum nodes per pass of a block; a thread keeps its up
 // to eight edges in registers between the sum and the division, wider nodes go through memory.
+template <bool NOISE>
 __global__ void __launch_bounds__(SOFT_THREADS, 4) soft_params_kernel(
     float* __restrict__ w, uint32_t ld, uint32_t S, uint32_t St, uint32_t rows, const float* __restrict__ params,
     uint32_t Sp, const float* __restrict__ u, double inv_t, const uint32_t* __restrict__ grp_node, uint32_t n_groups,
@@ -476,20 +493,20 @@ __global__ void __launch_bounds__(SOFT_THREADS, 4) soft_params_kernel(
       pid0 = n_pid0[n]; cnt = n_ecount[n];
     }
     const float* pp = params + ps + (size_t)Sp * pid0;
-    const float* pu = u ? u + s0 + s + (size_t)S * pid0 : nullptr;
+    const float* pu = NOISE ? u + s0 + s + (size_t)S * pid0 : nullptr;
     float* pw = w + (size_t)pid0 * ld + s0 + s;
     float x[8], y[8], sum = 0.0f;
 #pragma unroll
     for (uint32_t k = 0; k < 8; ++k) {
       const uint32_t j = jg + k * JG;
       x[k] = j < cnt ? pp[(size_t)Sp * j] : 0.0f;
-      y[k] = u && j < cnt ? __ldcs(pu + (size_t)S * j) : 0.5f;
+      y[k] = NOISE && j < cnt ? __ldcs(pu + (size_t)S * j) : 0.5f;
     }
 #pragma unroll
     for (uint32_t k = 0; k < 8; ++k)
-      if (jg + k * JG < cnt) { x[k] = soft_weight(x[k], y[k], u != nullptr, inv_t, &tab); sum += x[k]; }
+      if (jg + k * JG < cnt) { x[k] = soft_weight<NOISE>(x[k], y[k], inv_t, &tab); sum += x[k]; }
     for (uint32_t j = jg + 8 * JG; j < cnt; j += JG) {
-      const float e = soft_weight(pp[(size_t)Sp * j], u ? pu[(size_t)S * j] : 0.5f, u != nullptr, inv_t, &tab);
+      const float e = soft_weight<NOISE>(pp[(size_t)Sp * j], NOISE ? pu[(size_t)S * j] : 0.5f, inv_t, &tab);
       pw[(size_t)ld * j] = e;
       sum += e;
     }
@@ -503,6 +520,95 @@ __global__ void __launch_bounds__(SOFT_THREADS, 4) soft_params_kernel(
     for (uint32_t k = 0; k < 8; ++k)
       if (jg + k * JG < cnt) pw[(size_t)ld * (jg + k * JG)] = x[k] / total;
     for (uint32_t j = jg + 8 * JG; j < cnt; j += JG) pw[(size_t)ld * j] /= total;
+  }
+}
+
+// The same from row-major sets and noise ([S, P] and [S, edges] as a row-major host framework holds them): lanes over a
+// node's edges, warps over the sets; the weights turn through shared memory into the [edge][set] order of the walk below.
+// The next node's values are fetched while this one's are worked on.  A transposition of both matrices ahead of the
+// column kernel cost 140 us at 24 x 1.7 M edges; this kernel takes 253 us (333 with tables that lanes share and without
+// the prefetch, 312 with two branches an edge and a division in place of the product with a reciprocal in fp64), the
+// column kernel 285 without the transpositions.
+constexpr uint32_t SOFT_ROWS_K = 256;   // edges of a node that the tile holds
+template <bool NOISE>
+__global__ void __launch_bounds__(SOFT_THREADS, 3) soft_params_rows_kernel(
+    float* __restrict__ w, uint32_t ld, uint32_t S, const float* __restrict__ params, uint64_t ss,
+    const float* __restrict__ u, uint64_t us, double inv_t, const uint32_t* __restrict__ grp_node, uint32_t n_groups,
+    const uint32_t* __restrict__ n_pid0, const uint32_t* __restrict__ n_ecount) {
+  __shared__ SoftTables tab;
+  __shared__ double inv_tot[32];
+  extern __shared__ float soft_tile[];   // [edges of the widest node][33]
+  soft_tables_fill(&tab);
+  const uint32_t s0 = blockIdx.y * 32, sw = min(32u, S - s0), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float x[4][2], y[4][2], xn[4][2], yn[4][2];   // 64 edges of up to four sets a warp, and those of the next node
+  const float* const mine = params + (s0 + warp) * ss + lane;   // this lane's edge of the warp's first set; further sets
+  const float* const noise = u + (s0 + warp) * us + lane;       // eight rows on
+  auto fetch = [&](float (&x)[4][2], float (&y)[4][2], uint32_t pid, uint32_t n) {   // n edges from pid
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      if (warp + 8 * k >= sw) break;
+      const float* const px = mine + 8 * k * ss + pid;
+      const float* const py = noise + 8 * k * us + pid;
+#pragma unroll
+      for (uint32_t h = 0; h < 2; ++h) {
+        const bool in = lane + 32 * h < n;
+        x[k][h] = in ? px[32 * h] : 0.0f;
+        if (NOISE) y[k][h] = in ? __ldcs(py + 32 * h) : 0.5f;
+      }
+    }
+  };
+  uint32_t pid0 = 0, cnt = 0, pid1 = 0, cnt1 = 0;   // of this node and of the next one
+  if (blockIdx.x < n_groups) { const uint32_t n = grp_node[blockIdx.x]; pid0 = n_pid0[n]; cnt = n_ecount[n]; }
+  if (blockIdx.x + gridDim.x < n_groups) { const uint32_t n = grp_node[blockIdx.x + gridDim.x]; pid1 = n_pid0[n]; cnt1 = n_ecount[n]; }
+  fetch(x, y, pid0, cnt);
+  for (uint32_t g = blockIdx.x; g < n_groups; g += gridDim.x) {
+    const uint32_t g2 = g + 2 * gridDim.x;
+    const uint32_t n2 = g2 < n_groups ? grp_node[g2] : 0;
+    fetch(xn, yn, pid1, cnt1);
+    const uint32_t pid2 = g2 < n_groups ? n_pid0[n2] : 0, cnt2 = g2 < n_groups ? n_ecount[n2] : 0;
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+    for (uint32_t j0 = 0; j0 < cnt; j0 += 64) {
+      if (j0) fetch(x, y, pid0 + j0, cnt - j0);
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) {
+        if (warp + 8 * k >= sw) break;
+        bool ok = true;
+        float e[2];
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) e[h] = soft_weight_fast<NOISE>(x[k][h], y[k][h], inv_t, &tab, ok);
+        if (!ok)
+#pragma unroll
+          for (uint32_t h = 0; h < 2; ++h) e[h] = soft_weight<NOISE>(x[k][h], y[k][h], inv_t, &tab);
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h)
+          if (j0 + lane + 32 * h < cnt) {
+            soft_tile[(j0 + lane + 32 * h) * 33 + warp + 8 * k] = e[h];
+            sum[k] += e[h];
+          }
+      }
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      if (warp + 8 * k >= sw) break;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+      if (lane == 0) inv_tot[warp + 8 * k] = 1.0 / (double)sum[k];
+    }
+    __syncthreads();
+    const uint32_t step_j = SOFT_THREADS / sw, step_s = SOFT_THREADS % sw;   // 256 elements further in [edge][set] order
+    uint32_t j = threadIdx.x / sw, s = threadIdx.x % sw;
+    float* const out = w + (size_t)pid0 * ld + s0;
+    while (j < cnt) {
+      out[j * ld + s] = (float)((double)soft_tile[j * 33 + s] * inv_tot[s]);   // the quotient, rounded once
+      j += step_j; s += step_s;
+      if (s >= sw) { s -= sw; ++j; }
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+#pragma unroll
+      for (uint32_t h = 0; h < 2; ++h) { x[k][h] = xn[k][h]; y[k][h] = yn[k][h]; }
+    pid0 = pid1; cnt = cnt1; pid1 = pid2; cnt1 = cnt2;
   }
 }
 
@@ -587,14 +693,14 @@ __global__ void __launch_bounds__(SOFT_THREADS) soft_down_kernel(SoftLayer a) {
 }
 
 __global__ void soft_leaf_kernel(const float* __restrict__ td, uint32_t ld, uint32_t S,
-                                 const float* __restrict__ params, uint32_t Sp, uint32_t n_inputs, uint32_t V,
+                                 const float* __restrict__ params, uint64_t ss, uint64_t pld, uint32_t n_inputs, uint32_t V,
                                  const uint32_t* __restrict__ in_node, const uint32_t* __restrict__ in_var,
                                  const uint32_t* __restrict__ in_cats, const uint64_t* __restrict__ in_poff,
                                  uint64_t P, const float* __restrict__ theta, float* __restrict__ out) {
   uint32_t i = blockIdx.x * blockDim.y + threadIdx.y;
   uint32_t s = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= n_inputs || s >= S) return;
-  const size_t ps = Sp == 1 ? 0 : s, pld = Sp;
+  const size_t ps = s * ss;   // parameter p of set s lies at s * ss + p * pld
   float tp = td[(size_t)in_node[i] * ld + s];
   uint32_t C = in_cats[i], var = in_var[i];
   uint64_t off = in_poff[i];
@@ -665,8 +771,8 @@ extern "C" int32_t pcb_sample_hard(pcb_circuit* c, pcb_workspace* ws, const floa
   return PCB_OK;
 }
 
-extern "C" int32_t pcb_sample_soft(pcb_circuit* c, pcb_workspace* ws, const float* params_dev, uint32_t Sp,
-                                   const float* u_dev, float temperature, uint32_t S, float* out_dev, pcb_stream s) {
+static int32_t sample_soft_impl(pcb_circuit* c, pcb_workspace* ws, const float* params_dev, uint32_t Sp,
+                                const float* u_dev, float temperature, uint32_t S, float* out_dev, bool rows, pcb_stream s) {
   PCB_REQUIRE(c && ws && params_dev && out_dev, "null argument");
   PCB_REQUIRE(ws->c == c, "workspace belongs to another circuit");
   PCB_REQUIRE(S >= 1 && (Sp == 1 || Sp == S), "params must hold 1 or S parameter sets");
@@ -682,11 +788,16 @@ extern "C" int32_t pcb_sample_soft(pcb_circuit* c, pcb_workspace* ws, const floa
   PCB_CUDA(cudaMemsetAsync(out_dev, 0, (size_t)S * c->V * c->max_cats * sizeof(float), st));
   if (c->n_groups) {
     // about eight edges per thread: sum nodes that share a pass of a block
-    const uint32_t rows = std::max(1u, std::min(J, J * 8 / std::max(1u, c->max_group)));
-    const uint32_t passes = (c->n_groups + rows - 1) / rows;
+    const uint32_t pass = std::max(1u, std::min(J, J * 8 / std::max(1u, c->max_group)));
+    const uint32_t passes = (c->n_groups + pass - 1) / pass;
     ++c->prof.launches[PCB_K_SAMPLE];
-    soft_params_kernel<<<dim3(std::min(passes, std::max(1u, 148 * 4 / tiles)), tiles), SOFT_THREADS, 0, st>>>(
-        ws->eprob, ld, S, St, rows, params_dev, Sp, u_dev, 1.0 / (double)temperature, c->grp_node, c->n_groups,
+    if (rows)
+      (u_dev ? soft_params_rows_kernel<true> : soft_params_rows_kernel<false>)<<<
+          dim3(std::min(c->n_groups, std::max(1u, 148 * 3 / tiles)), tiles), SOFT_THREADS, c->max_group * 33 * sizeof(float), st>>>(
+          ws->eprob, ld, S, params_dev, Sp == 1 ? 0 : c->P, u_dev, c->n_inner, 1.0 / (double)temperature, c->grp_node,
+          c->n_groups, c->n_pid0, c->n_ecount);
+    else (u_dev ? soft_params_kernel<true> : soft_params_kernel<false>)<<<dim3(std::min(passes, std::max(1u, 148 * 4 / tiles)), tiles), SOFT_THREADS, 0, st>>>(
+        ws->eprob, ld, S, St, pass, params_dev, Sp, u_dev, 1.0 / (double)temperature, c->grp_node, c->n_groups,
         c->n_pid0, c->n_ecount);
   }
   static PcbPerDeviceOnce once;
@@ -719,11 +830,22 @@ extern "C" int32_t pcb_sample_soft(pcb_circuit* c, pcb_workspace* ws, const floa
   if (c->n_inputs) {
     Shape2 sh = shape_for(S, c->n_inputs);
     ++c->prof.launches[PCB_K_SAMPLE];
-    soft_leaf_kernel<<<sh.grid, sh.block, 0, st>>>(td, ld, S, params_dev, Sp, c->n_inputs, c->V, c->in_node, c->in_var,
+    soft_leaf_kernel<<<sh.grid, sh.block, 0, st>>>(td, ld, S, params_dev, rows ? (Sp == 1 ? 0 : c->P) : (Sp == 1 ? 0 : 1), rows ? 1 : Sp, c->n_inputs, c->V, c->in_node, c->in_var,
                                                    c->in_cats, c->in_poff, c->P, c->theta, out_dev);
   }
   PCB_CUDA(cudaGetLastError());
   return PCB_OK;
+}
+
+extern "C" int32_t pcb_sample_soft(pcb_circuit* c, pcb_workspace* ws, const float* params_dev, uint32_t Sp,
+                                   const float* u_dev, float temperature, uint32_t S, float* out_dev, pcb_stream s) {
+  return sample_soft_impl(c, ws, params_dev, Sp, u_dev, temperature, S, out_dev, false, s);
+}
+
+extern "C" int32_t pcb_sample_soft_rows(pcb_circuit* c, pcb_workspace* ws, const float* params_dev, uint32_t Sp,
+                                        const float* u_dev, float temperature, uint32_t S, float* out_dev, pcb_stream s) {
+  PCB_REQUIRE(c && c->max_group <= SOFT_ROWS_K, "row-major sets: at most 256 edges per sum node");
+  return sample_soft_impl(c, ws, params_dev, Sp, u_dev, temperature, S, out_dev, true, s);
 }
 
 // ---- conditioned top-down probabilities ------------------------------------------------------------------
@@ -782,7 +904,7 @@ extern "C" int32_t pcb_cond_td_prob(pcb_circuit* c, pcb_workspace* ws, const int
   if (c->n_inputs) {
     Shape2 sh = shape_for(S, c->n_inputs);
     ++c->prof.launches[PCB_K_SAMPLE];
-    soft_leaf_kernel<<<sh.grid, sh.block, 0, st>>>(td, ld, S, c->theta, 1, c->n_inputs, c->V, c->in_node, c->in_var,
+    soft_leaf_kernel<<<sh.grid, sh.block, 0, st>>>(td, ld, S, c->theta, 0, 1, c->n_inputs, c->V, c->in_node, c->in_var,
                                                    c->in_cats, c->in_poff, c->P, c->theta, out_dev);
   }
   PCB_CUDA(cudaGetLastError());

@@ -431,6 +431,14 @@ function map_pc_parameters!(params1::CuMatrix{Float32}, params2::CuMatrix{Float3
     params1
 end
 
+"Relaxed samples from row-major sets and uniforms ([P, S] and [edges, S] as Julia sees them)"
+function gumbel_sample_rows!(out, c::PcbCircuit, ws, params::CuMatrix{Float32}, u, temperature; S = size(params, 2))
+    check(ccall((:pcb_sample_soft_rows, libpcb200), Int32,
+                (Ptr{Cvoid}, Ptr{Cvoid}, CuPtr{Cfloat}, UInt32, CuPtr{Cfloat}, Cfloat, UInt32, CuPtr{Cfloat}, Ptr{Cvoid}),
+                c.handle, ws, params, size(params, 2), u === nothing ? CU_NULL : u, temperature, S, out, stream()))
+    out
+end
+
 "[S, P] parameters from a row-major buffer ([P, S] as Julia sees it)"
 function param_columns!(dst::CuMatrix{Float32}, src::CuMatrix{Float32})
     check(ccall((:pcb_param_columns, libpcb200), Int32, (CuPtr{Cfloat}, CuPtr{Cfloat}, UInt32, UInt64, Ptr{Cvoid}),

@@ -41,3 +41,19 @@ def test_relaxed_samples_extreme_noise(oracle, temperature):
     out = api.gumbel_sample(m, p, 5, 2, temperature, u=u).cpu().numpy()
     ref = oracle.sample_soft(fc, p, u, temperature, S, 2)[0]
     assert np.isfinite(ref).all() and rel_err(out, ref) <= TOL
+
+
+@pytest.mark.parametrize("v,k,c,S", [(7, 31, 5, 2), (5, 65, 2, 33), (4, 256, 2, 40)])
+def test_relaxed_samples_of_row_major_sets(oracle, v, k, c, S):
+    """Row-major device matrices are read as they are (a remainder of lanes, of warps and of a tile of sets; the widest
+    node the tile takes); the same values from the host, and uniforms with unused columns, go through the columns."""
+    torch, api = _cuda()
+    fc = random_hclt(v, k, c, 3 + v)
+    m = api.CuMetaBitsProbCircuit(fc)
+    p = _param_sets(oracle, fc, S, 1)
+    u = np.random.default_rng(2).random((S, m.num_inner_params), dtype=np.float32)
+    u[:, ::7], u[:, 1::7] = 0.0, 1 - 2.0 ** -24
+    ref = oracle.sample_soft(fc, p, u, 0.7, S, c)[0]
+    wide = torch.from_numpy(np.concatenate([u, u[:, :3]], 1)).cuda()
+    for pp, uu in ((torch.from_numpy(p).cuda(), torch.from_numpy(u).cuda()), (p, u), (torch.from_numpy(p).cuda(), wide)):
+        assert rel_err(api.gumbel_sample(m, pp, v, c, 0.7, u=uu).cpu().numpy(), ref) <= TOL
