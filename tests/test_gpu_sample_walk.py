@@ -31,3 +31,27 @@ def test_samples_equal_the_oracle(oracle, v, k, c, S, per_sample, extreme):
             u.reshape(-1)[::3] = 0.5
     x = api.sample(m, p if per_sample else p[0], u_sum, u_leaf).cpu().numpy()
     assert np.array_equal(x, oracle.sample_hard(fc, p if per_sample else p[0], u_sum, u_leaf, S))
+
+
+@pytest.mark.parametrize("v,k,c,S", [(12, 16, 2, 300), (9, 70, 70, 900), (20, 17, 9, 2400)])
+@pytest.mark.parametrize("lo,hi,impossible", [(-95.0, -85.0, False), (-89.0, -88.0, True), (-300.0, -80.0, True)])
+def test_low_log_weights(oracle, v, k, c, S, lo, hi, impossible):
+    """Sets that are not normalised: every log-weight of a node lies where its exponential, or the race time, leaves the
+    fp32 range; with and without impossible entries beside them.  Both walks."""
+    torch, api = _cuda()
+    fc = random_hclt(v, k, c, v + k)
+    m = api.CuMetaBitsProbCircuit(fc)
+    rng = np.random.default_rng(k)
+    p = rng.uniform(lo, hi, fc.num_parameters).astype(np.float32)
+    if impossible:
+        p[::3] = -np.inf
+    shp = api.noise_shapes(m, S)
+    u_sum, u_leaf = rng.random(shp[0], dtype=np.float32), rng.random(shp[1], dtype=np.float32)
+    for u in (u_sum, u_leaf):   # next to one: the smallest race times
+        u.reshape(-1)[::5] = 1 - rng.random(u.reshape(-1)[::5].size).astype(np.float32) * 1e-2
+    want = oracle.sample_hard(fc, p, u_sum, u_leaf, S)
+    assert np.array_equal(api.sample(m, p, u_sum, u_leaf).cpu().numpy(), want)
+    n = min(S, 100)
+    x = torch.empty(v, n, dtype=torch.int32, device="cuda").t()
+    api.sample_static(m, torch.from_numpy(p).cuda()[:, None], torch.from_numpy(u_sum[:n]).cuda(), torch.from_numpy(u_leaf[:n]).cuda(), x)
+    assert np.array_equal(x.cpu().numpy(), want[:n])
