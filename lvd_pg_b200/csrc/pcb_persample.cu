@@ -294,7 +294,8 @@ __global__ void __launch_bounds__(NB_TPB) norm_block_kernel(
   float* const w = x + (size_t)K * NB_EX;               // [NB_PAR][K]
   {
     const uint32_t e = threadIdx.x % NB_EX, b = b0 + e;
-    const float m = b < B ? blk_mx[(size_t)blk.mx_row * ld + b] : 0.0f;
+    const float top = b < B ? blk_mx[(size_t)blk.mx_row * ld + b] : 0.0f;
+    const float m = top == -INFINITY ? INFINITY : top;   // an example for which no child is possible: exp(x - inf) = 0
 #pragma unroll 4
     for (uint32_t j = threadIdx.x / NB_EX; j < K; j += NB_TPB / NB_EX) {
       float t = 0.0f;

@@ -70,3 +70,57 @@ def flat_stats(fc, edge_aggr_down, heap, edge2param):
         out[pos:pos + c] = heap[hs + c:hs + 2 * c]
         pos += c
     return out
+
+
+def under_one_root(fcs, children, user_tag=False):
+    """One circuit over the nodes and variables of `fcs` with a new root sum on top: `children` are (circuit, 1-based
+    node id) pairs, equally weighted; `user_tag` makes it the fake root of a multi-head circuit.  Runs of consecutive
+    nodes stay consecutive."""
+    from lvd_pg_b200.circuit import PCB_SUM, TAG_FIRST, TAG_LAST, TAG_USER, finish_flat
+    node0 = np.concatenate([[0], np.cumsum([f.num_nodes for f in fcs])])
+    heap0 = np.concatenate([[0], np.cumsum([len(f.heap) for f in fcs])])
+    cat = lambda xs: np.concatenate([np.asarray(x, np.int64) for x in xs])
+    up = {"up_parent": [], "up_prime": [], "up_sub": [], "up_logp": [], "up_tag": []}
+    ends, total = [], 0
+    for lay in range(max(len(f.up_layer_ends) for f in fcs)):
+        for f, n0 in zip(fcs, node0):
+            if lay >= len(f.up_layer_ends):
+                continue
+            sl = slice(int(f.up_layer_ends[lay - 1]) if lay else 0, int(f.up_layer_ends[lay]))
+            for name in up:
+                x = getattr(f, name)[sl]
+                if name in ("up_parent", "up_prime", "up_sub"):
+                    x = np.where(x > 0, x.astype(np.int64) + n0, 0)
+                up[name].append(x)
+            total += sl.stop - sl.start
+        ends.append(total)
+    h = len(children)
+    root = int(node0[-1]) + 1
+    up["up_parent"].append(np.full(h, root))
+    up["up_prime"].append(np.array([node0[i] + n for i, n in children]))
+    up["up_sub"].append(np.zeros(h, np.int64))
+    up["up_logp"].append(np.full(h, -np.log(h), np.float32))
+    tag = np.full(h, TAG_USER if user_tag else 0, np.uint8)
+    tag[0] |= TAG_FIRST
+    tag[-1] |= TAG_LAST
+    up["up_tag"].append(tag)
+    ends.append(total + h)
+    kind = np.concatenate([f.node_kind for f in fcs] + [[PCB_SUM]])
+    hstart = cat([np.where(f.node_num_cats > 0, f.node_heap_start.astype(np.int64) + o, 0) for f, o in zip(fcs, heap0)] + [[0]])
+    return finish_flat(kind, cat([f.node_var for f in fcs] + [[0]]), cat([f.node_num_cats for f in fcs] + [[0]]), hstart,
+                       cat([f.node_fixed for f in fcs] + [[0]]), cat(up["up_parent"]), cat(up["up_prime"]), cat(up["up_sub"]),
+                       np.concatenate(up["up_logp"]), np.concatenate(up["up_tag"]), ends,
+                       cat([f.input_node_ids.astype(np.int64) + n for f, n in zip(fcs, node0)]),
+                       np.concatenate([f.heap for f in fcs]), max(f.num_vars for f in fcs))
+
+
+def without_root(fc):
+    """`fc` without its last node and that node's edges: nodes for `under_one_root`, no circuit of its own."""
+    out = fc.copy()
+    keep = fc.up_parent != fc.num_nodes
+    for name in ("up_parent", "up_prime", "up_sub", "up_logp", "up_tag"):
+        setattr(out, name, getattr(fc, name)[keep])
+    out.up_layer_ends = np.unique(np.cumsum(keep)[fc.up_layer_ends.astype(np.int64) - 1])
+    for name in ("node_kind", "node_var", "node_num_cats", "node_heap_start", "node_fixed"):
+        setattr(out, name, getattr(fc, name)[:-1])
+    return out
