@@ -58,6 +58,9 @@ __device__ __forceinline__ float4 max4(float4 a, float4 b) {
 __device__ __forceinline__ float4 exp4(float4 v, float4 m) {   // exp(v - m)
   return make_float4(__expf(v.x - m.x), __expf(v.y - m.y), __expf(v.z - m.z), __expf(v.w - m.w));
 }
+__device__ __forceinline__ float4 exp4_below(float4 mx, float4 v) {
+  return make_float4(pcb_exp_below(mx.x, v.x), pcb_exp_below(mx.y, v.y), pcb_exp_below(mx.z, v.z), pcb_exp_below(mx.w, v.w));
+}
 __device__ __forceinline__ float4 splat(float v) { return make_float4(v, v, v, v); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 
@@ -284,7 +287,7 @@ __global__ void __launch_bounds__(TPB, BATCH <= 2 ? 4 : 2) chain_down_kernel(Cha
       for (uint32_t u = 0; u < BATCH; ++u) v[u] = r1 + RSTEP * u < R ? ld4(a.mars + (size_t)(k.p0 + r1 + RSTEP * u) * ld + b) : splat(0.0f);
 #pragma unroll
       for (uint32_t u = 0; u < BATCH; ++u)
-        if (r1 + RSTEP * u < R) st4(y + (r1 + RSTEP * u) * XP + q * 4, exp4(mx, v[u]));
+        if (r1 + RSTEP * u < R) st4(y + (r1 + RSTEP * u) * XP + q * 4, exp4_below(mx, v[u]));
     }
     float2 xv[2][2];   // exp(M - mx) of this thread's outputs: [examples 8 j][children 8 h]
 #pragma unroll

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(NT) dense_bwd_child_kernel(float* __restrict__
         float g = 0.0f;
         if (r < k.R && b < ld && mx != -INFINITY) {
           size_t o = (size_t)(k.p0 + r) * ld + b;
-          g = flows[o] * __expf(mx - mars[o]);
+          g = flows[o] * pcb_exp_below(mx, mars[o]);
         }
         Gs[rl][bl] = g;
       }

@@ -449,8 +449,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) dense_mn_kernel(const __grid_cons
 #pragma unroll
         for (uint32_t ps = 0; ps < 2; ++ps) {
           float4 v;   // x: mars of the parent, y: flows of the parent
-          v.x = r.y[ps].x * __expf(mx4.x - r.x[ps].x); v.y = r.y[ps].y * __expf(mx4.y - r.x[ps].y);
-          v.z = r.y[ps].z * __expf(mx4.z - r.x[ps].z); v.w = r.y[ps].w * __expf(mx4.w - r.x[ps].w);
+          v.x = r.y[ps].x * pcb_exp_below(mx4.x, r.x[ps].x); v.y = r.y[ps].y * pcb_exp_below(mx4.y, r.x[ps].y);
+          v.z = r.y[ps].z * pcb_exp_below(mx4.z, r.x[ps].z); v.w = r.y[ps].w * pcb_exp_below(mx4.w, r.x[ps].w);
           if ((cb + i) * KC + ps * 8u + warp >= kdim) v = make_float4(0.f, 0.f, 0.f, 0.f);
           const float4 h = make_float4(tf32_hi(v.x), tf32_hi(v.y), tf32_hi(v.z), tf32_hi(v.w));
           const uint32_t o = aoff + ps * 4096u;

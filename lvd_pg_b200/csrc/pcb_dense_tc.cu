@@ -383,7 +383,7 @@ __device__ __forceinline__ void store_chunk(const ProdCtx& c, const ProdInv& v, 
 #pragma unroll
       for (uint32_t j = 0; j < 4; ++j) {
         const float val = MODE == MODE_FWD ? __expf(r.ra[q * 4 + j] - v.mx4[j])
-                                           : r.ra[q * 4 + j] * __expf(v.mx4[j] - r.rm[q * 4 + j]);
+                                           : r.ra[q * 4 + j] * pcb_exp_below(v.mx4[j], r.rm[q * 4 + j]);
         put_split(a_hi, a_lo, sw_off(row0 + j, kk), val);
       }
     }
@@ -397,7 +397,7 @@ __device__ __forceinline__ void store_chunk(const ProdCtx& c, const ProdInv& v, 
 #pragma unroll
       for (uint32_t q = 0; q < 8; ++q) {
         const float val = MODE == MODE_FWD ? __expf(r.ra[g * 8 + q] - v.mx[g])
-                                           : r.ra[g * 8 + q] * __expf(v.mx[g] - r.rm[g * 8 + q]);
+                                           : r.ra[g * 8 + q] * pcb_exp_below(v.mx[g], r.rm[g * 8 + q]);
         put_split(a_hi, a_lo, base + ((q ^ r7) << 4), val);
       }
     }

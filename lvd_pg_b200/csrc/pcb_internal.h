@@ -380,6 +380,9 @@ __device__ __forceinline__ void pcb_copy4_async(float* dst, const float* src) {
 __device__ __forceinline__ void pcb_copy16_async(float* dst, const float* src) {   // both 16-byte aligned
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
+// exp(mx - value) for the flow of a sum node whose value lies that far below its block's maximum.  Beyond e^87 the node has
+// next to none of the block's flow (none at all where its value is -inf): the clamp keeps 0 * inf out of the sums.
+__device__ __forceinline__ float pcb_exp_below(float mx, float value) { return __expf(fminf(mx - value, 87.0f)); }
 __device__ __forceinline__ void pcb_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 #endif
 

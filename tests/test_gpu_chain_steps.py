@@ -74,3 +74,39 @@ def test_impossible_children(oracle):
     api.backward(m, ws)
     flows_ref, _ = oracle.backward(ref, mars_ref)
     assert rel_err(m.flows(ws, B)[possible], flows_ref[possible]) <= TOL
+
+
+@pytest.mark.parametrize("impl", [{}, {"PCB_CHAIN": "0"}, {"PCB_TC_IMPL": "km"}, {"PCB_DENSE_IMPL": "simt"}],
+                         ids=["rule", "tensor", "km", "simt"])
+@pytest.mark.parametrize("k,rows", [(32, 97), (72, 40)])
+def test_dead_state(oracle, monkeypatch, impl, k, rows):
+    """A latent state that cannot have produced some rows, and one that is e^100 less likely than its neighbours, in
+    blocks that are possible otherwise: their value lies far below the block's maximum, their flow is 0, and the flows of
+    the children do not see them.  The oracle takes -1e4 for -inf (0 * exp(-inf + inf) has no value)."""
+    for key, val in impl.items():
+        monkeypatch.setenv(key, val)
+    torch, api = _cuda()
+    fcs = []
+    for zero in (-np.inf, -1e4):
+        fc = st.hclt_flat(_tree("random", 9), 3, k, seed=5)
+        start = fc.node_heap_start.astype(np.int64) - 1
+        sums = np.nonzero(np.bincount(fc.up_parent[fc.edge_is_sum].astype(np.int64), minlength=fc.num_nodes + 1) == k)[0]
+        blocks = sums[sums != fc.num_nodes].reshape(-1, k)      # consecutive states of one variable
+        assert np.all(np.diff(blocks, axis=1) == 1)
+        for rows_of in blocks:
+            for state, value in ((3, zero), (7, -100.0)):       # all weight on one child, whose leaf never takes category 0
+                e = np.nonzero(fc.up_parent == rows_of[state])[0]
+                fc.up_logp[e] = zero
+                fc.up_logp[e[5 + state]] = 0.0
+                fc.heap[start[int(fc.up_sub[e[5 + state]]) - 1]] = value
+        fcs.append(fc)
+    data, _ = random_data(rows, 9, 3, 9)
+    ref, m = fcs[1], api.CuMetaBitsProbCircuit(fcs[0])
+    mars_ref = oracle.forward(ref, data)
+    flows_ref, _ = oracle.backward(ref, mars_ref)
+    ws, B = api.forward(m, api.DeviceData(data, m.device))
+    api.backward(m, ws)
+    dead = mars_ref < mars_ref.max(1, keepdims=True) - 5000.0
+    assert dead.any() and np.isfinite(mars_ref[:, -1]).all() and not dead[:, -1].any()
+    assert rel_err(m.mars(ws, B)[:, -1], mars_ref[:, -1]) <= TOL
+    assert rel_err(m.flows(ws, B), flows_ref) <= TOL
