@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(TPB, 2) edge_narrow_kernel(
       const uint32_t r = g + 32 * u;
       float4 y = splat(0.0f), x = splat(0.0f);
       if (r < rows) {
-        const float4 e = exp4(mx, pm[u]);
+        const float4 e = exp4_below(mx, pm[u]);
         y = make_float4(v0 ? pf[u].x * e.x : 0.f, v1 ? pf[u].y * e.y : 0.f, v2 ? pf[u].z * e.z : 0.f, v3 ? pf[u].w * e.w : 0.f);
       }
       if (r < cols) {

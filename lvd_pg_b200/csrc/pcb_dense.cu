@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(NT) dense_bwd_edge_kernel(const float* __restr
       float g = 0.0f;
       if (bok && r < k.R && mx != -INFINITY) {
         size_t o = (size_t)(k.p0 + r) * ld + b;
-        g = flows[o] * __expf(mx - mars[o]);
+        g = flows[o] * pcb_exp_below(mx, mars[o]);
       }
       Gs[rl][bl] = g;
     }

@@ -410,9 +410,9 @@ __device__ __forceinline__ void store_chunk(const ProdCtx& c, const ProdInv& v, 
       // masked through the max (exp(-inf) = 0) instead of per element
       static_assert(PW % 8 == 0, "row & 7 must not depend on q");
       const uint32_t base = w * 128u + (((cpos ^ (w & 7u)) << 4) | csub);
-      const float mxa = r.vok ? r.mx : -INFINITY, mxb = r.vok ? r.mx : INFINITY;
+      const float mxb = r.vok ? r.mx : INFINITY;
 #pragma unroll
-      for (uint32_t q = 0; q < QA; ++q) put_split(a_hi, a_lo, base + q * (PW * 128u), r.ra[q] * __expf(mxa - r.rm[q]));
+      for (uint32_t q = 0; q < QA; ++q) put_split(a_hi, a_lo, base + q * (PW * 128u), r.vok ? r.ra[q] * pcb_exp_below(r.mx, r.rm[q]) : 0.0f);
       if (tmark) *tmark = gtime();
 #pragma unroll
       for (uint32_t q = 0; q < QB; ++q) put_split(b_hi, b_lo, base + q * (PW * 128u), __expf(r.rb[q] - mxb));
@@ -422,7 +422,7 @@ __device__ __forceinline__ void store_chunk(const ProdCtx& c, const ProdInv& v, 
     for (uint32_t q = 0; q < QA; ++q) {
       const uint32_t row = w + PW * q;
       const bool ok = r.vok && (v.rmask >> q & 1u);
-      put_split(a_hi, a_lo, row * 128u + (((cpos ^ (row & 7u)) << 4) | csub), ok ? r.ra[q] * __expf(r.mx - r.rm[q]) : 0.0f);
+      put_split(a_hi, a_lo, row * 128u + (((cpos ^ (row & 7u)) << 4) | csub), ok ? r.ra[q] * pcb_exp_below(r.mx, r.rm[q]) : 0.0f);
     }
     if (tmark) *tmark = gtime();
 #pragma unroll

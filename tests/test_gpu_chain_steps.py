@@ -81,8 +81,8 @@ def test_impossible_children(oracle):
 @pytest.mark.parametrize("k,rows", [(32, 97), (72, 40)])
 def test_dead_state(oracle, monkeypatch, impl, k, rows):
     """A latent state that cannot have produced some rows, and one that is e^100 less likely than its neighbours, in
-    blocks that are possible otherwise: their value lies far below the block's maximum, their flow is 0, and the flows of
-    the children do not see them.  The oracle takes -1e4 for -inf (0 * exp(-inf + inf) has no value)."""
+    blocks that are possible otherwise: their value lies far below the block's maximum, their flow is 0, and neither the
+    flows of the children nor the statistics see them.  The oracle takes -1e4 for -inf (0 * exp(-inf + inf) has no value)."""
     for key, val in impl.items():
         monkeypatch.setenv(key, val)
     torch, api = _cuda()
@@ -103,10 +103,13 @@ def test_dead_state(oracle, monkeypatch, impl, k, rows):
     data, _ = random_data(rows, 9, 3, 9)
     ref, m = fcs[1], api.CuMetaBitsProbCircuit(fcs[0])
     mars_ref = oracle.forward(ref, data)
-    flows_ref, _ = oracle.backward(ref, mars_ref)
+    flows_ref, aggr_ref = oracle.backward(ref, mars_ref)
     ws, B = api.forward(m, api.DeviceData(data, m.device))
+    m.lib.pcb_clear_flows(m.handle, 0.0, None)
     api.backward(m, ws)
     dead = mars_ref < mars_ref.max(1, keepdims=True) - 5000.0
     assert dead.any() and np.isfinite(mars_ref[:, -1]).all() and not dead[:, -1].any()
     assert rel_err(m.mars(ws, B)[:, -1], mars_ref[:, -1]) <= TOL
     assert rel_err(m.flows(ws, B), flows_ref) <= TOL
+    sum_edges = ref.edge_is_sum[ref.down2up.astype(np.int64) - 1]
+    assert rel_err(m.edge_aggr()[sum_edges], aggr_ref[sum_edges]) <= TOL
