@@ -134,6 +134,55 @@ __device__ __forceinline__ void contract(float (&acc)[2][4], const float* w, uin
   }
 }
 
+// the maximum / sum over the rows of a tile's example quads: over the four rows of a warp, then over the warps
+template <typename Op>
+__device__ __forceinline__ float4 over_rows(float4 v, float4 (&red)[TPB / 32][8], Op op) {
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (uint32_t o = 8; o < 32; o <<= 1)
+    v = op(v, make_float4(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o),
+                          __shfl_xor_sync(0xffffffffu, v.z, o), __shfl_xor_sync(0xffffffffu, v.w, o)));
+  __syncthreads();   // what `red` held has been read
+  if (lane < 8) red[warp][lane] = v;
+  __syncthreads();
+  v = red[0][lane & 7];
+#pragma unroll
+  for (uint32_t u = 1; u < TPB / 32; ++u) v = op(v, red[u][lane & 7]);
+  return v;
+}
+
+// A single sum node over consecutive children (the root, so the likelihood itself): in fp32 and with the weights inside
+// the maximum, as the kernel of single nodes sums it, so that children far below one without weight count in full.
+__device__ __forceinline__ void up_single(const ChainArgs& a, const PcbDenseBlock& k, float* w, float4 (&red)[TPB / 32][8]) {
+  const uint32_t q = threadIdx.x & 7, g = threadIdx.x >> 3, ld = a.ld, K = k.K;
+  float* const x = w + ((K + 3u) & ~3u);   // [K][XP]
+  for (uint32_t t = threadIdx.x; t < K; t += TPB) w[t] = a.theta[k.pid0 + t];
+  __syncthreads();
+  pcb_grid_dep_wait();   // everything above is the step's parameters
+  for (uint32_t tile = blockIdx.x % a.tile_ctas; tile < a.tiles; tile += a.tile_ctas) {
+    const uint32_t b = tile * EX + q * 4;
+    const float* const pa = a.mars + (size_t)k.c0 * ld + b;
+    const float* const pb = a.mars + (size_t)(k.d0 != PCB_NONE ? k.d0 : k.c0) * ld + b;
+    float4 mx = splat(-INFINITY);
+#pragma unroll 2
+    for (uint32_t t = g; t < K; t += RSTEP) {
+      float4 v = ld4(pa + (size_t)t * ld);
+      if (k.d0 != PCB_NONE) v = add4(v, ld4(pb + (size_t)t * ld));
+      v = add4(v, splat(w[t]));
+      mx = max4(mx, v);
+      st4(x + t * XP + q * 4, v);
+    }
+    mx = over_rows(mx, red, [](float4 u, float4 v) { return max4(u, v); });
+    float4 s = splat(0.0f);   // an example for which no child is possible: NaN here, -inf below
+    for (uint32_t t = g; t < K; t += RSTEP) s = add4(s, exp4(*reinterpret_cast<const float4*>(x + t * XP + q * 4), mx));
+    s = over_rows(s, red, [](float4 u, float4 v) { return add4(u, v); });
+    if (g == 0)
+      st4(a.mars + (size_t)k.p0 * ld + b,
+          make_float4(mx.x == -INFINITY ? -INFINITY : __logf(s.x) + mx.x, mx.y == -INFINITY ? -INFINITY : __logf(s.y) + mx.y,
+                      mx.z == -INFINITY ? -INFINITY : __logf(s.z) + mx.z, mx.w == -INFINITY ? -INFINITY : __logf(s.w) + mx.w));
+  }
+}
+
 // mars[r][b] = log(sum_t exp(theta[r][t]) * exp(M[t][b] - mx[b])) + mx[b], M = prime + sub, mx the maximum over t.
 // A CTA walks the example tiles tile0, tile0 + tile_ctas, ... with its weights in place; the first rows of the next tile
 // are fetched while this one is multiplied.  BATCH: rows per thread whose loads are in flight together.
@@ -153,6 +202,10 @@ __global__ void __launch_bounds__(TPB, BATCH <= 2 ? 4 : 2) chain_up_kernel(Chain
   const uint32_t rest = blockIdx.x / a.tile_ctas, bi = rest / a.chunks, r0 = rest % a.chunks * OUT;
   const PcbDenseBlock k = bi < a.nblk ? a.blk[bi] : a.thin[bi - a.nblk];
   if (r0 >= k.R) return;
+  if (bi >= a.nblk) {
+    up_single(a, k, reinterpret_cast<float*>(chain_smem), red);
+    return;
+  }
   const uint32_t rows = min(OUT, k.R - r0), K = k.K, K8 = (K + 7u) & ~7u, wp = K8 + 4u, ld = a.ld;
   float* const w = reinterpret_cast<float*>(chain_smem);   // [OUT][wp]
   float* const x = w + OUT * wp;                           // [K8][XP]
@@ -218,7 +271,7 @@ __global__ void __launch_bounds__(TPB, BATCH <= 2 ? 4 : 2) chain_up_kernel(Chain
     for (uint32_t u = 0; u < TPB / 32; ++u) mx = max4(mx, red[u][q]);
     if (g == 0) {
       st4(mxs + q * 4, mx);
-      if (r0 == 0 && k.mx_row != PCB_NONE) st4(a.blk_mx + (size_t)k.mx_row * ld + b, mx);
+      if (r0 == 0) st4(a.blk_mx + (size_t)k.mx_row * ld + b, mx);
     }
     // an example for which no child is possible: exp(x - inf) = 0
     const float4 sh = make_float4(mx.x == -INFINITY ? INFINITY : mx.x, mx.y == -INFINITY ? INFINITY : mx.y,

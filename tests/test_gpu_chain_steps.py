@@ -113,3 +113,24 @@ def test_dead_state(oracle, monkeypatch, impl, k, rows):
     assert rel_err(m.flows(ws, B), flows_ref) <= TOL
     sum_edges = ref.edge_is_sum[ref.down2up.astype(np.int64) - 1]
     assert rel_err(m.edge_aggr()[sum_edges], aggr_ref[sum_edges]) <= TOL
+
+
+@pytest.mark.parametrize("weight", [-np.inf, -200.0, -110.0])
+def test_root_of_unlikely_states(oracle, weight):
+    """The root's most likely child has (almost) no weight: the others, e^150 below it, make up the likelihood."""
+    torch, api = _cuda()
+    k = 32
+    fc = st.hclt_flat(_tree("random", 8), 3, k, seed=5)
+    start = fc.node_heap_start.astype(np.int64) - 1
+    e = np.nonzero(fc.up_parent == fc.num_nodes)[0]
+    leaves = start[fc.up_sub[e].astype(np.int64) - 1]
+    fc.heap[leaves[1:]] = -150.0          # category 0 of the root's variable is next to impossible but in state 0
+    fc.up_logp[e[0]] = weight
+    data, _ = random_data(70, 8, 3, 9)
+    m = api.CuMetaBitsProbCircuit(fc)
+    mars_ref = oracle.forward(fc, data)
+    ws, B = api.forward(m, api.DeviceData(data, m.device))
+    assert rel_err(m.mars(ws, B)[:, -1], mars_ref[:, -1]) <= TOL
+    flows_ref, _ = oracle.backward(fc, mars_ref)
+    api.backward(m, ws)
+    assert rel_err(m.flows(ws, B), flows_ref) <= TOL
