@@ -228,7 +228,9 @@ int32_t compile(const pcb_circuit_desc* d, pcb_circuit* c) {
   std::vector<uint8_t> in_dense(N, 0), dense_child(N, 0);
   c->h_dense.clear();
   c->h_dense_off.assign(c->L + 2, 0);
-  auto indeg = [&](uint32_t n) { return in_off[n + 1] - in_off[n]; };
+  // a head counts as one more parent: its flow starts at the mask, so neither a block nor a fused product may own it,
+  // and the fake root reads its value
+  auto indeg = [&](uint32_t n) { return in_off[n + 1] - in_off[n] + (node_head[n] != PCB_NONE ? 1u : 0u); };
   for (uint32_t lay = 1; lay <= c->L; ++lay) {
     c->h_dense_off[lay] = (uint32_t)c->h_dense.size();
     auto& ln = layer_nodes[lay];

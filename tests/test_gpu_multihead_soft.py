@@ -5,7 +5,7 @@ import pytest
 
 from lvd_pg_b200 import structures as st
 from lvd_pg_b200.circuit import Sum, compile_circuit, compile_multihead
-from tests.helpers import random_data, rel_err
+from tests.helpers import random_data, rel_err, under_one_root
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-4  # relative, fp32
@@ -241,3 +241,40 @@ def test_soft_regularised_leaves(oracle, width):
         assert abs(float(lls.item()) - ll_ref) <= TOL * abs(ll_ref)
         p = api.vectorize_parameters(m)
         assert np.abs(np.exp(p) - np.exp(oracle.vectorize(ref))).max() <= TOL
+
+
+@pytest.mark.parametrize("kind", ["factor_of_a_product", "child_of_a_block", "product"])
+@pytest.mark.parametrize("chain", ["1", "0"])
+def test_heads_inside_the_circuit(oracle, monkeypatch, kind, chain):
+    """A head that is an inner node of another head's circuit: its flow is what its parents send and its own mask."""
+    monkeypatch.setenv("PCB_CHAIN", chain)
+    torch, api = _cuda()
+    # variable 1, below the root, has two inner children, 2 and 3 (products of their states); 4 is alone below 2
+    parent = np.array([-1, 0, 1, 1, 2, 3, 4], np.int64)
+    k = 16
+    flat = st.hclt_flat(parent, 3, k, seed=4)
+    prod = np.nonzero(flat.node_kind == 1)[0]
+    assert len(prod) == k
+    if kind == "product":
+        head = int(prod[2]) + 1
+    elif kind == "factor_of_a_product":
+        head = int(flat.up_prime[flat.up_parent == prod[2] + 1][0])
+    else:   # prime children of sums that are not products: the states below a single child
+        e = flat.edge_is_sum & (flat.node_kind[flat.up_prime.astype(np.int64) - 1] == 2)
+        head = int(np.unique(flat.up_prime[e])[2])
+    fc = under_one_root([flat], [(0, flat.num_nodes), (0, head)], user_tag=True)
+    roots = np.array([flat.num_nodes, head], np.uint32)
+    m = api.CuMultiHeadBitsProbCircuit(fc)
+    assert m.root_ids.tolist() == roots.tolist()
+    data, _ = random_data(70, 7, 3, 5)
+    mask = _mask(70, 2, 9)
+    dd, dmask = api.DeviceData(data, m.device), api.colmajor(mask, m.device)
+    mars_ref = oracle.forward_ex(fc, data)
+    flows_ref, aggr_ref = oracle.backward_ex(fc, mars_ref, roots, mask)
+    ws, B = api.forward_ex(m, dd, head_mask=dmask)
+    m.lib.pcb_clear_flows(m.handle, 0.0, None)
+    api.backward(m, ws)
+    assert rel_err(m.mars(ws, B), mars_ref) <= TOL
+    assert rel_err(m.flows(ws, B), flows_ref) <= TOL
+    sum_edges = fc.edge_is_sum[fc.down2up.astype(np.int64) - 1]
+    assert rel_err(m.edge_aggr()[sum_edges], aggr_ref[sum_edges]) <= TOL
