@@ -672,6 +672,9 @@ int32_t pcb_ws_ensure_sets(pcb_workspace* ws, uint32_t S, int need) {
   if ((need & (PCB_WS_NODES | PCB_WS_EDGES)) && S > ws->S_cap) {
     for (void* p : {(void*)ws->klds, (void*)ws->grads, (void*)ws->eprob}) if (p) cudaFree(p);
     ws->klds = ws->grads = ws->eprob = nullptr;
+    if (ws->kld_exec) cudaGraphExecDestroy(ws->kld_exec);   // recorded with these buffers
+    ws->kld_exec = nullptr;
+    ws->have_kld_key = false;
     ws->S_cap = S;
     // a handful of sets stays unpadded: the per-node values of neighbouring nodes then share 32-byte
     // sectors, which is what the gathers of a single-set KLD chain pay for

@@ -36,3 +36,25 @@ def test_param_columns(S, P):
     y = api._columns(m, x)
     assert y.is_contiguous() and torch.equal(y, x.t())
     assert torch.equal(api._columns(m, x[:, ::2]), x[:, ::2].t())    # not row-major: the general path
+
+
+def test_adam_steps_around_more_sets(oracle):
+    """A KLD of several sets grows the buffers that the captured single-set step was recorded with."""
+    torch, api = _cuda()
+    fc = random_hclt(8, 17, 3, 4)
+    sets = _param_sets(oracle, fc, 40, 1)
+    p, q0 = torch.from_numpy(sets[0]).cuda(), torch.from_numpy(sets[1])
+    got = []
+    for others in (False, True):
+        m = api.CuMetaBitsProbCircuit(fc)
+        opt = api.KldAdam(m, q0.cuda().clone(), p)
+        klds = []
+        for step in range(9):
+            if others and step in (4, 7):
+                S = 12 if step == 4 else 40
+                api.kld(m, torch.from_numpy(sets[:S]).cuda(), torch.from_numpy(sets[:S][::-1].copy()).cuda())
+            klds.append(opt.step().item())
+        got.append((klds, opt.q.cpu().numpy()))
+    # the sums of the node gradients are atomics: their order differs from run to run
+    np.testing.assert_allclose(got[1][0], got[0][0], rtol=1e-5)
+    np.testing.assert_allclose(got[1][1], got[0][1], rtol=1e-4, atol=1e-4)
