@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(LST) leaf_flow_sorted_kernel(
   }
 }
 
-// Leaf statistics, lanes over leaves.  A block takes 32 leaves of one variable and walks the batch in slices of 256
+// Leaf statistics, lanes over leaves.  A block takes 32 leaves of one variable and walks its share of the batch in slices of 256
 // examples: the rows of the leaves land in a tile in shared memory (16-byte loads along the examples, XOR-swizzled so
 // that a column of 32 leaves lies in 32 banks; the next slice is in flight), then every warp walks its eighth of the
 // slice's examples IN SORTED ORDER OF THEIR VALUE with one leaf per lane.  All lanes meet the same value at the same
@@ -466,11 +466,12 @@ __global__ void __launch_bounds__(LTT) leaf_flow_tile_kernel(
       }
     }
   };
-  fetch(0);
+  const uint32_t first = blockIdx.y * LTS, step = gridDim.y * LTS;   // this block's slices
+  fetch(first);
   for (uint32_t x = threadIdx.x; x < LTL * pitch; x += LTT) lt_hist[x] = 0.0f;
   float* const h = lt_hist + lane * pitch;
   const float* const column = tile + lane * LTS;
-  for (uint32_t b0 = 0; b0 < B; b0 += LTS) {
+  for (uint32_t b0 = first; b0 < B; b0 += step) {
     const uint32_t word = __ldg(order + ((size_t)(b0 / LTS) * V + var) * LTS + threadIdx.x);   // 32 sorted examples of this warp
     __syncthreads();   // the tile has been read (and, first, the histograms are clear)
     float4* const to = reinterpret_cast<float4*>(tile) + warp * 4 * (LTS / 4);
@@ -483,7 +484,7 @@ __global__ void __launch_bounds__(LTT) leaf_flow_tile_kernel(
       to[3 * (LTS / 4) + g] = make_float4(next[3][u].w, next[3][u].z, next[3][u].y, next[3][u].x);
     }
     __syncthreads();
-    if (b0 + LTS < B) fetch(b0 + LTS);
+    if (b0 + step < B) fetch(b0 + step);
     uint32_t seg = __shfl_sync(0xffffffffu, word, 0) >> 16;
     const uint32_t last = __shfl_sync(0xffffffffu, word, 31) >> 16;
     bool edge = true;   // the first run may have begun in the warp before
@@ -1234,7 +1235,13 @@ static int32_t backward_impl(pcb_circuit* c, pcb_workspace* ws, const float* wei
       }));
       if (sorted_beside) PCB_CUDA(cudaStreamWaitEvent(st, c->ev_sort, 0));
       auto* kern = weights_dev ? leaf_flow_tile_kernel<true> : leaf_flow_tile_kernel<false>;
-      kern<<<c->n_lgrps * LTG, LTT, LTL * ((c->max_cats + 2) | 1u) * sizeof(float), st>>>(
+      // few leaves and many examples: the slices of a batch are dealt out so that there are about four blocks per SM
+      // (a step of 8 variables x 16 latents x 65536 examples: 2 categories 1150 -> 252 us, 100 categories 1343 -> 261 us;
+      // 64 variables x 16384 examples x 100 categories 752 -> 443 us)
+      const uint32_t tiles = std::max(c->n_lgrps, (c->n_inputs + LTL - 1) / LTL), slices = (B + LTS - 1) / LTS;
+      // (and no histogram adds up more than 256 slices one after the other)
+      const uint32_t parts = std::min(65535u, std::max((slices + 255) / 256, std::min(slices, 148 * 4 / tiles)));
+      kern<<<dim3(c->n_lgrps * LTG, parts), LTT, LTL * ((c->max_cats + 2) | 1u) * sizeof(float), st>>>(
           ws->flows, ws->ld, B, c->aggr, c->in_node, c->in_cats, c->in_foff, c->lgrp_var, c->lgrp_off, c->lchunk_inputs,
           c->max_cats, ws->leaf_order, c->V, ws->row_ids, ws->row_start, weights_dev);
     } else if (c->max_cats <= LSC && want_sorted) {

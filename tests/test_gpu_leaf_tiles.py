@@ -28,3 +28,9 @@ def test_against_oracle(oracle, k, c, rows, missing, weighted):
     heap = m.heap()
     flow = np.concatenate([np.arange(h - 1 + c, h + 2 * c) for h in fc.node_heap_start[fc.input_node_ids.astype(np.int64) - 1].astype(np.int64)])
     assert rel_err(heap[flow], 2.0 * ref.heap[flow]) <= TOL
+
+
+@pytest.mark.parametrize("k,c,rows", [(5, 2, 20000), (16, 3, 37000), (33, 100, 30111)])
+def test_few_leaves_and_many_examples(oracle, k, c, rows):
+    """The slices of a batch dealt out over blocks: as many as blocks, one more, several per block."""
+    test_against_oracle(oracle, k, c, rows, 0.1, True)
