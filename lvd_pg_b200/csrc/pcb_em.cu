@@ -391,36 +391,39 @@ __global__ void __launch_bounds__(LTT) leaf_sort_kernel(
     const uint8_t* __restrict__ miss, uint64_t num_rows, const int32_t* __restrict__ row_ids, uint32_t row_start) {
   __shared__ uint32_t cursor[LSC + 4];
   __shared__ uint16_t xs[LTS];
-  const uint32_t var = blockIdx.x, b0 = blockIdx.y * LTS, tid = threadIdx.x, lane = tid & 31;
-  const uint32_t nb = min(LTS, B - b0), miss_bin = max_cats + 1, nbins = max_cats + 2;
-  uint32_t* const out = order + ((size_t)blockIdx.y * V + var) * LTS;
-  for (uint32_t x = tid; x <= nbins; x += LTT) cursor[x] = 0;
-  stage_values(xs, b0, nb, var, data, miss, num_rows, row_ids, row_start);
-  __syncthreads();
-  const uint32_t x = tid >= nb ? LT_NOSEG : xs[tid] == 0xffff ? miss_bin : (uint32_t)xs[tid];
-  const bool in = x <= miss_bin;
-  if (in) atomicAdd(&cursor[x + 1], 1u);
-  __syncthreads();
-  if (tid < 32) {   // starts of the segments: exclusive sums of their sizes
-    uint32_t carry = 0;
-    for (uint32_t base = 0; base <= nbins; base += 32) {
-      const uint32_t idx = base + lane;
-      uint32_t v = idx <= nbins ? cursor[idx] : 0u;
+  const uint32_t var = blockIdx.x, tid = threadIdx.x, lane = tid & 31, miss_bin = max_cats + 1, nbins = max_cats + 2;
+  for (uint32_t slice = blockIdx.y; slice < (B + LTS - 1) / LTS; slice += gridDim.y) {   // one unless there are more than the grid holds
+    const uint32_t b0 = slice * LTS, nb = min(LTS, B - b0);
+    uint32_t* const out = order + ((size_t)slice * V + var) * LTS;
+    for (uint32_t x = tid; x <= nbins; x += LTT) cursor[x] = 0;
+    stage_values(xs, b0, nb, var, data, miss, num_rows, row_ids, row_start);
+    __syncthreads();
+    const uint32_t x = tid >= nb ? LT_NOSEG : xs[tid] == 0xffff ? miss_bin : (uint32_t)xs[tid];
+    const bool in = x <= miss_bin;
+    if (in) atomicAdd(&cursor[x + 1], 1u);
+    __syncthreads();
+    if (tid < 32) {   // starts of the segments: exclusive sums of their sizes
+      uint32_t carry = 0;
+      for (uint32_t base = 0; base <= nbins; base += 32) {
+        const uint32_t idx = base + lane;
+        uint32_t v = idx <= nbins ? cursor[idx] : 0u;
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, v, d);
-        if ((int)lane >= d) v += u;
+        for (int d = 1; d < 32; d <<= 1) {
+          const uint32_t u = __shfl_up_sync(0xffffffffu, v, d);
+          if ((int)lane >= d) v += u;
+        }
+        v += carry;
+        if (idx <= nbins) cursor[idx] = v;
+        carry = __shfl_sync(0xffffffffu, v, 31);
       }
-      v += carry;
-      if (idx <= nbins) cursor[idx] = v;
-      carry = __shfl_sync(0xffffffffu, v, 31);
     }
+    __syncthreads();
+    const uint32_t total = cursor[nbins];
+    __syncthreads();
+    if (in) out[atomicAdd(&cursor[x], 1u)] = tid | (x << 16);
+    if (tid >= total) out[tid] = LT_NOSEG << 16;
+    __syncthreads();
   }
-  __syncthreads();
-  const uint32_t total = cursor[nbins];
-  __syncthreads();
-  if (in) out[atomicAdd(&cursor[x], 1u)] = tid | (x << 16);
-  if (tid >= total) out[tid] = LT_NOSEG << 16;
 }
 
 template <bool WEIGHTED>
@@ -643,7 +646,7 @@ __global__ void __launch_bounds__(SFT) leaf_forward_soft_kernel(
   __shared__ __align__(16) float x[SOFT_MAX_CATS * SFP], p[PCB_LEAF_GROUP * SOFT_MAX_CATS];
   __shared__ float ms[SFE];
   __shared__ uint32_t s_cats[PCB_LEAF_GROUP], top;
-  const uint32_t l0 = lgrp_off[blockIdx.x], nl = lgrp_off[blockIdx.x + 1] - l0, b0 = blockIdx.y * SFE, nb = min(SFE, B - b0);
+  const uint32_t l0 = lgrp_off[blockIdx.x], nl = lgrp_off[blockIdx.x + 1] - l0;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) top = 0;
   __syncthreads();
@@ -656,31 +659,35 @@ __global__ void __launch_bounds__(SFT) leaf_forward_soft_kernel(
     const float* tab = theta + in_poff[linputs[l0 + l]];
     for (uint32_t c = lane; c < Cp; c += 32) p[l * Cp + c] = c < s_cats[l] ? expf(__ldg(tab + c)) : 0.0f;
   }
-  soft_stage(x, ms, b0, nb, top, Cp, lgrp_var[blockIdx.x], num_vars, soft, num_rows, row_ids, row_start);
-  __syncthreads();
-  for (uint32_t l = warp; l < nl; l += SFT / 32) {   // one example per lane
-    float acc = 0.0f;
-    const float4* pl = reinterpret_cast<const float4*>(p + l * Cp);   // Cp is a multiple of four
-    for (uint32_t c = 0; c < Cp; c += 4) {
-      const float4 w = pl[c / 4];
-      acc = fmaf(w.x, x[c * SFP + lane], acc);
-      acc = fmaf(w.y, x[(c + 1) * SFP + lane], acc);
-      acc = fmaf(w.z, x[(c + 2) * SFP + lane], acc);
-      acc = fmaf(w.w, x[(c + 3) * SFP + lane], acc);
+  for (uint32_t b0 = blockIdx.y * SFE; b0 < B; b0 += gridDim.y * SFE) {   // one tile unless there are more than the grid holds
+    const uint32_t nb = min(SFE, B - b0);
+    soft_stage(x, ms, b0, nb, top, Cp, lgrp_var[blockIdx.x], num_vars, soft, num_rows, row_ids, row_start);
+    __syncthreads();
+    for (uint32_t l = warp; l < nl; l += SFT / 32) {   // one example per lane
+      float acc = 0.0f;
+      const float4* pl = reinterpret_cast<const float4*>(p + l * Cp);   // Cp is a multiple of four
+      for (uint32_t c = 0; c < Cp; c += 4) {
+        const float4 w = pl[c / 4];
+        acc = fmaf(w.x, x[c * SFP + lane], acc);
+        acc = fmaf(w.y, x[(c + 1) * SFP + lane], acc);
+        acc = fmaf(w.z, x[(c + 2) * SFP + lane], acc);
+        acc = fmaf(w.w, x[(c + 3) * SFP + lane], acc);
+      }
+      if (lane >= nb) continue;
+      const uint32_t i = linputs[l0 + l];
+      float v = ms[lane] + logf(acc);
+      if (!soft_in_range(acc)) {
+        const float* tab = theta + in_poff[i];
+        const float* sp = soft + (size_t)data_row(row_ids, row_start, b0 + lane) + (size_t)num_rows * lgrp_var[blockIdx.x];
+        const size_t cs = (size_t)num_rows * num_vars;
+        float mx = -INFINITY, sum = 0.0f;
+        for (uint32_t c = 0; c < s_cats[l]; ++c) mx = fmaxf(mx, sp[c * cs] + __ldg(tab + c));
+        for (uint32_t c = 0; c < s_cats[l]; ++c) sum += expf(sp[c * cs] + __ldg(tab + c) - mx);
+        v = mx == -INFINITY ? -INFINITY : mx + logf(sum);
+      }
+      mars[(size_t)in_node[i] * ld + b0 + lane] = v;
     }
-    if (lane >= nb) continue;
-    const uint32_t i = linputs[l0 + l];
-    float v = ms[lane] + logf(acc);
-    if (!soft_in_range(acc)) {
-      const float* tab = theta + in_poff[i];
-      const float* sp = soft + (size_t)data_row(row_ids, row_start, b0 + lane) + (size_t)num_rows * lgrp_var[blockIdx.x];
-      const size_t cs = (size_t)num_rows * num_vars;
-      float mx = -INFINITY, sum = 0.0f;
-      for (uint32_t c = 0; c < s_cats[l]; ++c) mx = fmaxf(mx, sp[c * cs] + __ldg(tab + c));
-      for (uint32_t c = 0; c < s_cats[l]; ++c) sum += expf(sp[c * cs] + __ldg(tab + c) - mx);
-      v = mx == -INFINITY ? -INFINITY : mx + logf(sum);
-    }
-    mars[(size_t)in_node[i] * ld + b0 + lane] = v;
+    if (b0 + gridDim.y * SFE < B) __syncthreads();
   }
 }
 
@@ -1012,7 +1019,7 @@ static int32_t forward_impl(pcb_circuit* c, pcb_workspace* ws, const pcb_evidenc
   if (c->n_inputs) {
     PcbProfScope ps(c, st, PCB_K_LEAF_FWD);
     if (ws->soft && c->max_cats <= SOFT_MAX_CATS) {
-      leaf_forward_soft_kernel<<<dim3(c->n_lgrps, (B + SFE - 1) / SFE), SFT, 0, st>>>(
+      leaf_forward_soft_kernel<<<dim3(c->n_lgrps, std::min(65535u, (B + SFE - 1) / SFE)), SFT, 0, st>>>(
           ws->mars, ws->ld, B, c->theta, c->in_node, c->in_cats, c->in_poff, c->lgrp_var, c->lgrp_off, c->lchunk_inputs,
           pcb_round_up(c->max_cats, 4), c->V, ws->soft, ev.num_rows, ev.row_ids_dev, ev.row_start);
     } else if (ws->soft || ws->soft_reg > 0.0f) {
@@ -1168,7 +1175,7 @@ static int32_t backward_impl(pcb_circuit* c, pcb_workspace* ws, const float* wei
       PCB_CUDA(cudaStreamWaitEvent(c->side2, c->ev_fork2, 0));
     }
     { PcbProfScope ps(c, ss, PCB_K_LEAF_FLOW);
-      leaf_sort_kernel<<<dim3(c->V, (B + LTS - 1) / LTS), LTT, 0, ss>>>(
+      leaf_sort_kernel<<<dim3(c->V, std::min(65535u, (B + LTS - 1) / LTS)), LTT, 0, ss>>>(
           ws->leaf_order, c->V, B, c->max_cats, ws->data, ws->miss, ws->num_rows, ws->row_ids, ws->row_start); }
     if (sorted_beside) PCB_CUDA(cudaEventRecord(c->ev_sort, c->side2));
   }

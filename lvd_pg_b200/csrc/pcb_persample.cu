@@ -233,41 +233,45 @@ __global__ void __launch_bounds__(32 * SPLIT_W) norm_split_kernel(
     const uint32_t* __restrict__ e_sub, const int32_t* __restrict__ row_ids, uint32_t row_start, float* __restrict__ out,
     uint64_t out_rows) {
   __shared__ float part[SPLIT_W][32];
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, b = blockIdx.y * 32 + lane;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t n = grp_node[blockIdx.x];
   const uint4 sn = s_node[n];
-  const bool on = b < B;
-  const int64_t row = on ? data_row(row_ids, row_start, b) : 0;
-  const float pf = on ? flows[(size_t)n * ld + b] : 0.0f, pm = on ? mars[(size_t)n * ld + b] : 0.0f;
-  auto edge_flow = [&](uint32_t j) {
-    if (!on) return 0.0f;
-    const uint32_t sb = e_sub[sn.x + j];
-    float child = mars[(size_t)e_prime[sn.x + j] * ld + b] + p.at(row, (uint64_t)sn.z + j);
-    if (sb != PCB_NONE) child += mars[(size_t)sb * ld + b];
-    return pf == 0.0f ? 0.0f : pf * __expf(child - pm);
-  };
-  float ef[SPLIT_REG], total = 0.0f;
+  for (uint32_t b0 = blockIdx.y * 32; b0 < B; b0 += gridDim.y * 32) {   // one tile unless there are more than the grid holds
+    const uint32_t b = b0 + lane;
+    const bool on = b < B;
+    const int64_t row = on ? data_row(row_ids, row_start, b) : 0;
+    const float pf = on ? flows[(size_t)n * ld + b] : 0.0f, pm = on ? mars[(size_t)n * ld + b] : 0.0f;
+    auto edge_flow = [&](uint32_t j) {
+      if (!on) return 0.0f;
+      const uint32_t sb = e_sub[sn.x + j];
+      float child = mars[(size_t)e_prime[sn.x + j] * ld + b] + p.at(row, (uint64_t)sn.z + j);
+      if (sb != PCB_NONE) child += mars[(size_t)sb * ld + b];
+      return pf == 0.0f ? 0.0f : pf * __expf(child - pm);
+    };
+    float ef[SPLIT_REG], total = 0.0f;
 #pragma unroll
-  for (uint32_t k = 0; k < SPLIT_REG; ++k) {
-    const uint32_t j = warp + k * SPLIT_W;
-    ef[k] = j < sn.y ? edge_flow(j) : 0.0f;
-    total += ef[k];
-  }
-  for (uint32_t j = warp + SPLIT_REG * SPLIT_W; j < sn.y; j += SPLIT_W) total += edge_flow(j);
-  part[warp][lane] = total;
-  __syncthreads();
-  total = 1e-8f;
-  for (uint32_t k = 0; k < SPLIT_W; ++k) total += part[k][lane];
-  if (!on) return;
-  const float inv = 1.0f / total;
-  float* const o = out + (size_t)row + (size_t)out_rows * sn.z;
+    for (uint32_t k = 0; k < SPLIT_REG; ++k) {
+      const uint32_t j = warp + k * SPLIT_W;
+      ef[k] = j < sn.y ? edge_flow(j) : 0.0f;
+      total += ef[k];
+    }
+    for (uint32_t j = warp + SPLIT_REG * SPLIT_W; j < sn.y; j += SPLIT_W) total += edge_flow(j);
+    part[warp][lane] = total;
+    __syncthreads();
+    total = 1e-8f;
+    for (uint32_t k = 0; k < SPLIT_W; ++k) total += part[k][lane];
+    __syncthreads();   // the parts have been read
+    if (!on) continue;
+    const float inv = 1.0f / total;
+    float* const o = out + (size_t)row + (size_t)out_rows * sn.z;
 #pragma unroll
-  for (uint32_t k = 0; k < SPLIT_REG; ++k) {
-    const uint32_t j = warp + k * SPLIT_W;
-    if (j < sn.y) o[(size_t)out_rows * j] = __logf(ef[k] * inv + 1e-8f);
+    for (uint32_t k = 0; k < SPLIT_REG; ++k) {
+      const uint32_t j = warp + k * SPLIT_W;
+      if (j < sn.y) o[(size_t)out_rows * j] = __logf(ef[k] * inv + 1e-8f);
+    }
+    for (uint32_t j = warp + SPLIT_REG * SPLIT_W; j < sn.y; j += SPLIT_W)
+      o[(size_t)out_rows * j] = __logf(edge_flow(j) * inv + 1e-8f);
   }
-  for (uint32_t j = warp + SPLIT_REG * SPLIT_W; j < sn.y; j += SPLIT_W)
-    o[(size_t)out_rows * j] = __logf(edge_flow(j) * inv + 1e-8f);
 }
 
 // The dense blocks with the circuit's own parameters.  An edge's flow is pf * w * x / sum(w * x) with x = exp(child -
@@ -532,7 +536,7 @@ extern "C" int32_t pcb_normalized_flows(pcb_circuit* c, pcb_workspace* ws, const
   }
   if (n_groups && n_groups <= 64) {
     ++c->prof.launches[PCB_K_MISC];
-    norm_split_kernel<<<dim3(n_groups, (B + 31) / 32), 32 * SPLIT_W, 0, st>>>(
+    norm_split_kernel<<<dim3(n_groups, std::min(65535u, (B + 31) / 32)), 32 * SPLIT_W, 0, st>>>(
         ws->flows, ws->mars, ws->ld, B, p, groups, c->s_node, c->e_prime, c->e_sub, ev->row_ids_dev, ev->row_start, out_dev,
         ev->num_rows);
   } else if (n_groups && quads) {
