@@ -347,10 +347,36 @@ __global__ void __launch_bounds__(256) kld_up_warp_kernel(KldLayer a) {
   if (i >= a.count) return;
   const uint32_t n = a.nodes[i], e0 = a.n_estart[n], cnt = a.n_ecount[n], pid0 = a.n_pid0[n];
   const bool issum = a.kind[n] == PCB_SUM;
+  uint32_t pr[KLD_PRE], sb[KLD_PRE];
+  float wgt[KLD_PRE], dif[KLD_PRE];
+#pragma unroll
+  for (int r = 0; r < KLD_PRE; ++r) {
+    const uint32_t j = lane + 32 * r;
+    pr[r] = sb[r] = PCB_NONE; wgt[r] = 1.0f; dif[r] = 0.0f;
+    if (j < cnt) {
+      pr[r] = a.e_prime[e0 + j]; sb[r] = a.e_sub[e0 + j];
+      if (issum) {
+        const float x = a.p1[s + (size_t)S * (pid0 + j)], y = a.p2[s + (size_t)S * (pid0 + j)];
+        wgt[r] = expf(x);
+        dif[r] = x - y;
+      }
+    }
+    keep(pr[r]); keep(sb[r]); keep(wgt[r]); keep(dif[r]);
+  }
   pcb_grid_dep_wait();
-  float acc = 0.0f;
-#pragma unroll 2
-  for (uint32_t j = lane; j < cnt; j += 32) {
+  float k0[KLD_PRE], k1[KLD_PRE], acc = 0.0f;   // an edge without a second child reads the first one again
+#pragma unroll
+  for (int r = 0; r < KLD_PRE; ++r) {
+    const uint32_t first = pr[r] != PCB_NONE ? pr[r] : n;
+    k0[r] = klds[(size_t)first * ld];
+    k1[r] = klds[(size_t)(sb[r] != PCB_NONE ? sb[r] : first) * ld];
+  }
+#pragma unroll
+  for (int r = 0; r < KLD_PRE; ++r) {
+    const float k = k0[r] + (sb[r] != PCB_NONE ? k1[r] : 0.0f);
+    if (pr[r] != PCB_NONE) acc += issum ? wgt[r] * (k + dif[r]) : k;
+  }
+  for (uint32_t j = lane + 32 * KLD_PRE; j < cnt; j += 32) {
     float k = klds[(size_t)a.e_prime[e0 + j] * ld];
     const uint32_t sb = a.e_sub[e0 + j];
     if (sb != PCB_NONE) k += klds[(size_t)sb * ld];
@@ -936,9 +962,26 @@ __global__ void __launch_bounds__(256) kld1_push_kernel(KldLayer a) {
   if (i >= a.count) return;
   const uint32_t n = a.nodes[i], e0 = a.n_estart[n], cnt = a.n_ecount[n], pid0 = a.n_pid0[n];
   const bool issum = a.kind[n] == PCB_SUM;
+  uint32_t pr[KLD_PRE], sb[KLD_PRE];
+  float wgt[KLD_PRE];
+#pragma unroll
+  for (int r = 0; r < KLD_PRE; ++r) {
+    const uint32_t j = lane + 32 * r;
+    pr[r] = sb[r] = PCB_NONE; wgt[r] = 0.0f;
+    if (j < cnt) {
+      pr[r] = a.e_prime[e0 + j]; sb[r] = a.e_sub[e0 + j];
+      wgt[r] = issum ? expf(a.p1[pid0 + j]) : 1.0f;
+    }
+    keep(pr[r]); keep(sb[r]); keep(wgt[r]);
+  }
   pcb_grid_dep_wait();
   const float pg = grads[(size_t)n * ld];
-  for (uint32_t j = lane; j < cnt; j += 32) {
+#pragma unroll
+  for (int r = 0; r < KLD_PRE; ++r) {
+    if (pr[r] != PCB_NONE) atomicAdd(grads + (size_t)pr[r] * ld, pg * wgt[r]);
+    if (sb[r] != PCB_NONE) atomicAdd(grads + (size_t)sb[r] * ld, pg * wgt[r]);
+  }
+  for (uint32_t j = lane + 32 * KLD_PRE; j < cnt; j += 32) {
     const float eg = issum ? pg * expf(a.p1[pid0 + j]) : pg;
     atomicAdd(grads + (size_t)a.e_prime[e0 + j] * ld, eg);
     if (a.e_sub[e0 + j] != PCB_NONE) atomicAdd(grads + (size_t)a.e_sub[e0 + j] * ld, eg);
