@@ -689,9 +689,16 @@ __global__ void renorm_kernel(float* __restrict__ theta, uint32_t n_groups, cons
   for (uint32_t j = lane; j < cnt; j += 32) theta[off + j] -= ls;
 }
 
-// Up to this many sets the warp-per-(node, set) kernels are the faster chain (784 variables x 64 latents, both passes
-// with the caller's copies: two sets 240 against 264 us, four sets 397 against 228 us).
-constexpr uint32_t KLD_WARP_SETS = 2;
+// Which chain a call of a few sets takes: a warp per (node, set), or the tiles of the layer kernels.  One and two sets go
+// by warps, as the fused step's upward pass does.  Up to eight go by warps where that is the shorter chain: in circuits
+// without dense blocks (a thread of a layer kernel walks such a node's edges alone) and in small ones (both passes on the
+// device, warps against tiles: 100 variables x 8 latents, four sets 37 against 98 us, eight 37 against 109; 100 x 32, four
+// sets 47 against 55, eight 56 against 58; 300 x 32, three sets 70 against 78, four 74 against 76, six 96 against 82;
+// 784 x 16, three sets 67 against 68, four 76 against 66; 784 x 64, three sets 285 against 109).
+constexpr uint32_t KLD_WARP_SETS = 2, KLD_WARP_SETS_SMALL = 8;
+bool kld_by_warps(const pcb_circuit* c, uint32_t S) {
+  return S <= KLD_WARP_SETS || (S <= KLD_WARP_SETS_SMALL && (c->n_dense == 0 || (uint64_t)S * c->n_inner <= 500000));
+}
 
 // what the kernels of step t need; the caller adds the loose nodes and the shares of a CTA
 KldLayer kld_layer(pcb_circuit* c, pcb_workspace* ws, const float* p1, const float* p2, uint32_t S, uint32_t t) {
@@ -777,7 +784,7 @@ extern "C" int32_t pcb_kld(pcb_circuit* c, pcb_workspace* ws, const float* param
     uint32_t R = 1, K = 1;
     pcb_step_extent(c, t, R, K);
     for (uint32_t i = c->h_st_thin_off[t]; i < c->h_st_thin_off[t + 1]; ++i) K = std::max(K, c->h_thin[i].K);
-    if (S <= KLD_WARP_SETS) {
+    if (kld_by_warps(c, S)) {
       PCB_CUDA(kld_launch_warps(c, kld_up_warp_kernel, a, blocks, R, st));
       continue;
     }
@@ -807,7 +814,7 @@ extern "C" int32_t pcb_kld_backward(pcb_circuit* c, pcb_workspace* ws, const flo
   cudaStream_t st = (cudaStream_t)s;
   const uint32_t ld = ws->ldS;
   bool chained = false;   // the first launch of the pass waits for whatever the caller's stream holds before it
-  if (S <= KLD_WARP_SETS) {
+  if (kld_by_warps(c, S)) {
     for (int64_t lay = c->L; lay >= 0; --lay) {
       const uint32_t o0 = c->h_down_all_off[lay], o1 = c->h_down_all_off[lay + 1];
       if (o1 == o0) continue;

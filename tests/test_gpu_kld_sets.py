@@ -8,8 +8,9 @@ from tests.test_gpu_kld_sample import TOL, _cuda, _param_sets
 pytestmark = pytest.mark.gpu
 
 # (variables, latents, categories, sets): sets that do not divide the block, one set more than a tile, a child list
-# longer than the staged values (272 x 32 > 2048) with more steps per thread than are parked, single-child chains
-SHAPES = [(9, 17, 3, 3), (12, 64, 2, 24), (6, 272, 2, 33), (7, 72, 5, 32), (5, 130, 2, 5), (6, 16, 2, 65)]
+# longer than the staged values (272 x 32 > 2048) with more steps per thread than are parked, single-child chains, few
+# sets on either side of the line between warps and tiles, no dense blocks
+SHAPES = [(9, 17, 3, 3), (20, 130, 2, 3), (20, 130, 2, 5), (40, 70, 2, 4), (30, 64, 2, 8), (9, 8, 3, 8), (9, 8, 3, 9), (12, 64, 2, 24), (6, 272, 2, 33), (7, 72, 5, 32), (5, 130, 2, 5), (6, 16, 2, 65)]
 
 
 @pytest.mark.parametrize("v,k,c,S", SHAPES)
