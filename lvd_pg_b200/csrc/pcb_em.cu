@@ -241,6 +241,7 @@ __global__ void __launch_bounds__(LST) leaf_flow_sorted_kernel(
   const uint32_t l0 = lgrp_off[grp], nl = lgrp_off[grp + 1] - l0;
   // segments: values 0 .. max_cats (a value equal to a leaf's category count lands in that leaf's
   // extra slot, larger ones are dropped, as in the atomic kernel), then the missing-value segment
+  constexpr uint32_t NOSEG = 0xffffffffu;
   const uint32_t miss_bin = max_cats + 1, nbins = max_cats + 2;
   if (tid == 0) {
     for (int r = 0; r < LSR; ++r) pcbtc::mbar_init(&bar[r], 1);
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(LST) leaf_flow_sorted_kernel(
   if (tid == 0) for (uint32_t l = 0; l < min(nl, (uint32_t)LSR - 1u); ++l) request(l);
   // counting sort of the examples by value
   for (uint32_t b = tid; b < nb; b += LST) {
-    const uint32_t x = xs[b] == 0xffff ? miss_bin : (uint32_t)xs[b];
+    const uint32_t x = xs[b] == 0xffff ? miss_bin : xs[b] <= max_cats ? (uint32_t)xs[b] : NOSEG;
     if (x <= miss_bin) atomicAdd(&binoff[x + 1], 1u);
   }
   __syncthreads();
@@ -287,12 +288,11 @@ __global__ void __launch_bounds__(LST) leaf_flow_sorted_kernel(
   for (uint32_t x = tid; x < nbins; x += LST) cursor[x] = binoff[x];
   __syncthreads();
   for (uint32_t b = tid; b < nb; b += LST) {
-    const uint32_t x = xs[b] == 0xffff ? miss_bin : (uint32_t)xs[b];
+    const uint32_t x = xs[b] == 0xffff ? miss_bin : xs[b] <= max_cats ? (uint32_t)xs[b] : NOSEG;
     if (x <= miss_bin) perm[atomicAdd(&cursor[x], 1u)] = (uint16_t)b;
   }
   __syncthreads();
   // this thread's sorted positions LSE * tid .. + LSE - 1: example, segment, weight
-  constexpr uint32_t NOSEG = 0xffffffffu;
   uint32_t pos[LSE], seg[LSE];
   float wv[LSE];
   {
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(LTT) leaf_sort_kernel(
     for (uint32_t x = tid; x <= nbins; x += LTT) cursor[x] = 0;
     stage_values(xs, b0, nb, var, data, miss, num_rows, row_ids, row_start);
     __syncthreads();
-    const uint32_t x = tid >= nb ? LT_NOSEG : xs[tid] == 0xffff ? miss_bin : (uint32_t)xs[tid];
+    const uint32_t x = tid >= nb ? LT_NOSEG : xs[tid] == 0xffff ? miss_bin : xs[tid] <= max_cats ? (uint32_t)xs[tid] : LT_NOSEG;
     const bool in = x <= miss_bin;
     if (in) atomicAdd(&cursor[x + 1], 1u);
     __syncthreads();

@@ -34,3 +34,23 @@ def test_against_oracle(oracle, k, c, rows, missing, weighted):
 def test_few_leaves_and_many_examples(oracle, k, c, rows):
     """The slices of a batch dealt out over blocks: as many as blocks, one more, several per block."""
     test_against_oracle(oracle, k, c, rows, 0.1, True)
+
+
+@pytest.mark.parametrize("impl", ["", "sorted", "atomic"])
+def test_values_that_no_leaf_has(monkeypatch, impl):
+    """A value one past the extra slot is no missing value: it is dropped, as every larger one."""
+    monkeypatch.setenv("PCB_LEAF_FLOW_IMPL", impl)
+    torch, api = _cuda()
+    fc = random_hclt(5, 17, 3, 3)
+    data, _ = random_data(300, 5, 3, 11)
+    var = int(fc.node_var[fc.input_node_ids[0] - 1]) - 1     # its leaves are not the last: their tables are followed by others
+    data[::7, var] = 4
+    m = api.CuMetaBitsProbCircuit(fc)
+    ws, B = api.forward(m, api.DeviceData(data, m.device))
+    m.lib.pcb_clear_flows(m.handle, 0.0, None)
+    api.backward(m, ws)
+    flows, heap = m.flows(ws, B), m.heap()
+    for n in np.nonzero((fc.node_kind == 0) & (fc.node_var == var + 1))[0]:
+        h = int(fc.node_heap_start[n]) - 1 + 3
+        want = [flows[data[:, var] == x, n].sum() for x in range(3)] + [0.0]
+        np.testing.assert_allclose(heap[h:h + 4], want, rtol=1e-4, atol=1e-6)
