@@ -450,7 +450,9 @@ __device__ __forceinline__ float soft_exp(double z, const SoftTables* t) {
   return (float)__hiloint2double(__double2hiint(p) + ((n >> 5) << 20), __double2loint(p));
 }
 
-// the tables serve u in [0, 1) and |z| < 600; `ok` is cleared for anything else
+// the tables serve u in [0, 1), |z| < 600 and temperatures down to 1/256 (their noise is off by up to 1.5e-10, which the
+// temperature divides: past that it would exceed the fp32 rounding of the weight); `ok` is cleared for anything else
+constexpr double SOFT_TABLE_INV_T = 256.0;
 template <bool NOISE>
 __device__ __forceinline__ float soft_weight_fast(float logp, float u, double inv_t, const SoftTables* t, bool& ok) {
   double g = 0.0;
@@ -459,7 +461,7 @@ __device__ __forceinline__ float soft_weight_fast(float logp, float u, double in
     ok = ok && __float_as_uint(u) < 0x3f800000u;
   }
   const double z = ((double)logp + g) * inv_t;
-  ok = ok && fabs(z) < 600.0;
+  ok = ok && fabs(z) < 600.0 && inv_t <= SOFT_TABLE_INV_T;
   return soft_exp(z, t);
 }
 template <bool NOISE>

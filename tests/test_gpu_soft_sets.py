@@ -57,3 +57,28 @@ def test_relaxed_samples_of_row_major_sets(oracle, v, k, c, S):
     wide = torch.from_numpy(np.concatenate([u, u[:, :3]], 1)).cuda()
     for pp, uu in ((torch.from_numpy(p).cuda(), torch.from_numpy(u).cuda()), (p, u), (torch.from_numpy(p).cuda(), wide)):
         assert rel_err(api.gumbel_sample(m, pp, v, c, 0.7, u=uu).cpu().numpy(), ref) <= TOL
+
+
+@pytest.mark.parametrize("temperature", [0.7, 1.0 / 300, 1e-4])
+@pytest.mark.parametrize("rows", [True, False])
+def test_relaxed_weights_at_low_temperatures(temperature, rows):
+    """Edges whose log-weight and noise nearly cancel, so that the temperature divides small sums: against 64 bits.  The
+    inputs are exact, the weights and their sums are rounded a few times."""
+    torch, api = _cuda()
+    v, k, S = 2, 64, 8
+    fc = random_hclt(v, k, k, 1)      # one sum node; leaf i always takes category i
+    m = api.CuMetaBitsProbCircuit(fc)
+    u = np.random.default_rng(1).uniform(0.01, 0.99, (S, k)).astype(np.float32)
+    gumbel = lambda: -np.log(-np.log(u.astype(np.float64) * (1.0 - 1e-6) + 1e-6))
+    p = np.full((S, fc.num_parameters), -np.inf, np.float32)
+    p[:, :k] = (np.random.default_rng(2).uniform(-3, 3, (S, k)) * temperature - gumbel()).astype(np.float32)
+    leaves = p[:, k:].reshape(S, v, k, k)
+    leaves[:, :, np.arange(k), np.arange(k)] = 0.0
+    z = (p[:, :k].astype(np.float64) + gumbel()) / temperature
+    want = np.exp(z - z.max(1, keepdims=True))
+    want /= want.sum(1, keepdims=True)
+    dp, du = torch.from_numpy(p).cuda(), torch.from_numpy(u).cuda()
+    if not rows:
+        dp, du = dp.t().contiguous().t(), du.t().contiguous().t()
+    got = api.gumbel_sample(m, dp, v, k, temperature, u=du).cpu().numpy()
+    assert np.abs(got - want[:, None, :]).max() <= 5e-7 * want.max()
