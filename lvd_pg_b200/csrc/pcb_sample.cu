@@ -52,18 +52,14 @@ __device__ __forceinline__ void warp_argmax(double& key, uint32_t& idx) {
 // Bound: x = u (1 - 1e-6) + 1e-6 carries a relative error <= 2.4e-7, __logf an absolute error <= 3.6e-7 on [0.5, 2] and
 // three ulp elsewhere, so inner = -log x is off by 6e-7 / inner + 4e-7; __expf by 2.4e-7 + 1.2e-7 |logp|, the product by
 // 6e-8; eps is four times the sum.  Entries with inner below 1e-4 or exp(-logp) below 1e-30 have no bounds and always
-// stay candidates (lower bound 0, upper bound infinity).  A race time past 1e37 has no upper bound, and its lower bound
-// is what is known of it: only an entry of weight 0 is later than every other.
+// stay candidates (lower bound 0, upper bound infinity).  Where exp(-logp) or the product leaves the fp32 range the upper
+// bound is infinity and the lower one that of 3e38.
 __device__ __forceinline__ void race(float lp, float u, float& lo, float& hi) {
-  const float inner = -__logf(fmaf(u, 0.999999f, 1e-6f)), inv = __expf(-lp), r = inner * inv;
-  const float eps = __fdividef(2.4e-6f, inner) + 3.2e-6f + 5e-7f * fabsf(lp);
+  const float inner = -__logf(fmaf(u, 0.999999f, 1e-6f)), inv = __expf(-lp), r = inner * fminf(inv, 3e38f), least = fminf(r, 3e38f);
+  const float eps = __fdividef(2.4e-6f, inner) + 3.2e-6f + 5e-7f * fminf(fabsf(lp), 100.0f);
   const bool none = inner < 1e-4f || inv < 1e-30f;
-  lo = none ? 0.0f : r - r * eps;
-  hi = none ? INFINITY : r + r * eps;
-  if (r >= 1e37f && !none) {
-    hi = INFINITY;
-    lo = lp == -INFINITY ? INFINITY : inv == INFINITY ? fminf(inner, 1.0f) * 3e38f : 9e36f;   // eps is below 3%
-  }
+  lo = none ? 0.0f : least - least * eps;
+  hi = none || !(inv < 3e38f) ? INFINITY : r + r * eps;
 }
 
 __device__ __noinline__ uint32_t warp_exact64(float lp0, float u0, bool c0, float lp1, float u1, bool c1, uint32_t lane) {
