@@ -446,9 +446,9 @@ __device__ __forceinline__ float soft_exp(double z, const SoftTables* t) {
   return (float)__hiloint2double(__double2hiint(p) + ((n >> 5) << 20), __double2loint(p));
 }
 
-// the tables serve u in [0, 1), |z| < 600 and temperatures down to 1/256 (their noise is off by up to 1.5e-10, which the
-// temperature divides: past that it would exceed the fp32 rounding of the weight); `ok` is cleared for anything else
-constexpr double SOFT_TABLE_INV_T = 256.0;
+// the tables serve u in [0, 1), |z| < 600 and temperatures down to 1/512 (their noise is off by up to 3.6e-11, which the
+// temperature divides: 1.9e-8 there, a third of the fp32 rounding of the weight); `ok` is cleared for anything else
+constexpr double SOFT_TABLE_INV_T = 512.0;
 template <bool NOISE>
 __device__ __forceinline__ float soft_weight_fast(float logp, float u, double inv_t, const SoftTables* t, bool& ok) {
   double g = 0.0;

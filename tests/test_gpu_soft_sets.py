@@ -59,7 +59,7 @@ def test_relaxed_samples_of_row_major_sets(oracle, v, k, c, S):
         assert rel_err(api.gumbel_sample(m, pp, v, c, 0.7, u=uu).cpu().numpy(), ref) <= TOL
 
 
-@pytest.mark.parametrize("temperature", [0.7, 1.0 / 300, 1e-4])
+@pytest.mark.parametrize("temperature", [0.7, 1.0 / 300, 1e-6])
 @pytest.mark.parametrize("rows", [True, False])
 def test_relaxed_weights_at_low_temperatures(temperature, rows):
     """Edges whose log-weight and noise nearly cancel, so that the temperature divides small sums: against 64 bits.  The
