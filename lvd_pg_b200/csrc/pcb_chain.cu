@@ -153,6 +153,7 @@ __device__ __forceinline__ float4 over_rows(float4 v, float4 (&red)[TPB / 32][8]
 
 // A single sum node over consecutive children (the root, so the likelihood itself): in fp32 and with the weights inside
 // the maximum, as the kernel of single nodes sums it, so that children far below one without weight count in full.
+template <uint32_t BATCH>
 __device__ __forceinline__ void up_single(const ChainArgs& a, const PcbDenseBlock& k, float* w, float4 (&red)[TPB / 32][8]) {
   const uint32_t q = threadIdx.x & 7, g = threadIdx.x >> 3, ld = a.ld, K = k.K;
   float* const x = w + ((K + 3u) & ~3u);   // [K][XP]
@@ -164,7 +165,7 @@ __device__ __forceinline__ void up_single(const ChainArgs& a, const PcbDenseBloc
     const float* const pa = a.mars + (size_t)k.c0 * ld + b;
     const float* const pb = a.mars + (size_t)(k.d0 != PCB_NONE ? k.d0 : k.c0) * ld + b;
     float4 mx = splat(-INFINITY);
-#pragma unroll 2
+#pragma unroll BATCH
     for (uint32_t t = g; t < K; t += RSTEP) {
       float4 v = ld4(pa + (size_t)t * ld);
       if (k.d0 != PCB_NONE) v = add4(v, ld4(pb + (size_t)t * ld));
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(TPB, BATCH <= 2 ? 4 : 2) chain_up_kernel(Chain
   const PcbDenseBlock k = bi < a.nblk ? a.blk[bi] : a.thin[bi - a.nblk];
   if (r0 >= k.R) return;
   if (bi >= a.nblk) {
-    up_single(a, k, reinterpret_cast<float*>(chain_smem), red);
+    up_single<BATCH>(a, k, reinterpret_cast<float*>(chain_smem), red);
     return;
   }
   const uint32_t rows = min(OUT, k.R - r0), K = k.K, K8 = (K + 7u) & ~7u, wp = K8 + 4u, ld = a.ld;
