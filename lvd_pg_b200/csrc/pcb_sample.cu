@@ -449,15 +449,16 @@ __device__ __forceinline__ float soft_exp(double z, const SoftTables* t) {
 // the tables serve u in [0, 1), |z| < 600 and temperatures down to 1/512 (their noise is off by up to 3.6e-11, which the
 // temperature divides: 1.9e-8 there, a third of the fp32 rounding of the weight); `ok` is cleared for anything else
 constexpr double SOFT_TABLE_INV_T = 512.0;
+__device__ __forceinline__ double soft_z_max(double inv_t) { return inv_t <= SOFT_TABLE_INV_T ? 600.0 : 0.0; }
 template <bool NOISE>
-__device__ __forceinline__ float soft_weight_fast(float logp, float u, double inv_t, const SoftTables* t, bool& ok) {
+__device__ __forceinline__ float soft_weight_fast(float logp, float u, double inv_t, double z_max, const SoftTables* t, bool& ok) {
   double g = 0.0;
   if (NOISE) {
     g = -soft_log(-soft_log(fma((double)u, 1.0 - 1e-6, 1e-6), t), t);
     ok = ok && __float_as_uint(u) < 0x3f800000u;
   }
   const double z = ((double)logp + g) * inv_t;
-  ok = ok && fabs(z) < 600.0 && inv_t <= SOFT_TABLE_INV_T;
+  ok = ok && fabs(z) < z_max;
   return soft_exp(z, t);
 }
 template <bool NOISE>
@@ -467,9 +468,9 @@ __device__ __noinline__ float soft_weight_any(float logp, float u, double inv_t)
   return (float)exp(((double)logp + g) * inv_t);
 }
 template <bool NOISE>
-__device__ __forceinline__ float soft_weight(float logp, float u, double inv_t, const SoftTables* t) {
+__device__ __forceinline__ float soft_weight(float logp, float u, double inv_t, double z_max, const SoftTables* t) {
   bool ok = true;
-  const float e = soft_weight_fast<NOISE>(logp, u, inv_t, t, ok);
+  const float e = soft_weight_fast<NOISE>(logp, u, inv_t, z_max, t, ok);
   return ok ? e : soft_weight_any<NOISE>(logp, u, inv_t);
 }
 
@@ -483,6 +484,7 @@ __global__ void __launch_bounds__(SOFT_THREADS, 4) soft_params_kernel(
   __shared__ SoftTables tab;
   __shared__ float red[SOFT_THREADS];
   soft_tables_fill(&tab);
+  const double z_max = soft_z_max(inv_t);
   const uint32_t s0 = blockIdx.y * St, sw = min(St, S - s0), J = SOFT_THREADS / St, JG = J / rows;
   const uint32_t q = threadIdx.x / St, s = threadIdx.x % St, r = q / JG, jg = q % JG;
   const bool lane_on = q < JG * rows && s < sw;
@@ -506,9 +508,9 @@ __global__ void __launch_bounds__(SOFT_THREADS, 4) soft_params_kernel(
     }
 #pragma unroll
     for (uint32_t k = 0; k < 8; ++k)
-      if (jg + k * JG < cnt) { x[k] = soft_weight<NOISE>(x[k], y[k], inv_t, &tab); sum += x[k]; }
+      if (jg + k * JG < cnt) { x[k] = soft_weight<NOISE>(x[k], y[k], inv_t, z_max, &tab); sum += x[k]; }
     for (uint32_t j = jg + 8 * JG; j < cnt; j += JG) {
-      const float e = soft_weight<NOISE>(pp[(size_t)Sp * j], NOISE ? pu[(size_t)S * j] : 0.5f, inv_t, &tab);
+      const float e = soft_weight<NOISE>(pp[(size_t)Sp * j], NOISE ? pu[(size_t)S * j] : 0.5f, inv_t, z_max, &tab);
       pw[(size_t)ld * j] = e;
       sum += e;
     }
@@ -541,6 +543,7 @@ __global__ void __launch_bounds__(SOFT_THREADS, 3) soft_params_rows_kernel(
   __shared__ double inv_tot[32];
   extern __shared__ float soft_tile[];   // [edges of the widest node][33]
   soft_tables_fill(&tab);
+  const double z_max = soft_z_max(inv_t);
   const uint32_t s0 = blockIdx.y * 32, sw = min(32u, S - s0), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float x[4][2], y[4][2], xn[4][2], yn[4][2];   // 64 edges of up to four sets a warp, and those of the next node
   const float* const mine = params + (s0 + warp) * ss + lane;   // this lane's edge of the warp's first set; further sets
@@ -577,10 +580,10 @@ __global__ void __launch_bounds__(SOFT_THREADS, 3) soft_params_rows_kernel(
         bool ok = true;
         float e[2];
 #pragma unroll
-        for (uint32_t h = 0; h < 2; ++h) e[h] = soft_weight_fast<NOISE>(x[k][h], y[k][h], inv_t, &tab, ok);
+        for (uint32_t h = 0; h < 2; ++h) e[h] = soft_weight_fast<NOISE>(x[k][h], y[k][h], inv_t, z_max, &tab, ok);
         if (!ok)
 #pragma unroll
-          for (uint32_t h = 0; h < 2; ++h) e[h] = soft_weight<NOISE>(x[k][h], y[k][h], inv_t, &tab);
+          for (uint32_t h = 0; h < 2; ++h) e[h] = soft_weight<NOISE>(x[k][h], y[k][h], inv_t, z_max, &tab);
 #pragma unroll
         for (uint32_t h = 0; h < 2; ++h)
           if (j0 + lane + 32 * h < cnt) {
