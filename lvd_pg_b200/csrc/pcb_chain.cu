@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(TPB, BATCH <= 2 ? 4 : 2) chain_down_kernel(Cha
 // G = flows[r] * exp(mx - mars[r]), X = exp(M[t] - mx).  pcb_dense_edge.cu works in tiles of 128 x 256 outputs, of which
 // a block of 32 latents fills a thirtieth; here a CTA owns 64 x 64 outputs of one block in registers (mma.sync, operands
 // as above) and walks its share of the examples in tiles of 32, the rows of the next tile in flight.  Bound: HBM (four
-// rows per latent and example).  2159 blocks of 32 x 32 at 512 examples: 576 -> 317 us (beside the chain).
+// rows per latent and example).  2159 blocks of 32 x 32 at 512 examples: 576 -> 317 us beside the chain, 233 us alone.
 constexpr uint32_t EP = EX + 4;   // pitch of both operand tiles: eight rows x four examples of a fragment in 32 banks
 __global__ void __launch_bounds__(TPB, 2) edge_narrow_kernel(
     const float* __restrict__ mars, const float* __restrict__ flows, const float* __restrict__ blk_mx,

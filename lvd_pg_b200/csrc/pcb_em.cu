@@ -613,7 +613,12 @@ __global__ void leaf_flow_gen_kernel(const float* __restrict__ flows, const floa
 // The sum of a leaf whose probable categories all have negligible weights can leave the fp32 range that way: such a
 // value (outside [1e-30, 1e30], or not a number) is computed as above, and so is its share of the statistics.
 // Bound: the gather of the weights (rows of a batch are scattered) until there are enough blocks for the FMA pipes.
-// 300 examples x 7200 leaves x 33 categories: forward 321 -> 47 us, statistics 184 -> 55 us.
+// 300 examples x 7200 leaves x 33 categories: forward 321 -> 50 us, statistics 184 -> 49 us.
+// SOFT_MAX_CATS is what the two tiles of the forward kernel take of its 48 KB of static shared memory (36 + 64 words per
+// category; 64 fill half of it, the next multiple of 64 would not fit) and the sums that a thread of the statistics
+// holds (16).  More categories stay with the general kernels: 512 leaves x 4096 examples, 64 categories 93 and 84 us, 65
+// categories 917 and 451 us.  CPT follows the categories because the products of the statistics do: 33 categories with ten
+// sums a thread 39 us, with sixteen 60 us; 8 with two 23 us, with sixteen 45 us; 16 with four 27 us, with sixteen 49 us.
 constexpr uint32_t SOFT_MAX_CATS = 64, SFT = 256, SFE = 32, SFP = SFE + 4;   // threads, examples of a tile, pitch of a row
 
 __device__ __forceinline__ bool soft_in_range(float sum) { return sum >= 1e-30f && sum <= 1e30f; }

@@ -19,9 +19,11 @@
 //   * one thread issues the MMAs into one of two 128 x 256 accumulators (all 512 columns of tensor memory);
 //   * eight epilogue warps turn the counts of the other accumulator into sum p log(p / (p_a p_b)) per variable pair
 //     (the pseudocount spread over the table as in the reference) under the next tile's contraction.  The logarithm
-//     of a smoothed count is looked up: there are only rows + 1 of them.
-// Bound: the tensor pipe (512 clocks per stage) and shared memory (the MMAs read 48 KB per stage, 384 clocks, next
-// to the byte stores).  3072 variables x 32 categories x 4096 rows: 283 -> 22.9 ms (64 categories and more: 15.5 - 17.6 ms).
+//     of a smoothed count is looked up while all rows + 1 of them fit in shared memory (MAX_TABLE); with more rows every
+//     cell takes a logf.
+// Bound: no single unit.  Issue slots are 66% busy (producers and epilogue), the tensor pipe is active 38% of the time, the
+// MMAs read 48 KB of shared memory per stage next to the byte stores.  3072 variables x 32 categories x 4096 rows, this
+// kernel alone: 283 -> 22.9 ms, the whole call 23.6 - 26.2 ms with the clock (64 categories and more: 15.5 - 17.6 ms).
 #include <algorithm>
 #include <string>
 

@@ -244,10 +244,10 @@ __global__ void sample_hard_kernel(uint32_t S, const float* __restrict__ params,
 // records together.  Leaves of few categories are decided by their lanes, each on its own; a product's edges go to the
 // next round's list; the sum nodes of the piece are taken one after another by the whole warp, the parameters and noise
 // of the next one on their way, and the edges they select reach the list with one counter update.  The selection is the
-// same computation as in the one-warp walk, so the samples are the same bit for bit.  Bound: instruction issue (two
-// thirds of the slots at 4096 samples).  A warp per node, leaves included, with keys from two logarithms and a maximum
-// by five shuffles: 4096 samples of 784 variables x 64 latents 1573 us, now 450 us; the noise it must read (470 MB) is
-// 72 us of HBM.
+// same computation as in the one-warp walk, so the samples are the same bit for bit.  Bound: instruction issue (62%
+// of the slots at 4096 samples) and the loads a visit depends on.  A warp per node, leaves included, with keys from two
+// logarithms and a maximum by five shuffles: 4096 samples of 784 variables x 64 latents 1573 us, now 495 us (both alone
+// on the GPU); the noise it must read (470 MB) is 72 us of HBM.
 // CW: warps per sample.  One warp fills its lanes best and has nobody to wait for; where the samples alone do not fill
 // the GPU, more warps shorten the walk of each.
 constexpr uint32_t LANE_CATS = 8;               // categories up to which a leaf is decided by one lane
@@ -405,8 +405,8 @@ __global__ void __launch_bounds__(CW * 32, CW == 1 ? 32 : 40 / CW) sample_hard_c
 // logarithm and exponential by table and short polynomial (P. T. P. Tang, ACM TOMS 15 (1989) and 16 (1990)): the
 // result is rounded to fp32 (6e-8), a hundred times the error of these series, and ten fp64 operations per logarithm
 // replace the forty or more of one that is exact to the last bit.  Arguments outside the tables' range (u outside
-// [0, 1), |z| >= 600, NaN) take the CUDA functions.  Instruction issue is the bound (66% of the slots, fp64 units at a
-// fifth): the checks of a pair of edges share one branch, the noise-free variant is a kernel of its own.
+// [0, 1), |z| >= 600, NaN) take the CUDA functions.  Instruction issue is the bound (66% of the slots, fp64 units at
+// 28%): the checks of a pair of edges share one branch, the noise-free variant is a kernel of its own.
 constexpr uint32_t SOFT_THREADS = 256;
 // Every entry is there once for each lane of a half warp, so that lanes with different entries meet no bank twice (with
 // one copy a lookup of 128 and 256 entries took three times the passes): 32 entries, and two more terms of the series.
