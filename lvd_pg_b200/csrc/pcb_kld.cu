@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(KLD_THREADS) kld_up_layer_kernel(KldLayer a) {
   }
 }
 
-// One or two sets: one warp per (sum node, set), lanes over the node's edges.  Such a call is a chain of short dependent
+// A few sets (kld_by_warps): one warp per (sum node, set), lanes over the node's edges.  Such a call is a chain of short dependent
 // launches, so everything that does not depend on the step below (the run of children or the edge list, both parameters
 // of the first 64 edges and exp of one) is fetched BEFORE the wait on the preceding launch; after it only the children's
 // values are gathered, all of them in flight at once, so a step costs one round trip to L2.
