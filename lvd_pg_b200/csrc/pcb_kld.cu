@@ -306,32 +306,41 @@ __global__ void __launch_bounds__(256) kld_up_warp_kernel(KldLayer a) {
       keep(wgt[r]); keep(dif[r]);
     }
     keep(nsrc);
-    __syncthreads();
+    if (nsrc) __syncthreads();   // the same for the block
     pcb_grid_dep_wait();
     KLD_T_WAITED();
     const uint32_t first = nsrc ? src[0] : b.c0, second = nsrc > 1 ? src[1] : first, sub = b.d0 != PCB_NONE ? b.d0 : first;
-    auto value = [&](uint32_t j, float& product) {
-      const float k0 = klds[(size_t)(first + j) * ld], k1 = klds[(size_t)(second + j) * ld], k2 = klds[(size_t)(sub + j) * ld];
-      product = k0 + (nsrc > 1 ? k1 : 0.0f);
-      for (uint32_t x = 2; x < nsrc; x += 4) {
-        float y[4];
-#pragma unroll
-        for (uint32_t k = 0; k < 4; ++k) y[k] = x + k < nsrc ? klds[(size_t)(src[x + k] + j) * ld] : 0.0f;
-        product += (y[0] + y[1]) + (y[2] + y[3]);
-      }
-      return product + (b.d0 != PCB_NONE ? k2 : 0.0f);
-    };
-    float k[KLD_PRE], pr[KLD_PRE], acc = 0.0f;
-#pragma unroll
-    for (int r = 0; r < KLD_PRE; ++r) k[r] = lane + 32 * r < b.K ? value(lane + 32 * r, pr[r]) : 0.0f;
+    // the first 64 children together, four sources of each in flight
+    float k[KLD_PRE], pr[KLD_PRE], ks[KLD_PRE], acc = 0.0f;
 #pragma unroll
     for (int r = 0; r < KLD_PRE; ++r) {
-      acc += wgt[r] * (k[r] + dif[r]);
+      const uint32_t j = min(lane + 32 * r, b.K - 1);
+      const float k0 = klds[(size_t)(first + j) * ld], k1 = klds[(size_t)(second + j) * ld], k2 = klds[(size_t)(sub + j) * ld];
+      pr[r] = k0 + (nsrc > 1 ? k1 : 0.0f);
+      ks[r] = b.d0 != PCB_NONE ? k2 : 0.0f;
+    }
+    for (uint32_t x = 2; x < nsrc; x += 4) {
+      float y[KLD_PRE][4];
+#pragma unroll
+      for (int r = 0; r < KLD_PRE; ++r)
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+          y[r][q] = x + q < nsrc ? klds[(size_t)(src[x + q] + min(lane + 32 * r, b.K - 1)) * ld] : 0.0f;
+#pragma unroll
+      for (int r = 0; r < KLD_PRE; ++r) pr[r] += (y[r][0] + y[r][1]) + (y[r][2] + y[r][3]);
+    }
+#pragma unroll
+    for (int r = 0; r < KLD_PRE; ++r) {
+      k[r] = pr[r] + ks[r];
+      acc += lane + 32 * r < b.K ? wgt[r] * (k[r] + dif[r]) : 0.0f;
       if (nsrc && i == 0 && lane + 32 * r < b.K) klds[(size_t)(b.c0 + lane + 32 * r) * ld] = pr[r];   // the products' own values
     }
     for (uint32_t j = lane + 32 * KLD_PRE; j < b.K; j += 32) {
-      float product;
-      const float v = value(j, product), x = a.p1[base + (size_t)S * j], y = a.p2[base + (size_t)S * j];
+      float product = klds[(size_t)(first + j) * ld] + (nsrc > 1 ? klds[(size_t)(second + j) * ld] : 0.0f);
+#pragma unroll 4
+      for (uint32_t x = 2; x < nsrc; ++x) product += klds[(size_t)(src[x] + j) * ld];
+      const float v = product + (b.d0 != PCB_NONE ? klds[(size_t)(sub + j) * ld] : 0.0f);
+      const float x = a.p1[base + (size_t)S * j], y = a.p2[base + (size_t)S * j];
       acc += expf(x) * (v + x - y);
       if (nsrc && i == 0) klds[(size_t)(b.c0 + j) * ld] = product;
     }
@@ -694,10 +703,16 @@ __global__ void renorm_kernel(float* __restrict__ theta, uint32_t n_groups, cons
 // without dense blocks (a thread of a layer kernel walks such a node's edges alone) and in small ones (both passes on the
 // device, warps against tiles: 100 variables x 8 latents, four sets 37 against 98 us, eight 37 against 109; 100 x 32, four
 // sets 47 against 55, eight 56 against 58; 300 x 32, three sets 70 against 78, four 74 against 76, six 96 against 82;
-// 784 x 16, three sets 67 against 68, four 76 against 66; 784 x 64, three sets 285 against 109).
+// 784 x 16, three sets 67 against 68, four 76 against 66; 784 x 64, three sets 285 against 109).  In a deep
+// circuit the launches count: the way down by warps goes by layers, so it has to have no more of them than steps, and a
+// step to be small (a chain of 300 variables x 64 latents: three sets 1635 against 2087 us, five 1763 against 2146; a
+// lane holds 64 edges ahead of the wait: a chain of 100 x 100 latents, three sets 896 against 833; an image tree of 768
+// variables x 16 latents, three sets 349 against 311).
 constexpr uint32_t KLD_WARP_SETS = 2, KLD_WARP_SETS_SMALL = 8;
 bool kld_by_warps(const pcb_circuit* c, uint32_t S) {
-  return S <= KLD_WARP_SETS || (S <= KLD_WARP_SETS_SMALL && (c->n_dense == 0 || (uint64_t)S * c->n_inner <= 500000));
+  if (S <= KLD_WARP_SETS || S > KLD_WARP_SETS_SMALL || c->n_dense == 0) return S <= KLD_WARP_SETS_SMALL;
+  const uint64_t work = (uint64_t)S * c->n_inner;
+  return c->n_steps <= 32 ? work <= 500000 : c->L == c->n_steps && c->max_dense_K <= 64 && work <= (uint64_t)25000 * c->n_steps;
 }
 
 // what the kernels of step t need; the caller adds the loose nodes and the shares of a CTA
