@@ -634,14 +634,21 @@ def _row_major(mbpc, p, columns: int) -> bool:
         and p.dtype == torch.float32 and p.device == mbpc.device and p.is_contiguous()
 
 
+def _param_columns(mbpc, p: torch.Tensor) -> torch.Tensor:
+    """[P, S] from a row-major float32 [S, P] on the device by the library's kernel."""
+    out = torch.empty(p.shape[1], p.shape[0], dtype=torch.float32, device=p.device)
+    with torch.cuda.device(p.device):
+        _lib.check(mbpc.lib.pcb_param_columns(_ptr(out), _ptr(p), p.shape[0], p.shape[1], _stream(p.device)))
+    return out
+
+
 def _columns(mbpc, p: torch.Tensor) -> torch.Tensor:
-    """`p.t().contiguous()`; a row-major float32 matrix of several rows goes through the library's own kernel."""
-    if p.dim() == 2 and p.dtype == torch.float32 and p.is_contiguous() and 1 < p.shape[0] < 32 * 65535 and p.shape[1] > 1 \
-            and not p.requires_grad:
-        out = torch.empty(p.shape[1], p.shape[0], dtype=torch.float32, device=p.device)
-        with torch.cuda.device(p.device):
-            _lib.check(mbpc.lib.pcb_param_columns(_ptr(out), _ptr(p), p.shape[0], p.shape[1], _stream(p.device)))
-        return out
+    """`p.t().contiguous()`; a large row-major float32 matrix goes through the library's own kernel.  us per call, torch
+    against the kernel: 24 x 1.7 M values 125 / 75, 12 x 1 M 33 / 29, 16 x 300 k 14.5 / 15.5, 8 x 1.7 M 37 / 41, 3 x 1 M
+    10 / 21; small ones are the host's 7 / 12."""
+    if p.dim() == 2 and p.dtype == torch.float32 and p.is_contiguous() and 12 <= p.shape[0] < 32 * 65535 \
+            and p.numel() >= 4_000_000 and not p.requires_grad:
+        return _param_columns(mbpc, p)
     return p.t().contiguous()
 
 

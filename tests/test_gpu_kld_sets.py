@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 # (variables, latents, categories, sets): sets that do not divide the block, one set more than a tile, a child list
 # longer than the staged values (272 x 32 > 2048) with more steps per thread than are parked, single-child chains, few
 # sets on either side of the line between warps and tiles, no dense blocks
-SHAPES = [(9, 17, 3, 3), (20, 130, 2, 3), (20, 130, 2, 5), (40, 70, 2, 4), (30, 64, 2, 8), (9, 8, 3, 8), (9, 8, 3, 9), (12, 64, 2, 24), (6, 272, 2, 33), (7, 72, 5, 32), (5, 130, 2, 5), (6, 16, 2, 65)]
+SHAPES = [(9, 17, 3, 3), (20, 130, 2, 3), (60, 40, 2, 8), (20, 130, 2, 5), (40, 70, 2, 4), (30, 64, 2, 8), (9, 8, 3, 8), (9, 8, 3, 9), (12, 64, 2, 24), (6, 272, 2, 33), (7, 72, 5, 32), (5, 130, 2, 5), (6, 16, 2, 65)]
 
 
 @pytest.mark.parametrize("v,k,c,S", SHAPES)
@@ -29,13 +29,14 @@ def test_layer_kernels_against_oracle(oracle, v, k, c, S):
     assert rel_err(g2.cpu().numpy(), ref["param_grads2"]) <= TOL
 
 
-@pytest.mark.parametrize("S,P", [(2, 2), (3, 129), (31, 128), (33, 1000), (70, 257)])
+@pytest.mark.parametrize("S,P", [(2, 2), (3, 129), (31, 128), (33, 1000), (70, 257), (13, 310001)])
 def test_param_columns(S, P):
     torch, api = _cuda()
     m = api.CuMetaBitsProbCircuit(random_hclt(4, 8, 2, 1))
     x = torch.randn(S, P, device="cuda")
     y = api._columns(m, x)
     assert y.is_contiguous() and torch.equal(y, x.t())
+    assert torch.equal(api._param_columns(m, x), x.t())
     assert torch.equal(api._columns(m, x[:, ::2]), x[:, ::2].t())    # not row-major: the general path
 
 
