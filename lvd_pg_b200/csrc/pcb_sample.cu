@@ -5,7 +5,7 @@
 //    its children on; a leaf does the same arg-max over its categories.  The keys that decide are
 //    fp64 values of the shared host/device routine of include/pcb200_gumbel.h; an fp32 evaluation
 //    with an error bound first removes the entries that cannot win (race, warp_select64).  One CTA per
-//    sample takes the pending edges of a round in parallel (sample_hard_cta_kernel); one warp per
+//    sample takes the pending work of a round in parallel (sample_hard_cta_kernel, sample_hard_nodes_kernel); one warp per
 //    sample with a stack (sample_hard_kernel) serves very wide circuits and the entry point that
 //    allocates nothing.
 //    This is the temperature -> 0 limit of the reference's relaxed sampler
@@ -400,6 +400,136 @@ __global__ void __launch_bounds__(CW * 32, CW == 1 ? 32 : 40 / CW) sample_hard_c
   }
 }
 
+// The same walk for deep circuits, whose rounds have fewer pending nodes than warps: a round's latency is all that counts.
+// Pending work is a list of NODES (at most one per variable): the children of a sum node's edges come with its parameters
+// and need no load of their own, and the two children of an edge go to different warps.  Edge lists against this way, 256
+// samples: chain of 300 variables x 64 latents 906 -> 489 us, image trees of 768 x 16 latents 359 -> 293, 1500 x 32 705 -> 510.
+// The children cost 512 bytes of L2 reads per visit, so wide circuits keep the edge lists (784 variables
+// x 64 latents, 2000 samples 373 against 492 us).
+template <uint32_t CW>
+__global__ void __launch_bounds__(CW * 32, 32 / CW) sample_hard_nodes_kernel(
+    uint32_t S, const float* __restrict__ params, uint32_t Sp, const float* __restrict__ u_sum,
+    const float* __restrict__ u_leaf, uint32_t R, uint32_t kmax, uint32_t cmax, uint32_t V, uint32_t N,
+    const uint32_t* __restrict__ e_prime, const uint32_t* __restrict__ e_sub, uint64_t P, const float* __restrict__ theta,
+    uint32_t cap, int32_t* __restrict__ x_out, int32_t* __restrict__ status, const uint4* __restrict__ s_node,
+    const uint4* __restrict__ s_leaf, bool exact) {
+  extern __shared__ uint32_t lists[];   // [2][cap]
+  __shared__ uint32_t count[2];
+  const uint32_t s = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t ps = Sp == 1 ? 0 : s, pld = Sp;
+  if (threadIdx.x == 0) { lists[0] = N - 1; count[0] = 1; count[1] = 0; }
+  __syncthreads();
+  uint32_t cur = 0;
+  for (uint32_t round = 0;; ++round) {
+    const uint32_t n_cur = count[cur];
+    if (n_cur == 0 || n_cur > cap) break;   // more than the list holds: the status word says so
+    if (round > N + 8u) {   // a circuit is at most N levels deep
+      if (threadIdx.x == 0) atomicMax(status, 2);
+      break;
+    }
+    __syncthreads();                       // every thread has read the count
+    if (threadIdx.x == 0) count[cur] = 0;  // this list is the next round's target after the one being filled
+    uint32_t* const out = lists + (cur ^ 1u) * cap;
+    uint32_t* const out_n = &count[cur ^ 1u];
+    const uint32_t per = min(32u, (n_cur + CW - 1) / CW);   // nodes of a warp's piece
+    for (uint32_t base = warp * per; base < n_cur; base += CW * per) {
+      const bool has = lane < per && base + lane < n_cur;
+      const uint4 nm = has ? s_node[lists[cur * cap + base + lane]] : make_uint4(0, 0, 0, 3u);
+      const uint32_t kd = nm.w & 3u;
+      if (kd == PCB_INPUT) {
+        uint32_t C = nm.y & 0xffffu, var = nm.y >> 16;
+        uint64_t off = nm.x;
+        if (nm.x == 0xffffffffu) {
+          const uint4 lm = s_leaf[nm.z];
+          C = lm.z; var = lm.w;
+          off = (uint64_t)lm.x | ((uint64_t)lm.y << 32);
+        }
+        if (C <= LANE_CATS) {
+          // fixed leaves keep their log-probs in the circuit, not in the caller's parameter matrix
+          const float* lp = off < P ? params + ps + pld * off : theta + off;
+          x_out[s + (size_t)S * var] = (int32_t)lane_select(lp, off < P ? pld : 1, u_leaf + ((size_t)s * V + var) * cmax, C, exact);
+        }
+      } else if (kd == PCB_PRODUCT) {
+        for (uint32_t j = 0; j < nm.y; ++j) {
+          const uint32_t pr = e_prime[nm.x + j], sb = e_sub[nm.x + j], kids = sb != PCB_NONE ? 2u : 1u;
+          const uint32_t pos = atomicAdd(out_n, kids);
+          if (pos + kids > cap) { atomicMax(status, 1); break; }
+          out[pos] = pr;
+          if (kids == 2) out[pos + 1] = sb;
+        }
+      }
+      // leaves of many categories: a warp each
+      const uint32_t my_cats = kd != PCB_INPUT ? 0u : nm.x == 0xffffffffu ? s_leaf[nm.z].z : nm.y & 0xffffu;
+      for (uint32_t m = __ballot_sync(0xffffffffu, my_cats > LANE_CATS); m; m &= m - 1) {
+        const uint32_t src = (uint32_t)__ffs(m) - 1u;
+        const uint32_t ex = __shfl_sync(0xffffffffu, nm.x, src), ey = __shfl_sync(0xffffffffu, nm.y, src), ez = __shfl_sync(0xffffffffu, nm.z, src);
+        uint32_t C = ey & 0xffffu, var = ey >> 16;
+        uint64_t off = ex;
+        if (ex == 0xffffffffu) {
+          const uint4 lm = s_leaf[ez];
+          C = lm.z; var = lm.w;
+          off = (uint64_t)lm.x | ((uint64_t)lm.y << 32);
+        }
+        const float* us = u_leaf + ((size_t)s * V + var) * cmax;
+        auto lpa = [&](uint32_t c) { return off < P ? params[ps + pld * (off + c)] : theta[off + c]; };
+        const uint32_t bi = warp_select(lpa, us, C, lane, exact);
+        if (lane == 0) x_out[s + (size_t)S * var] = (int32_t)bi;
+      }
+      // sum nodes, the operands of the next one and the children of its edges in flight
+      uint32_t m = __ballot_sync(0xffffffffu, kd == PCB_SUM);
+      if (!m) continue;
+      const uint32_t sums = m, below = (1u << lane) - 1u;
+      uint32_t prime = PCB_NONE, sub = PCB_NONE;
+      float lp0 = 0.f, u0 = 0.f, lp1 = 0.f, u1 = 0.f;
+      uint32_t pr0 = 0, sb0 = 0, pr1 = 0, sb1 = 0;
+      auto fetch = [&](uint32_t src) {
+        const uint32_t cnt = __shfl_sync(0xffffffffu, nm.y, src), pid = __shfl_sync(0xffffffffu, nm.z, src);
+        const uint32_t reg = __shfl_sync(0xffffffffu, nm.w, src) >> 2, e0 = __shfl_sync(0xffffffffu, nm.x, src);
+        const float* us = u_sum + ((size_t)s * R + reg) * kmax;
+        const float* pp = params + ps + pld * (size_t)pid;
+        if (lane < cnt) { lp0 = pp[pld * lane]; u0 = __ldcs(us + lane); pr0 = e_prime[e0 + lane]; sb0 = e_sub[e0 + lane]; }
+        if (lane + 32 < cnt) {
+          lp1 = pp[pld * (lane + 32)]; u1 = __ldcs(us + lane + 32);
+          pr1 = e_prime[e0 + lane + 32]; sb1 = e_sub[e0 + lane + 32];
+        }
+      };
+      fetch((uint32_t)__ffs(m) - 1u);
+      while (m) {
+        const uint32_t src = (uint32_t)__ffs(m) - 1u;
+        m &= m - 1;
+        const uint32_t cnt = __shfl_sync(0xffffffffu, nm.y, src);
+        const float a0 = lp0, b0 = u0, a1 = lp1, b1 = u1;
+        const uint32_t p0 = pr0, q0 = sb0, p1 = pr1, q1 = sb1;
+        if (m) fetch((uint32_t)__ffs(m) - 1u);
+        uint32_t bi;
+        if (cnt <= 64) {
+          bi = warp_select64(a0, b0, lane < cnt, a1, b1, lane + 32 < cnt, lane, exact);
+        } else {
+          const uint32_t pid = __shfl_sync(0xffffffffu, nm.z, src), reg = __shfl_sync(0xffffffffu, nm.w, src) >> 2;
+          bi = warp_select([&](uint32_t j) { return params[ps + pld * (size_t)(pid + j)]; }, u_sum + ((size_t)s * R + reg) * kmax, cnt, lane, exact);
+        }
+        const uint32_t pr = __shfl_sync(0xffffffffu, bi < 32 ? p0 : p1, bi & 31u), sb = __shfl_sync(0xffffffffu, bi < 32 ? q0 : q1, bi & 31u);
+        if (lane == src) {
+          prime = bi < 64 ? pr : e_prime[nm.x + bi];
+          sub = bi < 64 ? sb : e_sub[nm.x + bi];
+        }
+      }
+      const uint32_t subs = __ballot_sync(0xffffffffu, sub != PCB_NONE), total = __popc(sums) + __popc(subs);
+      uint32_t pos = 0;
+      if (lane == 0) pos = atomicAdd(out_n, total);
+      pos = __shfl_sync(0xffffffffu, pos, 0);
+      if (pos + total > cap) { if (lane == 0) atomicMax(status, 1); }
+      else if ((sums >> lane) & 1u) {
+        pos += __popc(sums & below) + __popc(subs & below);
+        out[pos] = prime;
+        if (sub != PCB_NONE) out[pos + 1] = sub;
+      }
+    }
+    __syncthreads();   // the next list is complete
+    cur ^= 1u;
+  }
+}
+
 // ---- relaxed sampling: exp((log p + gumbel) / T) of every sum edge, normalised per sum node ------------------
 // The keys are formed in fp64 like the reference's (sample.jl:24-54 promotes through its Float64 literals), with
 // logarithm and exponential by table and short polynomial (P. T. P. Tang, ACM TOMS 15 (1989) and 16 (1990)): the
@@ -743,12 +873,16 @@ extern "C" int32_t pcb_sample_hard(pcb_circuit* c, pcb_workspace* ws, const floa
           S, params_dev, Sp, u_sum_dev, u_leaf_dev, c->n_regions, c->max_group, c->max_cats, c->V, c->N, c->e_prime, c->e_sub,
           c->P, c->theta, ws->stack_cap, x_out_dev, status, c->s_node, c->s_leaf, c->sample_exact_keys);
     };
-    // warps per sample, 784 variables x 64 latents, us with 1 / 2 / 4 / 8: 4096 samples 512 / 629 / 664 / 912, 2048 samples
-    // 412 / 367 / 407 / 494, 1024 samples 396 / 295 / 243 / 320, 512 samples 376 / 269 / 199 / 187
-    if (S >= 148 * 16) walk(sample_hard_cta_kernel<1>, 1);
-    else if (S >= 148 * 10) walk(sample_hard_cta_kernel<2>, 2);
-    else if (S >= 148 * 5) walk(sample_hard_cta_kernel<4>, 4);
-    else walk(sample_hard_cta_kernel<8>, 8);
+    // Warps per sample by the samples that an SM holds at a time, of the call's or of those whose lists fit: 784 variables x
+    // 64 latents, us with 1 / 2 / 4 / 8: 4096 samples 512 / 629 / 664 / 912, 2048 samples 412 / 367 / 407 / 494, 1024 samples
+    // 396 / 295 / 243 / 320, 512 samples 376 / 269 / 199 / 187.  3072 variables leave nine: 3500 samples of an image tree
+    // 13.9 ms with one warp each, 6.4 ms with several.  Up to sixteen variables per layer a circuit counts as deep.
+    const uint32_t resident = std::min(S / 148, (uint32_t)(227 * 1024 / (2 * ws->stack_cap * 4 + 1088)));
+    const bool deep = c->V <= 16 * c->L;
+    if (resident >= 16) walk(sample_hard_cta_kernel<1>, 1);
+    else if (resident >= 10) deep ? walk(sample_hard_nodes_kernel<2>, 2) : walk(sample_hard_cta_kernel<2>, 2);
+    else if (resident >= (deep ? 4u : 5u)) deep ? walk(sample_hard_nodes_kernel<4>, 4) : walk(sample_hard_cta_kernel<4>, 4);   // CTAs of eight warps per SM
+    else deep ? walk(sample_hard_nodes_kernel<8>, 8) : walk(sample_hard_cta_kernel<8>, 8);
     PCB_CUDA(cudaGetLastError());
     int32_t h0 = 0;
     PCB_CUDA(cudaMemcpyAsync(&h0, status, sizeof(int32_t), cudaMemcpyDeviceToHost, st));

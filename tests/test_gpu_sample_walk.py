@@ -3,6 +3,7 @@ nodes of more edges than a warp holds, one parameter set and one per sample, and
 import numpy as np
 import pytest
 
+from lvd_pg_b200 import structures as st
 from tests.helpers import random_hclt
 from tests.test_gpu_kld_sample import _cuda, _param_sets
 
@@ -55,3 +56,23 @@ def test_low_log_weights(oracle, v, k, c, S, lo, hi, impossible):
     x = torch.empty(v, n, dtype=torch.int32, device="cuda").t()
     api.sample_static(m, torch.from_numpy(p).cuda()[:, None], torch.from_numpy(u_sum[:n]).cuda(), torch.from_numpy(u_leaf[:n]).cuda(), x)
     assert np.array_equal(x.cpu().numpy(), want[:n])
+
+
+@pytest.mark.parametrize("kind,v,k,c,S", [("chain", 60, 16, 3, 40), ("chain", 40, 70, 9, 700), ("star", 50, 20, 2, 300), ("chain", 30, 8, 4, 1300),
+                                          ("chain", 3300, 2, 2, 1500), ("random", 4000, 2, 3, 2300)])
+def test_deep_wide_and_large_trees(oracle, kind, v, k, c, S):
+    """Hundreds of rounds of one node, one round of many, and lists that leave few samples on an SM: every number of
+    warps per sample, products of many factors, children of edges past the first 64."""
+    torch, api = _cuda()
+    rng = np.random.default_rng(v)
+    parent = {"chain": np.array([-1] + list(range(v - 1))), "star": np.array([-1, 0] + [1] * (v - 2))}.get(kind)
+    if parent is None:
+        parent = st.root_tree_at_center(v, st.random_spanning_tree(v, rng))
+    fc = st.hclt_flat(parent.astype(np.int64), c, k, seed=v)
+    m = api.CuMetaBitsProbCircuit(fc)
+    p = oracle.vectorize(fc)
+    shp = api.noise_shapes(m, S)
+    u_sum, u_leaf = rng.random(shp[0], dtype=np.float32), rng.random(shp[1], dtype=np.float32)
+    x = api.sample(m, p, u_sum, u_leaf).cpu().numpy()
+    keep = np.arange(0, S, max(1, S // 100))     # the oracle on every so many samples
+    assert np.array_equal(x[keep], oracle.sample_hard(fc, p[None], u_sum[keep], u_leaf[keep], len(keep)))
